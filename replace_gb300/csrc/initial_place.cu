@@ -33,6 +33,7 @@
 #include <cstdio>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "device_common.cuh"
@@ -47,6 +48,14 @@ struct BiState {
   int i, restarts, done, need_restart, zero_x;
   int par;                 // kernel-per-phase form: which p / v buffer holds the current iterate
   int pad[2];
+};
+
+// An SpMV block's x window (first index and length, 0: none) and sliced form
+// (ip_sell_body): its sliced, staged and special rows, the staged entries'
+// first place in sval / scol and their number, and each warp's first entry.
+struct __align__(64) SellBlock {
+  int lo, span, sliced, staged, special, stage_at, stage_n, pad;
+  int warp_at[8];
 };
 
 struct IpDev {
@@ -72,8 +81,19 @@ struct IpDev {
   int32_t* rowptr;         // [2][n_mov + 1]
   int32_t* scan_part;      // block sums of the scan
   int32_t* col;            // [2][nnz_cap]
-  uint16_t* col16;         // [2][nnz_cap] column - the block's x window start (blocks with a window)
   float* val;
+  // sliced form of the blocks with an x window (ip_sell_body); sval and scol
+  // share the memory of the assembly's per-slot arrays and pin positions,
+  // which are dead once the rows are summed
+  float* sval;             // [2][sell_cap]
+  uint16_t* scol;          // [2][sell_cap] 4 (column - the block's x window start)
+  // per slot of a block (sell_slots places: the slices in warp order, then
+  // the staged and special rows): row in its block | length << 16, and the
+  // row's diagonal entry
+  uint2* slot;             // [2][slot_cap]
+  int32_t* sstage;         // [2][slot_cap] a staged slot's place in the stage
+  uint32_t* swidth;        // [2][slot_cap / 32] per slice: width | least length << 16
+  SellBlock* sblk;         // [2][parts]
   float* diag;             // [2][n_mov]
   float* b;                // [2][n_mov]
   float *x, *r, *r0, *s, *t;   // [2][n_mov]
@@ -87,8 +107,7 @@ struct IpDev {
   BiState* st_h;           // pinned mirror
   int parts = 0;
   int rows_blk = 0;        // rows per block of the kernel-per-phase SpMV (a multiple of 32)
-  int2* win;               // [2][parts] x window (first index, length) of each SpMV block; length 0: none
-  size_t nnz_cap = 0;
+  size_t nnz_cap = 0, sell_cap = 0, slot_cap = 0;
   char* mem = nullptr;
   size_t bytes = 0;
 };
@@ -399,19 +418,85 @@ __device__ __forceinline__ void ip_rowsum_body(const IpDev& D, int vb, int axis)
   D.b[axis * D.n_mov + i] = rhs;
 }
 
-// The x window of SpMV block vb: its own rows and every column its rows'
-// entries read, as (first index, length), or length 0 when that is wider
-// than kXWin (the block then gathers from global memory); for a block with
-// a window, its entries' columns relative to the window start in 16 bits.
+// The x window and the sliced form of SpMV block vb.
+//
+// The window: the block's own rows and every column its rows' entries read,
+// as (first index, length), or length 0 when that is wider than kXWinMax
+// (the block then gathers from global memory and reads the CSR arrays).
+//
+// The sliced form (sliced ELLPACK with rows sorted by length inside the
+// block: Monakov, Lokhmotov, Avetisyan, HiPEAC'10; Kreutzer et al., SIAM J.
+// Sci. Comput. 36, 2014) of a block with a window: its rows sorted by
+// descending length, 32 to a slice, each slice as wide as its longest row
+// (rounded up to four): groups of four consecutive entries of the slice's 32
+// rows side by side (one 16-byte load a lane), columns as byte offsets from
+// the window start in 16 bits.  The eight warps take the slices in a snake
+// over the descending widths, so that each gets wide and narrow ones, and a
+// warp's slices lie one after another, so that it reads one stream.  A lane
+// sums its own row in entry order; rows of equal length share a slice, so few
+// lanes idle (unsorted, a window of 32 rows runs as long as its longest row,
+// three times the mean).  Which slot a row gets does not matter to its sum.
+//
+// One row in fifteen bounds large nets and is several times longer than the
+// rest (a quarter of the entries): in slices, its chain of loads would be
+// the block's critical path.  Rows longer than T entries are staged instead:
+// their entries lie row after row, all warps stage the products in shared
+// memory, and then a lane sums each row from there.  T is the smallest length
+// from 32 to kSellMax whose longer rows fit the stage (stage_cap).  Rows the
+// direct form of spmv_window sums with the whole warp (kWarpRow) keep that
+// order, and rows that no stage takes (kTall) a warp each (special rows, from
+// the CSR arrays).  The blocks take their entries' space from sell_cap by an
+// atomic counter; a block that finds no room keeps the CSR form (window
+// length 0), which gives the same sums.
 constexpr int kXWinMax = 5632;
-__device__ __forceinline__ void ip_window_body(const IpDev& D, int vb, int axis) {
+constexpr int kSellMax = 128;
+// The least T, and the stage in floats a row.  A block of one row per thread
+// (the small systems, whose kernels are bound by latency alone) takes slices
+// of four groups at most, larger blocks longer
+// ones (initial place of 10k / 30k / 60k cells: 58.4 / 64.6 / 73.4 ms with 16
+// against 61.4 / 66.6 / 74.8 with 32; of 100k and 400k 79.4 / 151.8 against
+// 78.5 / 150.7).
+__host__ __device__ constexpr int sell_min(int rows_blk) { return rows_blk <= 256 ? 16 : 32; }
+constexpr int kSellBins = kSellMax + 3;        // lengths kSellMax .. 0, staged, special
+constexpr int kLongRow = 32;   // rows longer than this may take the whole warp (spmv_window)
+constexpr int kStage = 1024;   // floats of shared memory per warp (spmv_window's stage)
+constexpr uint32_t kWarpRow = 0xffffu, kTall = 0xfffeu;   // slot lengths that mark special rows
+// slots of a block of rows_blk rows: whole slices for eight warps, and a
+// place for every staged or special row
+__host__ __device__ constexpr int sell_slices(int rows_blk) { return (rows_blk / 32 + 7) / 8 * 8; }
+__host__ __device__ constexpr int sell_slots(int rows_blk) { return 32 * sell_slices(rows_blk) + rows_blk; }
+// slice s of the descending widths: the s / 8-th of warp ..., and its place
+// among np slices a warp
+__device__ __forceinline__ int slice_place(int s, int np) {
+  const int p = s >> 3, w = (p & 1) ? 7 - (s & 7) : (s & 7);
+  return w * np + p;
+}
+constexpr int kSellAhead = 1024;   // entries the warps may read past their last one (two rings of groups)
+constexpr int kSellNext = 5;   // counters[axis * 8 + kSellNext]: next free sliced entry
+
+// Staged products of one block: eight or four floats a row (the generated
+// netlists need 6.4 with T = 16, 3.4 with 32), as far as the stages hold them
+// beside the block's results and its slice table.
+constexpr int kSliceTable = 512;               // floats: 2 kXWinMax / 32 rounded up
+static_assert(kSliceTable >= 2 * kXWinMax / 32, "one int2 per slice");
+__device__ __forceinline__ int stage_cap(int rows_blk) {
+  return min((rows_blk <= 256 ? 8 : 4) * rows_blk, max(0, (kB / 32) * kStage - kSliceTable - rows_blk));
+}
+
+__device__ __forceinline__ void ip_sell_body(const IpDev& D, int vb, int axis) {
   __shared__ int sh[2][kB / 32];
+  __shared__ uint32_t slot_s[kXWinMax];
+  __shared__ int hist[160];
+  __shared__ int scan[kB];
+  __shared__ int s_lo, s_span, s_base, s_T, s_over, s_cursor, s_staged, s_special, s_stage_at;
   const int n = D.n_mov;
-  const int r0 = vb * D.rows_blk, r1 = min(r0 + D.rows_blk, n);
+  const int r0 = vb * D.rows_blk, r1 = min(r0 + D.rows_blk, n), R = r1 - r0;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int32_t* rp = D.rowptr + axis * (n + 1);
+  const int32_t* col = D.col + axis * D.nnz_cap;
+  const float* val = D.val + axis * D.nnz_cap;
   int lo = r0, hi = r1;
   if (r0 < r1) {
-    const int32_t* rp = D.rowptr + axis * (n + 1);
-    const int32_t* col = D.col + axis * D.nnz_cap;
     const int k1 = (int)min((size_t)rp[r1], D.nnz_cap);
     for (int k = rp[r0] + threadIdx.x; k < k1; k += blockDim.x) {
       const int c = col[k];
@@ -424,25 +509,180 @@ __device__ __forceinline__ void ip_window_body(const IpDev& D, int vb, int axis)
     lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
     hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
   }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (lane == 0) { sh[0][wid] = lo; sh[1][wid] = hi; }
+  if (threadIdx.x < 160) hist[threadIdx.x] = 0;
+  if (threadIdx.x == 0) { s_over = 0; s_cursor = 0; }
   __syncthreads();
-  __shared__ int s_lo;
   if (threadIdx.x == 0) {
     for (int w = 1; w < kB / 32; w++) { lo = min(lo, sh[0][w]); hi = max(hi, sh[1][w]); }
-    const bool fits = r0 < r1 && hi - lo <= kXWinMax;
-    D.win[axis * D.parts + vb] = make_int2(fits ? lo : 0, fits ? hi - lo : 0);
+    // (rows past the entry bound were dropped and reported by the fill)
+    const bool fits = r0 < r1 && hi - lo <= kXWinMax && (size_t)rp[r1] <= D.nnz_cap;
     s_lo = fits ? lo : -1;
+    s_span = fits ? hi - lo : 0;
+    if (!fits) D.sblk[axis * D.parts + vb].span = 0;
   }
   __syncthreads();
-  // the window-relative columns the SpMV reads (2 bytes an entry instead of 4)
   const int base = s_lo;
-  if (base >= 0) {
-    const int32_t* rp = D.rowptr + axis * (n + 1);
-    const int32_t* col = D.col + axis * D.nnz_cap;
-    uint16_t* col16 = D.col16 + axis * D.nnz_cap;
-    const int k1 = (int)min((size_t)rp[r1], D.nnz_cap);
-    for (int k = rp[r0] + threadIdx.x; k < k1; k += blockDim.x) col16[k] = (uint16_t)(col[k] - base);
+  if (base < 0) return;                            // block-uniform
+  // row i's length, or kWarpRow
+  auto length_of = [&](int i) {
+    const int s = rp[r0 + i], e = rp[r0 + i + 1];
+    const int w = r0 + (i & ~31);
+    const int total = rp[min(w + 32, r1)] - rp[w];
+    if (total > kStage && e - s > kLongRow) return kWarpRow;
+    return (uint32_t)min(e - s, 0xfffd);
+  };
+  // rows by descending length; hist[kSellMax - length], the longer ones' sum
+  for (int i = threadIdx.x; i < R; i += kB) {
+    const uint32_t len = length_of(i);
+    if (len == kWarpRow) atomicAdd(&hist[kSellMax + 2], 1);
+    else if (len <= (uint32_t)kSellMax) atomicAdd(&hist[kSellMax - len], 1);
+    else { atomicAdd(&s_over, (int)len); atomicAdd(&hist[kSellMax + 1], 1); }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    // the smallest T in [sell_min, kSellMax] whose longer rows fit the stage
+    const int cap = stage_cap(D.rows_blk), t_min = sell_min(D.rows_blk);
+    int T = kSellMax, sum = s_over, rows = hist[kSellMax + 1];
+    const bool tall = sum > cap;                   // not even the longest rows fit: a warp each
+    if (tall) {
+      hist[kSellMax + 2] += rows;
+      hist[kSellMax + 1] = rows = 0;
+    } else {
+      while (T > t_min && sum + T * hist[kSellMax - T] <= cap) {
+        sum += T * hist[kSellMax - T];
+        rows += hist[kSellMax - T];
+        hist[kSellMax - T] = 0;
+        T--;
+      }
+    }
+    hist[kSellMax + 1] = rows;
+    s_T = tall ? -1 : T;
+    s_staged = rows;
+    s_special = hist[kSellMax + 2];
+  }
+  __syncthreads();
+  if (wid == 0) {
+    // exclusive scan of the kSellBins bins, five per lane
+    static_assert(kSellBins <= 160, "five bins per lane");
+    int h[5], x = 0;
+#pragma unroll
+    for (int j = 0; j < 5; j++) { h[j] = hist[5 * lane + j]; x += h[j]; }
+    const int own = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    x -= own;
+#pragma unroll
+    for (int j = 0; j < 5; j++) { hist[5 * lane + j] = x; x += h[j]; }
+  }
+  __syncthreads();
+  const bool tall = s_T < 0;
+  const uint32_t T = tall ? kSellMax : s_T;
+  const size_t slot0 = axis * D.slot_cap + (size_t)vb * sell_slots(D.rows_blk);
+  const int tail = 32 * sell_slices(D.rows_blk);   // staged and special slots start here
+  const int n_sell = R - s_staged - s_special;
+  for (int i = threadIdx.x; i < R; i += kB) {
+    uint32_t len = length_of(i);
+    int bin;
+    if (len == kWarpRow) bin = kSellMax + 2;
+    else if (len <= T) bin = kSellMax - (int)len;
+    else if (!tall) bin = kSellMax + 1;
+    else { len = kTall; bin = kSellMax + 2; }
+    const int t = atomicAdd(&hist[bin], 1);
+    slot_s[t] = (uint32_t)i | (len << 16);
+    if (bin == kSellMax + 1)                       // its place in the stage
+      D.sstage[slot0 + tail + t - n_sell] = atomicAdd(&s_cursor, (int)len);
+  }
+  __syncthreads();
+  // slice widths, in the order the warps read them, and their first entries
+  const int ns = (n_sell + 31) / 32, np = (ns + 7) / 8;   // 8 np <= kXWinMax / 32 + 8 <= kB
+  static_assert(kXWinMax / 32 + 8 <= kB, "one slice per thread");
+  scan[threadIdx.x] = 0;
+  __syncthreads();
+  int width = 0, place = 0;
+  if ((int)threadIdx.x < ns) {
+    width = (int)(((slot_s[32 * threadIdx.x] >> 16) + 3) & ~3u);
+    place = slice_place(threadIdx.x, np);
+    scan[place] = 32 * width;
+  }
+  __syncthreads();
+  for (int o = 1; o < kB; o <<= 1) {
+    const int x = threadIdx.x >= o ? scan[threadIdx.x - o] : 0;
+    __syncthreads();
+    scan[threadIdx.x] += x;
+    __syncthreads();
+  }
+  if (threadIdx.x == kB - 1) {
+    const int need = scan[kB - 1] + (s_cursor + 63) / 64 * 64;
+    const unsigned at = atomicAdd(&D.counters[axis * 8 + kSellNext], (unsigned)need);
+    const bool fits = (size_t)at + need + kSellAhead <= D.sell_cap;
+    SellBlock q{};
+    if (fits) {
+      q.lo = s_lo;
+      q.span = s_span;
+      q.sliced = n_sell;
+      q.staged = s_staged;
+      q.special = s_special;
+      q.stage_at = (int)at + scan[kB - 1];
+      q.stage_n = s_cursor;
+      for (int w = 0; w < 8; w++) q.warp_at[w] = (int)at + (w && np ? scan[w * np - 1] : 0);
+    }
+    D.sblk[axis * D.parts + vb] = q;
+    s_base = fits ? (int)at : -1;
+    s_stage_at = q.stage_at;
+  }
+  __syncthreads();
+  if (s_base < 0) return;                          // block-uniform
+  const float* dg = D.diag + axis * n + r0;
+  auto slot_of = [&](uint32_t v) { return make_uint2(v, __float_as_uint(dg[v & 0xffffu])); };
+  if ((int)threadIdx.x < 8 * np) D.swidth[slot0 / 32 + threadIdx.x] = 0u;
+  __syncthreads();
+  if ((int)threadIdx.x < ns) {
+    // (the least length: up to it the rows need no length test)
+    const int least = 32 * threadIdx.x + 31 < n_sell ? (int)(slot_s[32 * threadIdx.x + 31] >> 16) : 0;
+    D.swidth[slot0 / 32 + place] = (uint32_t)(width | least << 16);
+  }
+  for (int t = threadIdx.x; t < s_staged + s_special; t += kB) D.slot[slot0 + tail + t] = slot_of(slot_s[n_sell + t]);
+  for (int s = wid; s < ns; s += kB / 32) {
+    const int t = 32 * s + lane, at_s = slice_place(s, np);
+    const uint32_t v = t < n_sell ? slot_s[t] : kTall << 16;
+    const int len = t < n_sell ? (int)(v >> 16) : 0;
+    const int k0 = t < n_sell ? rp[r0 + (v & 0xffffu)] : 0;
+    D.slot[slot0 + 32 * at_s + lane] = t < n_sell ? slot_of(v) : make_uint2(v, 0u);
+    const int w = (int)(((slot_s[32 * s] >> 16) + 3) & ~3u);
+    const size_t first = axis * D.sell_cap + s_base + scan[at_s] - 32 * w;
+    float4* ov = reinterpret_cast<float4*>(D.sval + first) + lane;
+    uint2* oc = reinterpret_cast<uint2*>(D.scol + first) + lane;
+    for (int k = 0; k < w; k += 4) {
+      float x[4];
+      uint32_t c[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const bool in = k + u < len;
+        x[u] = in ? val[k0 + k + u] : 0.0f;
+        c[u] = in ? (uint32_t)(col[k0 + k + u] - base) * 4u : 0u;
+      }
+      ov[8 * k] = make_float4(x[0], x[1], x[2], x[3]);
+      oc[8 * k] = make_uint2(c[0] | c[1] << 16, c[2] | c[3] << 16);
+    }
+  }
+  // the staged rows' entries, row after row
+  for (int t = wid; t < s_staged; t += kB / 32) {
+    const uint32_t v = slot_s[n_sell + t];
+    const int k0 = rp[r0 + (v & 0xffffu)], len = (int)(v >> 16);
+    const size_t at = axis * D.sell_cap + s_stage_at + D.sstage[slot0 + tail + t];
+    for (int k = lane; k < len; k += 32) {
+      D.sval[at + k] = val[k0 + k];
+      D.scol[at + k] = (uint16_t)((col[k0 + k] - base) * 4);
+    }
+  }
+  // (their space is a multiple of 64; the products are formed four at a time)
+  for (int k = s_cursor + threadIdx.x; k < (s_cursor + 63) / 64 * 64; k += kB) {
+    D.sval[axis * D.sell_cap + s_stage_at + k] = 0.0f;
+    D.scol[axis * D.sell_cap + s_stage_at + k] = 0;
   }
 }
 
@@ -467,7 +707,9 @@ __global__ void k_ip_fill(const __grid_constant__ IpDev D, const __grid_constant
   ip_fill_body(D, P, (int)blockIdx.x, (int)gridDim.x, (int)blockIdx.y);
 }
 __global__ void k_ip_rowsum(const __grid_constant__ IpDev D) { ip_rowsum_body(D, (int)blockIdx.x, (int)blockIdx.y); }
-__global__ void k_ip_window(const __grid_constant__ IpDev D) { ip_window_body(D, (int)blockIdx.x, (int)blockIdx.y); }
+__global__ void __launch_bounds__(kB) k_ip_sell(const __grid_constant__ IpDev D) {
+  ip_sell_body(D, (int)blockIdx.x, (int)blockIdx.y);
+}
 
 // ------------------------------------------------------------ solver
 // Sparse products: each warp takes windows of 32 consecutive rows (row
@@ -496,8 +738,6 @@ __global__ void k_ip_window(const __grid_constant__ IpDev D) { ip_window_body(D,
 // in the cooperative and cluster solves; the products are the same).
 // kFromL2: read xv through L2 only (in the cooperative and cluster solves
 // other blocks wrote it since this block last read it).
-constexpr int kLongRow = 32;
-constexpr int kStage = 1024;   // floats of shared memory per warp
 
 // dynamic shared memory of a launch whose blocks have `threads` threads
 constexpr size_t stage_bytes(int threads) { return (size_t)(threads / 32) * kStage * sizeof(float); }
@@ -505,10 +745,11 @@ constexpr size_t stage_bytes(int threads) { return (size_t)(threads / 32) * kSta
 // The kernel-per-phase SpMV gives each block a contiguous range of rows and
 // stages the slice of the multiplied vector that the range's entries read
 // (its x window: the lowest to the highest column, at most kXWin floats)
-// in shared memory after the warps' product stages, so that the gathers hit
-// shared memory instead of L1/L2.  A block whose window is wider reads the
-// vector from global memory.  Product stages (32 KB) and window (22 KB) fit
-// four blocks per SM, the occupancy the grid is sized for.
+// in shared memory, so that the gathers hit shared memory instead of L1/L2;
+// such a block reads its sliced form (block_product).  A block whose window
+// is wider reads the vector from global memory, in the staged form.  Stages
+// (32 KB) and window (22 KB) fit four blocks per SM, the occupancy the grid
+// is sized for.
 constexpr int kXWin = kXWinMax;
 constexpr size_t spmv_bytes() { return stage_bytes(kB) + (size_t)kXWin * sizeof(float); }
 
@@ -603,23 +844,14 @@ __device__ __forceinline__ float spmv_window(const C* __restrict__ col, const fl
 
 // (A x)_i for the warp's windows w0, w0 + step, ... below n_end, x_j = gx(j);
 // epi(i, value, aux[i]) for every row (kAuxX: aux_i = x_i).  All 32 lanes
-// call it together (w0 is warp-uniform).  kWin: every x_j is read from
-// xs[j - lo] (the block's x window in shared memory, which holds every
-// column the rows read).
-template <bool kFromL2 = false, int kBatch = 16, bool kPrefetch = true, bool kWin = false, bool kAuxX = false,
-          class GX, class Epi>
+// call it together (w0 is warp-uniform).
+template <bool kFromL2 = false, int kBatch = 16, bool kPrefetch = true, bool kAuxX = false, class GX, class Epi>
 __device__ __forceinline__ void spmv_rows(const IpDev& D, int axis, GX gx, const float* aux,
-                                          int w0, int step, float* stage, Epi epi, int n_end = -1,
-                                          const float* xs = nullptr, int lo = 0) {
+                                          int w0, int step, float* stage, Epi epi, int n_end = -1) {
   const int n = n_end < 0 ? D.n_mov : n_end;
   const int lane = threadIdx.x & 31;
-  // entry columns: window-relative 16-bit in window mode, absolute otherwise
-  auto ldc = [&](int c) { return kWin ? xs[c] : gx(c); };
-  // the rows' own operands (absolute row index)
-  auto ld = [&](int j) { return kWin ? xs[j - lo] : gx(j); };
   const int32_t* __restrict__ rp = D.rowptr + axis * (D.n_mov + 1);
   const int32_t* __restrict__ col = D.col + axis * D.nnz_cap;
-  const uint16_t* __restrict__ col16 = D.col16 + axis * D.nnz_cap;
   const float* __restrict__ val = D.val + axis * D.nnz_cap;
   const float* __restrict__ dg = D.diag + axis * D.n_mov;
   auto fetch = [&](int w) {
@@ -628,7 +860,7 @@ __device__ __forceinline__ void spmv_rows(const IpDev& D, int axis, GX gx, const
     if (i < n) {
       f.s = rp[i];
       f.e = rp[i + 1];
-      const float xi = ld(i);
+      const float xi = gx(i);
       f.acc = __fmul_rn(dg[i], xi);
       f.aux = kAuxX ? xi : (aux ? (kFromL2 ? __ldcg(aux + i) : aux[i]) : 0.0f);
     }
@@ -638,15 +870,10 @@ __device__ __forceinline__ void spmv_rows(const IpDev& D, int axis, GX gx, const
   RowFetch cur = fetch(w0);
   RowFetch next = fetch(w0 + step);
   for (int w = w0; w < n; w += step) {
-    if constexpr (kPrefetch) {
-      if constexpr (kWin) prefetch_window(col16, val, next, w + step + lane < n);
-      else prefetch_window(col, val, next, w + step + lane < n);
-    }
+    if constexpr (kPrefetch) prefetch_window(col, val, next, w + step + lane < n);
     const RowFetch next2 = fetch(w + 2 * step);
     const int i = w + lane;
-    float v;
-    if constexpr (kWin) v = spmv_window<kFromL2, kBatch>(col16, val, ldc, cur, i < n, stage);
-    else v = spmv_window<kFromL2, kBatch>(col, val, ldc, cur, i < n, stage);
+    const float v = spmv_window<kFromL2, kBatch>(col, val, gx, cur, i < n, stage);
     if (i < n) epi(i, v, cur.aux);
     cur = next;
     next = next2;
@@ -734,27 +961,248 @@ __device__ __forceinline__ float* warp_stage() {
   return stage_all + (threadIdx.x >> 5) * kStage;
 }
 
-// The block's SpMV rows [r0, r1) and its x window: x_j = gx(j) over the
-// window, written to shared memory (after the product stages) by the whole
-// block.
+// Four consecutive entries of a slice, as one lane holds them.
+struct SellGroup {
+  float4 v;
+  uint2 c;
+};
+
+__device__ __forceinline__ float lds_at(const float* xs, uint32_t byte) {
+  return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(xs) + byte);
+}
+
+// acc += entries kk .. of the group, in order; no test below `least`, the
+// rest up to the row's length
+__device__ __forceinline__ void add_group(float& acc, const SellGroup& g, const float* xs, int kk, int least,
+                                          int len) {
+  if (kk + 4 <= least) {
+    const float x0 = lds_at(xs, g.c.x & 0xffffu), x1 = lds_at(xs, g.c.x >> 16);
+    const float x2 = lds_at(xs, g.c.y & 0xffffu), x3 = lds_at(xs, g.c.y >> 16);
+    acc = __fadd_rn(acc, __fmul_rn(g.v.x, x0));
+    acc = __fadd_rn(acc, __fmul_rn(g.v.y, x1));
+    acc = __fadd_rn(acc, __fmul_rn(g.v.z, x2));
+    acc = __fadd_rn(acc, __fmul_rn(g.v.w, x3));
+  } else {
+    if (kk < len) acc = __fadd_rn(acc, __fmul_rn(g.v.x, lds_at(xs, g.c.x & 0xffffu)));
+    if (kk + 1 < len) acc = __fadd_rn(acc, __fmul_rn(g.v.y, lds_at(xs, g.c.x >> 16)));
+    if (kk + 2 < len) acc = __fadd_rn(acc, __fmul_rn(g.v.z, lds_at(xs, g.c.y & 0xffffu)));
+    if (kk + 3 < len) acc = __fadd_rn(acc, __fmul_rn(g.v.w, lds_at(xs, g.c.y >> 16)));
+  }
+}
+
+// The block's SpMV rows [r0, r1), its x window (xs[j - lo]) and the rows'
+// products vs[i - r0] (span 0: neither, the caller takes the CSR arrays).
 struct BlockRows {
   int r0, r1, lo, span;
   const float* xs;
+  float* vs;
 };
-template <class GX>
-__device__ __forceinline__ BlockRows block_rows(const IpDev& D, GX gx, int vb, int axis) {
+
+// (A x)_i of the block's rows when it has a window: fills the window (ld(j):
+// the operands of x_j as loaded; cb(raw): x_j from them; scalars(): run by
+// one thread before any cb), then sums the rows into vs; ends with a block
+// barrier (false: `stop`, nothing done).  What bounds it is latency: a load
+// from L2 takes about 850 cycles, and a block's chain of them sets the
+// kernel's time.  So the first groups of the warp's stream, its first rows
+// and the first staged entries load before the window, the window's operands
+// four at a time, and then a ring of two groups a warp (48 bytes a lane) runs
+// ahead of the sums over all its slices; four groups cost spills and measured
+// 1 % slower.  The ring's loads are unconditional and of one size: behind
+// conditions the compiler waits for each (5.4 thousand cycles for the slices
+// of a 256-row block instead of 2.7).  Against the form that staged every
+// product and summed 32 neighbouring rows a warp, the initial place of 400k
+// cells went 183 -> 148 ms, of 1M cells 369 -> 320, of 30k 65.6 -> 62.3.
+template <class Ld, class Cb, class Sc>
+__device__ __forceinline__ bool block_product(const IpDev& D, int axis, int vb, int stop, Ld ld, Cb cb, Sc scalars,
+                                              BlockRows& b) {
   extern __shared__ float stage_all[];
-  BlockRows b;
+  static_assert(kXWin + kSliceTable <= (kB / 32) * kStage, "a windowed block's rows and table fit the stages");
+  constexpr int nw = kB / 32;
+  constexpr int kRing = 2;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const size_t slot0 = axis * D.slot_cap + (size_t)vb * sell_slots(D.rows_blk);
+  const SellBlock* __restrict__ Q = D.sblk + axis * D.parts + vb;
   b.r0 = vb * D.rows_blk;
   b.r1 = min(b.r0 + D.rows_blk, D.n_mov);
-  const int2 w = D.win[axis * D.parts + vb];
-  b.lo = w.x;
-  b.span = w.y;
-  float* xs = stage_all + (kB / 32) * kStage;
-  for (int k = threadIdx.x; k < b.span; k += blockDim.x) xs[k] = gx(b.lo + k);
-  __syncthreads();
+  b.lo = Q->lo;
+  b.span = Q->span;
+  const int n_sell = Q->sliced, n_staged = Q->staged, n_special = Q->special;
+  const int stage_at = Q->stage_at, stage_n = Q->stage_n, at = Q->warp_at[wid];
+  const uint32_t* __restrict__ sw = D.swidth + slot0 / 32;
+  const int n_tab = sell_slices(D.rows_blk);
+  const uint32_t width_t = (int)threadIdx.x < n_tab ? __ldg(sw + threadIdx.x) : 0u;
+  b.vs = stage_all;
+  float* xs = stage_all + nw * kStage;
   b.xs = xs;
-  return b;
+  if (stop) return false;                            // (with the table's loads under way)
+  if (b.span == 0) {
+    if (threadIdx.x == 0) scalars();
+    __syncthreads();
+    return true;
+  }
+  // the window's first operands, four elements of each
+  decltype(ld(0)) raw[4];
+#pragma unroll
+  for (int u = 0; u < 4; u++) raw[u] = ld(b.lo + min((int)threadIdx.x + u * kB, b.span - 1));
+  float* stage = stage_all + D.rows_blk;
+  uint32_t* tab = reinterpret_cast<uint32_t*>(stage_all + nw * kStage - kSliceTable);
+  const int own = b.r0 - b.lo;
+  const int ns = (n_sell + 31) / 32, np = (ns + 7) / 8;
+  // slices of this warp: the snake's passes, the last one only where it reaches
+  const int last = ns - 8 * (np - 1);                 // slices of the last pass
+  const int mine = np - ((((np - 1) & 1) ? nw - 1 - wid : wid) < last ? 0 : 1);
+  // the warp's stream: the first groups, the first rows, the first staged
+  // entries (reads past a warp's or the block's last group stay in the array)
+  const float4* __restrict__ gv = reinterpret_cast<const float4*>(D.sval + axis * D.sell_cap + at) + lane;
+  const uint2* __restrict__ gc = reinterpret_cast<const uint2*>(D.scol + axis * D.sell_cap + at) + lane;
+  SellGroup ring[kRing];
+#pragma unroll
+  for (int u = 0; u < kRing; u++) {
+    ring[u].v = __ldg(gv + 32 * u);
+    ring[u].c = __ldg(gc + 32 * u);
+  }
+  const uint2* __restrict__ slots = D.slot + slot0 + 32 * np * wid + lane;
+  uint2 row = __ldg(slots);
+  const float4* sv = reinterpret_cast<const float4*>(D.sval + axis * D.sell_cap + stage_at);
+  const uint2* sc4 = reinterpret_cast<const uint2*>(D.scol + axis * D.sell_cap + stage_at);
+  const int n4 = (stage_n + 3) / 4;
+  float4 pv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  uint2 pc = make_uint2(0u, 0u);
+  if ((int)threadIdx.x < n4) { pv = __ldg(sv + threadIdx.x); pc = __ldg(sc4 + threadIdx.x); }
+  if ((int)threadIdx.x < n_tab) tab[threadIdx.x] = width_t;
+  if (threadIdx.x == 0) scalars();
+  __syncthreads();
+  for (int k = threadIdx.x;;) {
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (k + u * kB < b.span) xs[k + u * kB] = cb(raw[u]);
+    k += 4 * kB;
+    if (k >= b.span) break;
+#pragma unroll
+    for (int u = 0; u < 4; u++) raw[u] = ld(b.lo + min(k + u * kB, b.span - 1));
+  }
+  __syncthreads();
+  // staged products, the next four in flight per thread
+  for (int j = threadIdx.x; j < n4; j += kB) {
+    const float4 v = pv;
+    const uint2 c = pc;
+    if (j + kB < n4) { pv = __ldg(sv + j + kB); pc = __ldg(sc4 + j + kB); }
+    reinterpret_cast<float4*>(stage)[j] =
+        make_float4(__fmul_rn(v.x, lds_at(xs, c.x & 0xffffu)), __fmul_rn(v.y, lds_at(xs, c.x >> 16)),
+                    __fmul_rn(v.z, lds_at(xs, c.y & 0xffffu)), __fmul_rn(v.w, lds_at(xs, c.y >> 16)));
+  }
+  if (mine > 0) {
+    gv += 32 * kRing;
+    gc += 32 * kRing;
+    int p = 0, k = 0;
+    uint32_t wl = tab[np * wid];
+    int len = (row.x >> 16) < kTall ? (int)(row.x >> 16) : 0;
+    float acc = len >= 0 ? __fmul_rn(__uint_as_float(row.y), xs[own + (row.x & 0xffffu)]) : 0.0f;
+    uint2 row2 = __ldg(slots + (1 < mine ? 32 : 0));
+    bool go = true;
+    while (go) {
+#pragma unroll
+      for (int u = 0; u < kRing; u++) {
+        if (k < (int)(wl & 0xffffu)) add_group(acc, ring[u], xs, k, (int)(wl >> 16), len);
+        ring[u].v = __ldg(gv + 32 * u);
+        ring[u].c = __ldg(gc + 32 * u);
+        k += 4;
+        if (k >= (int)(wl & 0xffffu) && go) {
+          if ((row.x >> 16) < kTall) b.vs[row.x & 0xffffu] = acc;
+          p++;
+          go = p < mine;
+          if (go) {
+            row = row2;
+            wl = tab[np * wid + p];
+            k = 0;
+            len = (row.x >> 16) < kTall ? (int)(row.x >> 16) : 0;
+            acc = __fmul_rn(__uint_as_float(row.y), xs[own + (row.x & 0xffffu)]);
+            row2 = __ldg(slots + 32 * (p + 1 < mine ? p + 1 : p));
+          }
+        }
+      }
+      gv += 32 * kRing;
+      gc += 32 * kRing;
+    }
+  }
+  // special rows, a warp each
+  const uint2* __restrict__ tail = D.slot + slot0 + 32 * n_tab;
+  for (int t = n_staged + wid; t < n_staged + n_special; t += nw) {
+    const unsigned full = 0xffffffffu;
+    const uint2 e = tail[t];
+    const uint32_t rr = e.x & 0xffffu;
+    const int32_t* rp = D.rowptr + axis * (D.n_mov + 1) + b.r0 + rr;
+    const int32_t* col = D.col + axis * D.nnz_cap;
+    const float* val = D.val + axis * D.nnz_cap;
+    const int ks = rp[0], ke = rp[1];
+    float acc = __fmul_rn(__uint_as_float(e.y), xs[own + rr]);
+    if ((e.x >> 16) == kWarpRow) {
+      // the direct form's order: lanes stride over the entries, then a tree
+      float part = 0.0f;
+      for (int k = ks + lane; k < ke; k += 32) part = __fmaf_rn(val[k], xs[col[k] - b.lo], part);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) part = __fadd_rn(part, __shfl_xor_sync(full, part, o));
+      acc = __fadd_rn(acc, part);
+    } else {
+      // entry order: 32 products at a time, added one after another
+      for (int k0 = ks; k0 < ke; k0 += 32) {
+        const int k = k0 + lane;
+        const float x = k < ke ? __fmul_rn(val[k], xs[col[k] - b.lo]) : 0.0f;
+        const int m = min(32, ke - k0);
+        for (int j = 0; j < m; j++) acc = __fadd_rn(acc, __shfl_sync(full, x, j));
+      }
+    }
+    if (lane == 0) b.vs[rr] = acc;
+  }
+  // the staged rows' sums, from the last warps (the first have the wide slices)
+  const int32_t* __restrict__ sst = D.sstage + slot0 + 32 * n_tab;
+  const int t0 = kB - 1 - (int)threadIdx.x;
+  uint2 e = make_uint2(0u, 0u);
+  int place = 0;
+  if (t0 < n_staged) { e = __ldg(tail + t0); place = __ldg(sst + t0); }
+  __syncthreads();
+  for (int t = t0; t < n_staged; t += kB) {
+    if (t != t0) { e = __ldg(tail + t); place = __ldg(sst + t); }
+    const uint32_t rr = e.x & 0xffffu;
+    const int len = (int)(e.x >> 16);
+    const float* x = stage + place;
+    float acc = __fmul_rn(__uint_as_float(e.y), xs[own + rr]);
+    int k = 0;
+    for (; k + 8 <= len; k += 8) {
+      float a[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) a[u] = x[k + u];
+#pragma unroll
+      for (int u = 0; u < 8; u++) acc = __fadd_rn(acc, a[u]);
+    }
+    for (; k < len; k++) acc = __fadd_rn(acc, x[k]);
+    b.vs[rr] = acc;
+  }
+  __syncthreads();
+  return true;
+}
+
+// op of the thread's first row of block vb (loaded ahead of the products)
+__device__ __forceinline__ float first_row_operand(const IpDev& D, int vb, const float* __restrict__ op) {
+  const int i = vb * D.rows_blk + (int)threadIdx.x;
+  return (int)threadIdx.x < D.rows_blk && i < D.n_mov ? __ldg(op + i) : 0.0f;
+}
+
+// f(i, (A x)_i, op[i]) for the block's rows in the thread's order: first is
+// op of its first row; the others' load four at a time before the f that use
+// them (whose stores the loads could not pass).
+template <class F>
+__device__ __forceinline__ void for_block_rows(const BlockRows& b, const float* __restrict__ op, float first, F f) {
+  int i = b.r0 + threadIdx.x;
+  if (i < b.r1) f(i, b.vs[i - b.r0], first);
+  for (i += kB; i < b.r1; i += 4 * kB) {
+    float o[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) o[u] = op[min(i + u * kB, b.r1 - 1)];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (i + u * kB < b.r1) f(i + u * kB, b.vs[i + u * kB - b.r0], o[u]);
+  }
 }
 
 // buffer `par` of p or v (axis `axis`)
@@ -762,36 +1210,107 @@ __device__ __forceinline__ float* pv_buf(float* base, const IpDev& D, int par, i
   return base + ((size_t)par * 2 + axis) * D.n_mov;
 }
 
-// block partial sums of up to 2 products, then the last block of this axis
-// runs `fin` with the totals (fixed-order reduction)
+// The exact double of a float by integer operations: conversions run on the
+// FP64 pipe, which takes 15 cycles per warp instruction on this part.
+__device__ __forceinline__ double widen(float f) {
+  const unsigned u = __float_as_uint(f), e = u & 0x7f800000u;
+  if (e == 0u || e == 0x7f800000u)                  // zero, denormal, infinity, NaN
+    return (u << 1) == 0u ? __hiloint2double((int)u, 0) : (double)f;
+  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
+}
+__device__ __forceinline__ double widen(double d) { return d; }
+
+// The sums block_reduce_n forms of N values a thread over a block of 256
+// threads -- each warp's 32 lanes in a halving tree, then the eight warps'
+// sums in one -- computed by one warp: lane l holds the values of threads
+// 32 g + l, g < 8, in x[k * 8 + g].  The additions are the same ones (a sum's
+// two operands may swap), but 12 (N = 1) or 19 (N = 2) warp instructions
+// replace 45 or 90 on the narrow FP64 pipe: at each step of the tree a lane
+// keeps the half of its sums that its lane bit selects and sends the other
+// half.  tot[k] is returned to every lane.
+template <int N, class T>
+__device__ __forceinline__ void warp_block_sum(const T (&x)[8 * N], double (&tot)[N]) {
+  static_assert(N == 1 || N == 2, "one or two values");
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  double v[4 * N];
+  {
+    const bool hi = lane & 16;
+#pragma unroll
+    for (int j = 0; j < 4 * N; j++) {
+      const T keep = hi ? x[4 * N + j] : x[j], send = hi ? x[j] : x[4 * N + j];
+      v[j] = widen(keep) + widen(__shfl_xor_sync(full, send, 16));
+    }
+  }
+  auto halve = [&](auto n_c, int o) {               // n sums a lane -> n / 2
+    constexpr int h = decltype(n_c)::value / 2;
+    const bool hi = lane & o;
+#pragma unroll
+    for (int j = 0; j < h; j++) {
+      const double keep = hi ? v[h + j] : v[j], send = hi ? v[j] : v[h + j];
+      v[j] = keep + __shfl_xor_sync(full, send, o);
+    }
+  };
+  halve(std::integral_constant<int, 4 * N>{}, 8);
+  halve(std::integral_constant<int, 2 * N>{}, 4);
+  if constexpr (N == 2) halve(std::integral_constant<int, 2>{}, 2);
+  else v[0] += __shfl_xor_sync(full, v[0], 2);
+  v[0] += __shfl_xor_sync(full, v[0], 1);
+  // a lane's warp g: lane bits 16, 8, 4 (N = 1) or 8, 4, 2 (N = 2; bit 16: k)
+#pragma unroll
+  for (int o = N == 1 ? 16 : 8; o >= (N == 1 ? 4 : 2); o >>= 1) v[0] += __shfl_xor_sync(full, v[0], o);
+  if constexpr (N == 1) {
+    tot[0] = v[0];
+  } else {
+    tot[0] = __shfl_sync(full, v[0], 0);
+    tot[1] = __shfl_sync(full, v[0], 16);
+  }
+}
+
+// Block partial sums of up to 2 products, then the last block of this axis
+// runs `fin` with the totals (fixed-order reduction).  One warp forms both
+// sums (warp_block_sum); the others are done once their floats are in shared
+// memory.
 template <int N, class Fin>
 __device__ __forceinline__ void reduce_and_finish(const IpDev& D, int kernel_id, const float (&vf)[N], Fin fin,
                                                   int vb, int vgrid, int axis) {
-  __shared__ double sh[32 * N];
-  __shared__ bool last;
+  __shared__ float sh[N * kB];
   double* part = D.part + (size_t)(axis * 2) * D.parts;
-  double v[N];
 #pragma unroll
-  for (int k = 0; k < N; k++) v[k] = vf[k];      // the thread's rows in float, FP64 across threads
-  block_reduce_n<N>(v, part, D.parts, sh, vb);
-  if (threadIdx.x == 0) {
+  for (int k = 0; k < N; k++) sh[k * kB + threadIdx.x] = vf[k];   // the thread's rows in float, FP64 across threads
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  const int lane = threadIdx.x;
+  double r[N];
+  {
+    float x[8 * N];
+#pragma unroll
+    for (int g = 0; g < 8 * N; g++) x[g] = sh[(g >> 3) * kB + 32 * (g & 7) + lane];
+    warp_block_sum<N>(x, r);
+  }
+  int last = 0;
+  if (lane == 0) {
+#pragma unroll
+    for (int k = 0; k < N; k++) part[k * D.parts + vb] = r[k];
     __threadfence();
     last = atomicAdd(&D.counters[axis * 8 + kernel_id], 1u) == (unsigned)vgrid - 1;
   }
-  __syncthreads();
-  if (!last) return;
-  double tot[N];
+  if (!__shfl_sync(0xffffffffu, last, 0)) return;
+  __threadfence();                     // the other blocks' partials are visible to the whole warp
+  double x[8 * N];
 #pragma unroll
-  for (int k = 0; k < N; k++) tot[k] = 0.0;
-  for (int b = threadIdx.x; b < vgrid; b += blockDim.x)
+  for (int g = 0; g < 8 * N; g++) {
+    const int t = 32 * (g & 7) + lane;
+    x[g] = t < vgrid ? __ldcg(part + (size_t)(g >> 3) * D.parts + t) : 0.0;
+  }
+  for (int t0 = kB; t0 < vgrid; t0 += kB)
 #pragma unroll
-    for (int k = 0; k < N; k++) tot[k] += __ldcg(part + (size_t)k * D.parts + b);
-  __shared__ double tt[N];
-  block_reduce_n<N>(tot, tt, 1, sh, 0);
-  if (threadIdx.x == 0) {
-    double r[N];
-#pragma unroll
-    for (int k = 0; k < N; k++) r[k] = tt[k];
+    for (int g = 0; g < 8 * N; g++) {
+      const int t = t0 + 32 * (g & 7) + lane;
+      if (t < vgrid) x[g] += __ldcg(part + (size_t)(g >> 3) * D.parts + t);
+    }
+  warp_block_sum<N>(x, r);
+  if (lane == 0) {
     fin(D.st[axis], r);
     D.counters[axis * 8 + kernel_id] = 0u;
   }
@@ -811,7 +1330,6 @@ __device__ __forceinline__ void bi_residual_body(const IpDev& D, int init, int m
                                                  int axis) {
   float* stage = warp_stage();
   BiState& S = D.st[axis];
-  if (!init && (S.done || !S.need_restart)) return;
   const int n = D.n_mov;
   const float* bb = D.b + axis * n;
   float* x = D.x + axis * n;
@@ -819,7 +1337,9 @@ __device__ __forceinline__ void bi_residual_body(const IpDev& D, int init, int m
   float* r0 = D.r0 + axis * n;
   float v[2] = {0.0f, 0.0f};
   auto gx = [&](int j) { return x[j]; };
-  const BlockRows br = block_rows(D, gx, vb, axis);
+  const float first = first_row_operand(D, vb, bb);
+  BlockRows br;
+  if (!block_product(D, axis, vb, !init && (S.done || !S.need_restart), gx, [](float v) { return v; }, [] {}, br)) return;
   auto epi = [&](int i, float ax, float bi) {
     const float ri = bi - ax;
     r[i] = ri;
@@ -827,9 +1347,11 @@ __device__ __forceinline__ void bi_residual_body(const IpDev& D, int init, int m
     v[0] = __fmaf_rn(ri, ri, v[0]);
     v[1] = __fmaf_rn(bi, bi, v[1]);
   };
-  const int w0 = br.r0 + (threadIdx.x & ~31);
-  if (br.span) spmv_rows<false, 8, true, true>(D, axis, gx, bb, w0, kB, stage, epi, br.r1, br.xs, br.lo);
-  else spmv_rows<false, 8, true, false>(D, axis, gx, bb, w0, kB, stage, epi, br.r1);
+  if (br.span) {
+    for_block_rows(br, bb, first, epi);
+  } else {
+    spmv_rows<false, 8>(D, axis, gx, bb, br.r0 + (threadIdx.x & ~31), kB, stage, epi, br.r1);
+  }
   reduce_and_finish<2>(D, 0, v, [&](BiState& s, const double* t) {
     if (init) {
       s.r0sq = t[0];
@@ -853,40 +1375,44 @@ __device__ __forceinline__ void bi_residual_body(const IpDev& D, int init, int m
 // computed where it is read (the block's x window, its own rows for Xr, the
 // gathers of a block without a window) from the previous p and v, which
 // therefore live in a second buffer (S.par selects the current one).
-// kWB: entries per lane in flight in the window path (load scheduling only:
-// the arithmetic does not depend on it).
-template <int kWB = 8>
 __device__ __forceinline__ void bi_pv_body(const IpDev& D, int vb, int vgrid, int axis) {
   float* stage = warp_stage();
   const BiState& S = D.st[axis];
-  if (S.done) return;
-  // beta once per block: FP64 division is slow on this part
   __shared__ float sc[2];
-  if (threadIdx.x == 0) {
-    const double beta = (S.rho / S.rho_old) * (S.alpha / S.w);
-    sc[0] = (float)beta;                // Eigen's scalars are float
-    sc[1] = (float)S.w;
-  }
-  __syncthreads();
-  const float bf = sc[0], wf = sc[1];
-  const int par = S.par;
+  const int par = S.par, stop = S.done | S.need_restart;
+  const float first = first_row_operand(D, vb, D.r0 + axis * D.n_mov);
   const float* po = pv_buf(D.p, D, par, axis);
   const float* vo = pv_buf(D.v, D, par, axis);
   float* pn = pv_buf(D.p, D, par ^ 1, axis);
   float* vn = pv_buf(D.v, D, par ^ 1, axis);
   const float* r = D.r + axis * D.n_mov;
   const float* r0 = D.r0 + axis * D.n_mov;
-  auto gx = [&](int j) { return __fmaf_rn(bf, __fmaf_rn(-wf, vo[j], po[j]), r[j]); };
-  const BlockRows br = block_rows(D, gx, vb, axis);
-  for (int i = br.r0 + threadIdx.x; i < br.r1; i += blockDim.x) pn[i] = br.span ? br.xs[i - br.lo] : gx(i);
+  struct Raw { float p, v, r; };
+  auto ld = [&](int j) { return Raw{po[j], vo[j], r[j]}; };
+  auto cb = [&](const Raw& x) { return __fmaf_rn(sc[0], __fmaf_rn(-sc[1], x.v, x.p), x.r); };
+  auto gx = [&](int j) { return cb(ld(j)); };
+  // beta once per block: FP64 division is slow on this part
+  BlockRows br;
+  if (!block_product(D, axis, vb, stop, ld, cb, [&] {
+        const double beta = (S.rho / S.rho_old) * (S.alpha / S.w);
+        sc[0] = (float)beta;            // Eigen's scalars are float
+        sc[1] = (float)S.w;
+      }, br)) return;
   float acc[1] = {0.0f};
   auto epi = [&](int i, float vi, float r0i) {
     vn[i] = vi;
     acc[0] = __fmaf_rn(r0i, vi, acc[0]);
   };
-  const int w0 = br.r0 + (threadIdx.x & ~31);
-  if (br.span) spmv_rows<false, kWB, true, true>(D, axis, gx, r0, w0, kB, stage, epi, br.r1, br.xs, br.lo);
-  else spmv_rows<false, 4, true, false>(D, axis, gx, r0, w0, kB, stage, epi, br.r1);   // 3 gathers an entry
+  if (br.span) {
+    for_block_rows(br, r0, first, [&](int i, float vi, float r0i) {
+      pn[i] = br.xs[i - br.lo];
+      epi(i, vi, r0i);
+    });
+  } else {
+    for (int i = br.r0 + threadIdx.x; i < br.r1; i += blockDim.x) pn[i] = gx(i);
+    // 3 gathers an entry
+    spmv_rows<false, 4>(D, axis, gx, r0, br.r0 + (threadIdx.x & ~31), kB, stage, epi, br.r1);
+  }
   reduce_and_finish<1>(D, 1, acc, [&](BiState& s, const double* t) { s.alpha = s.rho / t[0]; }, vb, vgrid, axis);
 }
 
@@ -895,24 +1421,34 @@ __device__ __forceinline__ void bi_pv_body(const IpDev& D, int vb, int vgrid, in
 __device__ __forceinline__ void bi_st_body(const IpDev& D, int vb, int vgrid, int axis) {
   float* stage = warp_stage();
   const BiState& S = D.st[axis];
-  if (S.done) return;
+  const int stop = S.done | S.need_restart;
   const float af = (float)S.alpha;
   const float* vn = pv_buf(D.v, D, S.par ^ 1, axis);
   const float* r = D.r + axis * D.n_mov;
   float* s = D.s + axis * D.n_mov;
   float* t = D.t + axis * D.n_mov;
-  auto gx = [&](int j) { return __fmaf_rn(-af, vn[j], r[j]); };
-  const BlockRows br = block_rows(D, gx, vb, axis);
-  for (int i = br.r0 + threadIdx.x; i < br.r1; i += blockDim.x) s[i] = br.span ? br.xs[i - br.lo] : gx(i);
+  struct Raw { float v, r; };
+  auto ld = [&](int j) { return Raw{vn[j], r[j]}; };
+  auto cb = [&](const Raw& x) { return __fmaf_rn(-af, x.v, x.r); };
+  auto gx = [&](int j) { return cb(ld(j)); };
+  BlockRows br;
+  if (!block_product(D, axis, vb, stop, ld, cb, [] {}, br)) return;
   float acc[2] = {0.0f, 0.0f};
   auto epi = [&](int i, float ti, float si) {
     t[i] = ti;
     acc[0] = __fmaf_rn(ti, ti, acc[0]);
     acc[1] = __fmaf_rn(ti, si, acc[1]);
   };
-  const int w0 = br.r0 + (threadIdx.x & ~31);
-  if (br.span) spmv_rows<false, 8, true, true, true>(D, axis, gx, nullptr, w0, kB, stage, epi, br.r1, br.xs, br.lo);
-  else spmv_rows<false, 4, true, false, true>(D, axis, gx, nullptr, w0, kB, stage, epi, br.r1);
+  if (br.span) {
+    for (int i = br.r0 + threadIdx.x; i < br.r1; i += kB) {
+      const float si = br.xs[i - br.lo];
+      s[i] = si;
+      epi(i, br.vs[i - br.r0], si);
+    }
+  } else {
+    for (int i = br.r0 + threadIdx.x; i < br.r1; i += blockDim.x) s[i] = gx(i);
+    spmv_rows<false, 4, true, true>(D, axis, gx, nullptr, br.r0 + (threadIdx.x & ~31), kB, stage, epi, br.r1);
+  }
   reduce_and_finish<2>(D, 2, acc, [&](BiState& st, const double* tt) {
     st.w = tt[0] > 0.0 ? tt[1] / tt[0] : 0.0;
   }, vb, vgrid, axis);
@@ -921,7 +1457,7 @@ __device__ __forceinline__ void bi_st_body(const IpDev& D, int vb, int vgrid, in
 // x += alpha p + omega s; r = s - omega t; |r|^2 and r0 . r; next loop head
 __device__ __forceinline__ void bi_xr_body(const IpDev& D, int max_iter, int vb, int vgrid, int axis) {
   const BiState& S = D.st[axis];
-  if (S.done) return;
+  if (S.done || S.need_restart) return;
   const int n = D.n_mov;
   float* x = D.x + axis * n;
   float* r = D.r + axis * n;
@@ -1315,6 +1851,7 @@ __device__ __forceinline__ void ip_guess_body(const IpDev& D, int vb) {
   D.x[n + i] = (float)c.y;
   D.p[i] = D.p[n + i] = 0.0f;
   D.v[i] = D.v[n + i] = 0.0f;
+  if (i == 0) D.counters[kSellNext] = D.counters[8 + kSellNext] = 0u;   // the sliced form's next free entries
 }
 
 __global__ void k_ip_move(const __grid_constant__ IpDev D) { ip_move_body(D, (int)blockIdx.x); }
@@ -1329,11 +1866,13 @@ __global__ void k_ip_guess(const __grid_constant__ IpDev D) { ip_guess_body(D, (
 // arithmetic does not depend on the kernel they are compiled into).
 enum IpPhase {
   kIpPos = 0, kIpBound, kIpCount, kIpScanBlocks, kIpScanAdd, kIpRowptr, kIpFill, kIpRowsum, kIpGuess,
-  kIpResidualInit, kIpResidual, kIpPV, kIpST, kIpXr, kIpMove, kIpWindow
+  kIpResidualInit, kIpResidual, kIpPV, kIpST, kIpXr, kIpMove, kIpSell
 };
 
+// (three blocks per SM: at four the product phases spill, 341 against 307 ms
+// for the initial places of 16 jobs of 2k to 50k cells)
 template <int Ph>
-__global__ void __launch_bounds__(kB, 4) k_ipb(const IpDev* __restrict__ Ds, const IpParams* __restrict__ Ps,
+__global__ void __launch_bounds__(kB, 3) k_ipb(const IpDev* __restrict__ Ds, const IpParams* __restrict__ Ps,
                                             const int4* __restrict__ items) {
   // the job's tables in shared memory (IpDev is a few hundred bytes)
   __shared__ __align__(16) unsigned char raw[sizeof(IpDev)];
@@ -1358,11 +1897,11 @@ __global__ void __launch_bounds__(kB, 4) k_ipb(const IpDev* __restrict__ Ds, con
   else if constexpr (Ph == kIpGuess) ip_guess_body(D, vb);
   else if constexpr (Ph == kIpResidualInit) bi_residual_body(D, 1, Ps[it.x].max_iter, vb, vg, ax);
   else if constexpr (Ph == kIpResidual) bi_residual_body(D, 0, Ps[it.x].max_iter, vb, vg, ax);
-  else if constexpr (Ph == kIpPV) bi_pv_body<4>(D, vb, vg, ax);   // 4: no spills with the tables in shared memory
+  else if constexpr (Ph == kIpPV) bi_pv_body(D, vb, vg, ax);
   else if constexpr (Ph == kIpST) bi_st_body(D, vb, vg, ax);
   else if constexpr (Ph == kIpXr) bi_xr_body(D, Ps[it.x].max_iter, vb, vg, ax);
   else if constexpr (Ph == kIpMove) ip_move_body(D, vb);
-  else if constexpr (Ph == kIpWindow) ip_window_body(D, vb, ax);
+  else if constexpr (Ph == kIpSell) ip_sell_body(D, vb, ax);
 }
 
 // the scan of the block sums: one block of kScanT threads per (job, axis)
@@ -1405,11 +1944,11 @@ __global__ void k_ip_chunk_head(IpLoop* L, cudaGraphConditionalHandle h_chunk) {
 }
 
 // after a chunk: another one while a solve goes on and the host loop's
-// iteration bound allows (it counts 8 per chunk from 0)
+// chunk bound allows (every chunk finishes at least one iteration)
 __global__ void k_ip_chunk_tail(const BiState* st, IpLoop* L, cudaGraphConditionalHandle h_chunk) {
   const int n = ++L->chunks;
   const bool done = st[0].done && st[1].done;
-  cudaGraphSetConditional(h_chunk, (!done && 8 * n <= L->iter_limit) ? 1u : 0u);
+  cudaGraphSetConditional(h_chunk, (!done && n <= L->iter_limit) ? 1u : 0u);
 }
 
 // after the move: the round's error (solver.error() = sqrt(|r|^2 / |b|^2),
@@ -1444,6 +1983,8 @@ int solve_rows(size_t n) { return n <= (size_t)kSmallRows ? 1 : 4; }
 
 struct IpSizes {
   size_t nnz_cap = 1, bytes = 0;
+  size_t sell_cap = 64, slot_cap = 32;   // sliced entries and slots per axis
+  size_t shared = 0;   // bytes the assembly's per-slot arrays and the sliced entries share
   int grid = 1;        // SpMV blocks per axis
   int xr_grid = 1;     // x + r blocks per axis
   int parts = 1;       // block partials per axis and value (the larger grid)
@@ -1478,17 +2019,25 @@ IpSizes ip_sizes(const HostModel& m, int grid_cap) {
   z.xr_grid = nP <= (size_t)kSmallRows ? (z.grid + 3) / 4 : z.grid;
   z.parts = std::max(z.grid, z.xr_grid);
   const size_t scan_blocks = blocks_for((int)n_mp);
+  // the sliced entries with their padding (widths in fours, each slice as wide
+  // as its longest row) and the staged rows: 1.1 to 1.3 of the entries on
+  // generated netlists (and room for the last warp's reads ahead); a block that finds no room keeps the CSR form
+  z.sell_cap = (z.nnz_cap + 2 * z.nnz_cap / 5) / 128 * 128 + 128 * ((size_t)z.grid + 8);
+  z.slot_cap = (size_t)z.grid * sell_slots(z.rows_blk);
+  auto rnd = [](size_t b) { return (b + 255) / 256 * 256 + 256; };
+  z.shared = std::max(rnd(2 * n_mp * 4) * 3 + rnd(2 * (n_mp + 1) * 4) + rnd(m.n_pins * 8),
+                      rnd(2 * z.sell_cap * 4) + rnd(2 * z.sell_cap * 2));
   size_t bytes = 0;
-  auto add = [&](size_t b) { bytes += (b + 255) / 256 * 256 + 256; };
+  auto add = [&](size_t b) { bytes += rnd(b); };
   add((m.n_nets + 1) * 4); add(m.n_pins * 4); add(m.n_pins * 4); add(m.n_pins * 4);
   add(m.n_pins * 8); add(m.n_pins * 8); add((nP + 1) * 4); add(n_mp * 4);
-  add(nP * 8); add(m.n_pins * 8); add(m.n_nets * 16); add(2 * n_mp * 4); add(2 * (n_mp + 1) * 4);
-  add(2 * n_mp * 4); add(2 * n_mp * 4); add(2 * (nP + 1) * 4);
-  add(2 * scan_blocks * 4); add(2 * z.nnz_cap * 4); add(2 * z.nnz_cap * 2); add(2 * z.nnz_cap * 4);
+  add(nP * 8); add(m.n_nets * 16); bytes += z.shared; add(2 * (nP + 1) * 4);
+  add(2 * scan_blocks * 4); add(2 * z.nnz_cap * 4); add(2 * z.nnz_cap * 4);
+  add(2 * z.slot_cap * 8); add(2 * z.slot_cap * 4); add(2 * (z.slot_cap / 32) * 4);
+  add(2 * (size_t)z.parts * sizeof(SellBlock));
   for (int k = 0; k < 7; k++) add(2 * nP * 4);
   for (int k = 0; k < 2; k++) add(2 * 2 * nP * 4);
   add(2 * 2 * (size_t)z.parts * 8); add(4 * 2 * 2 * (size_t)z.parts * 8); add(sizeof(GridBar));
-  add(2 * (size_t)z.parts * 8);
   add(16 * 4); add(sizeof(IpLoop)); add(2 * sizeof(BiState));
   z.bytes = bytes;
   return z;
@@ -1604,6 +2153,8 @@ int ip_setup(HostModel& m, cudaStream_t s, int sm_count, void* pinned, cudaMemPo
   const int grid_cap = (coop_attr != 0 && per_sm > 0) ? std::max(1, per_sm * sm_count / 2) : sm_count * 8;
   const IpSizes z = ip_sizes(m, grid_cap);
   D.nnz_cap = z.nnz_cap;
+  D.sell_cap = z.sell_cap;
+  D.slot_cap = z.slot_cap;
   const int nb_mov = blocks_for(nP);
   const int grid = z.grid;
   D.parts = z.parts;
@@ -1628,16 +2179,26 @@ int ip_setup(HostModel& m, cudaStream_t s, int sm_count, void* pinned, cudaMemPo
   D.mov_pin_start = (int32_t*)take((nP + 1) * 4);
   D.mov_pins = (int32_t*)take(mp.size() * 4);
   D.ctr = (int2*)take(nP * 8);
-  D.pos = (int2*)take(m.n_pins * 8);
   D.bound = (int4*)take(m.n_nets * 16);
+  // the sliced entries overlay the assembly's arrays, dead once the rows
+  // are summed (every round writes these before it reads them)
+  char* const shared0 = cur;
   D.cnt = (int32_t*)take(2 * (size_t)D.n_mp * 4);
   D.slot_off = (int32_t*)take(2 * ((size_t)D.n_mp + 1) * 4);
   D.slot_diag = (float*)take(2 * (size_t)D.n_mp * 4);
   D.slot_rhs = (float*)take(2 * (size_t)D.n_mp * 4);
+  D.pos = (int2*)take(m.n_pins * 8);
+  cur = shared0;
+  D.sval = (float*)take(2 * D.sell_cap * 4);
+  D.scol = (uint16_t*)take(2 * D.sell_cap * 2);
+  cur = shared0 + z.shared;
+  D.slot = (uint2*)take(2 * D.slot_cap * 8);
+  D.sstage = (int32_t*)take(2 * D.slot_cap * 4);
+  D.swidth = (uint32_t*)take(2 * (D.slot_cap / 32) * 4);
+  D.sblk = (SellBlock*)take(2 * (size_t)D.parts * sizeof(SellBlock));
   D.rowptr = (int32_t*)take(2 * (nP + 1) * 4);
   D.scan_part = (int32_t*)take(2 * scan_blocks * 4);
   D.col = (int32_t*)take(2 * D.nnz_cap * 4);
-  D.col16 = (uint16_t*)take(2 * D.nnz_cap * 2);
   D.val = (float*)take(2 * D.nnz_cap * 4);
   D.diag = (float*)take(2 * nP * 4);
   D.b = (float*)take(2 * nP * 4);
@@ -1651,7 +2212,6 @@ int ip_setup(HostModel& m, cudaStream_t s, int sm_count, void* pinned, cudaMemPo
   D.part = (double*)take(2 * 2 * (size_t)D.parts * 8);
   D.cpart = (double*)take(4 * 2 * 2 * (size_t)D.parts * 8);
   D.bar = (GridBar*)take(sizeof(GridBar));
-  D.win = (int2*)take(2 * (size_t)D.parts * 8);
   D.counters = (unsigned*)take(16 * 4);
   D.loop = (IpLoop*)take(sizeof(IpLoop));
   D.st = (BiState*)take(2 * sizeof(BiState));
@@ -1747,9 +2307,9 @@ void ip_round_done(IpRun& R, int round, const BiState* st) {
 int run_initial_place(HostModel& m, cudaStream_t s, int sm_count, gpl_ip_stats* stats, Timer& timer,
                       void* pinned, cudaMemPool_t pool, cudaEvent_t sync_ev) {
   IpRun R;
+  const gpl_params& prm = m.p;
   int rc = ip_setup(m, s, sm_count, pinned, pool, sync_ev, R);
   if (rc) return rc;
-  const gpl_params& prm = m.p;
   IpDev& D = R.D;
   const IpParams& P = R.P;
   const int nP = R.nP, nb_mov = R.nb_mov, grid = R.grid, scan_blocks = R.scan_blocks;
@@ -1776,12 +2336,14 @@ int run_initial_place(HostModel& m, cudaStream_t s, int sm_count, gpl_ip_stats* 
     k_ip_fill<<<dim3(scan_blocks, 2), kB, 0, s>>>(D, P);
     k_ip_rowsum<<<g2, kB, 0, s>>>(D);
     k_ip_guess<<<nb_mov, kB, 0, s>>>(D);
-    k_ip_window<<<gs, kB, 0, s>>>(D);
+    k_ip_sell<<<gs, kB, 0, s>>>(D);
     k_bi_residual<<<gs, kB, spmv_bytes(), s>>>(D, 1, P.max_iter);
   };
   auto phase_chunk = [&]() {
+    // a restart is taken at the start of the next chunk; until then the
+    // iteration's kernels return at once
+    k_bi_residual<<<gs, kB, spmv_bytes(), s>>>(D, 0, P.max_iter);
     for (int k = 0; k < 8; k++) {
-      k_bi_residual<<<gs, kB, spmv_bytes(), s>>>(D, 0, P.max_iter);
       k_bi_pv<<<gs, kB, spmv_bytes(), s>>>(D);
       k_bi_st<<<gs, kB, spmv_bytes(), s>>>(D);
       k_bi_xr<<<gx, kB, 0, s>>>(D, P.max_iter);
@@ -1952,7 +2514,8 @@ int run_initial_place(HostModel& m, cudaStream_t s, int sm_count, gpl_ip_stats* 
       }
     }
     // BiCGSTAB phase by phase: chunks of iterations, then poll the done flags
-    for (int it = 0; !solved && it <= 2 * P.max_iter + 2; it += 8) {
+    // (a chunk finishes at least one iteration, a solve at most 2 max_iter)
+    for (int it = 0; !solved && it <= 2 * P.max_iter + 2; it++) {
       timer.begin(kKOther);
       if (chunk_exec) {
         if (cudaGraphLaunch(chunk_exec, s) != cudaSuccess) { rc = GPL_ERR_CUDA; break; }
@@ -1960,7 +2523,7 @@ int run_initial_place(HostModel& m, cudaStream_t s, int sm_count, gpl_ip_stats* 
         phase_chunk();
       }
       timer.end(kKOther);
-      timer.count(32);
+      timer.count(25);
       if (cudaGetLastError() != cudaSuccess) { rc = GPL_ERR_CUDA; break; }
       if (cudaMemcpyAsync(st_h, D.st, 2 * sizeof(BiState), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
           host_wait(s, sync_ev) != cudaSuccess) { rc = GPL_ERR_CUDA; break; }
@@ -2112,12 +2675,12 @@ int run_initial_place_batch(IpBatchJob* jobs, int n, int sm_count, int64_t* laun
       L(k_ipb<kIpFill>, kTScan, 0);
       L(k_ipb<kIpRowsum>, kTRowsum, 0);
       L(k_ipb<kIpGuess>, kTMov, 0);
-      L(k_ipb<kIpWindow>, kTSolve, 0);
+      L(k_ipb<kIpSell>, kTSolve, 0);
       L(k_ipb<kIpResidualInit>, kTSolve, spmv_bytes());
     };
     auto chunk = [&]() {
+      L(k_ipb<kIpResidual>, kTSolve, spmv_bytes());
       for (int k = 0; k < 8; k++) {
-        L(k_ipb<kIpResidual>, kTSolve, spmv_bytes());
         L(k_ipb<kIpPV>, kTSolve, spmv_bytes());
         L(k_ipb<kIpST>, kTSolve, spmv_bytes());
         L(k_ipb<kIpXr>, kTVec, 0);
@@ -2182,7 +2745,7 @@ int run_initial_place_batch(IpBatchJob* jobs, int n, int sm_count, int64_t* laun
         layout_changed = false;
       }
       if (!replay(assembly_exec, assembly, n_assembly)) { rc = GPL_ERR_CUDA; break; }
-      for (int it = 0; it <= 2 * maxit + 2; it += 8) {
+      for (int it = 0; it <= 2 * maxit + 2; it++) {
         if (!replay(chunk_exec, chunk, n_chunk) || cudaStreamSynchronize(bs) != cudaSuccess) {
           rc = GPL_ERR_CUDA;
           break;
