@@ -132,8 +132,8 @@ typedef struct gpl_params {
                                               grid and keeps the faster; the GEMM form only up to
                                               512 bins per axis, where it can be the faster: larger
                                               grids keep the FFT form untimed), 1 = FFT (register
-                                              FFTs per warp on 512^2 and 1024^2 grids, shared-memory
-                                              FFTs otherwise), 2 = tensor-core GEMMs (each value
+                                              FFTs on grids of 256 to 2048 bins per axis but 256^2,
+                                              shared-memory FFTs otherwise), 2 = tensor-core GEMMs (each value
                                               split into three bf16 terms, six products per GEMM;
                                               grids with both counts multiples of 128) */
   int32_t scatter_tile;                    /* scatter tile side in bins (16, 32 or 64); 0 = chosen
@@ -273,8 +273,9 @@ gpl_status gpl_nesterov_run(struct gpl_job* job, int32_t max_iters,
  * one CUDA graph.  Every job's iterations, log and result are bit-identical
  * to gpl_nesterov_run on that job alone.
  * The jobs: distinct, on one device, after gpl_nesterov_init, on the FFT
- * Poisson form with its shared-memory passes (poisson_path 1, a grid other
- * than 512 x 512 or 1024 x 1024; others return GPL_ERR_INVALID_ARG).
+ * Poisson form (poisson_path 1) and a grid other than 512 x 512 or
+ * 1024 x 1024 (those return GPL_ERR_INVALID_ARG).  On grids that take the
+ * register FFTs a job's Poisson passes stay its own launches.
  * max_iters: further iterations per job (<= 0: to the stop rule).  stats and
  * status are [n_jobs] (may be NULL): each job's progress and its
  * gpl_nesterov_run status; *kernel_launches (may be NULL): kernels

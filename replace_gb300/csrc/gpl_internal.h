@@ -450,8 +450,8 @@ void write_scatter_batch_args(const DeviceModel& d, void* dst);
 void write_cell_batch_args(const DeviceModel& d, const EvalArgs& a, void* dst);
 void write_wa_batch_args(const DeviceModel& d, const EvalArgs& a, void* dst);
 // the block-form Poisson passes of a job's grid: arguments, grids and
-// dynamic shared memory of passes A, B, C; false for the warp form
-// (512 x 512 and 1024 x 1024 grids) and the tensor-core form
+// dynamic shared memory of passes A, B, C; false for the group form
+// and the tensor-core form
 bool write_poisson_batch_args(const DeviceModel& d, void* dst_a, void* dst_b, void* dst_c,
                               int grid[3], size_t smem[3]);
 int scatter_batch_prepare_device();
@@ -472,6 +472,7 @@ struct BatchMember {
   bool start = true;        // its next evaluation starts an iteration
   int done = 0;             // iterations in this batch
   int limit = 0;            // iteration limit in this batch (0: to the stop rule)
+  bool own_poisson = false; // its grid takes the job's own Poisson launches
   gpl_iter_log* log = nullptr;
 };
 BatchRun* batch_create(int device, int capacity, int* rc);

@@ -1242,7 +1242,10 @@ int batch_join(BatchRun* B, int slot, gpl_job* j, int max_iters, gpl_iter_log* l
   const bool ok = write_poisson_batch_args(d, part[kTPa], part[kTPb], part[kTPc], g3, sm3);
   d.ctl = own_ctl;
   d.result = own_res;
-  if (!ok) { set_error("batch: Poisson arguments"); return GPL_ERR_INVALID_ARG; }
+  if (!ok) {                       // the job's own Poisson launches (group form)
+    g3[0] = g3[1] = g3[2] = 0;
+    sm3[0] = sm3[1] = sm3[2] = 0;
+  }
   // the job's own stream may still hold work (initialisation)
   GPL_CUDA(cudaStreamSynchronize(j->stream));
   for (int t = 0; t < kTables; t++)
@@ -1269,6 +1272,7 @@ int batch_join(BatchRun* B, int slot, gpl_job* j, int max_iters, gpl_iter_log* l
   BatchMember& m = B->members[slot];
   m = BatchMember();
   m.job = j;
+  m.own_poisson = !ok;
   m.limit = max_iters;
   m.log = log;
   const NesterovState& S = j->S;
@@ -1358,6 +1362,19 @@ int batch_launch_round(BatchRun& B) {
     if (!B.phase_used[p]) continue;
     rc = launch_poisson_batch(q, B.args[kTPa + q], items(p), count(p), grid(p), B.smem_p[q], B.s);
     nl++;
+  }
+  // members on grids the batched passes do not cover: the launches of the
+  // job alone, on the batch's control record
+  for (int k = 0; k < B.cap && !rc; k++) {
+    BatchMember& m = B.members[k];
+    if (!m.job || !m.running || !m.own_poisson) continue;
+    DeviceModel& d = m.job->d;
+    EvalCtl* own = d.ctl;
+    Timer quiet;
+    d.ctl = B.ctl_d + k;
+    rc = launch_poisson_job(d, false, B.s, quiet);
+    d.ctl = own;
+    nl += quiet.kernels;
   }
   if (!rc && B.phase_used[kBDgradBig]) {
     rc = launch_density_batch(kBDgradBig, B.args[kTCell], items(kBDgradBig), count(kBDgradBig), grid(kBDgradBig),

@@ -18,10 +18,11 @@
 // even/odd reordering for the DCT-II and its inverse for the DCT-III; an
 // IDST is a DCT-III of the reversed input with alternating output signs.
 //
-// Two forms of the same passes: on 512 x 512 and 1024 x 1024 grids one warp
-// per packed pair runs a register FFT (the "warp form", with the density in
-// its own kernel before pass A); other grids use one packed pair per
-// 256-thread block and radix-4 Stockham passes in shared memory.
+// Two forms of the same passes: on grids of 256 to 2048 bins per axis (but
+// 256 x 256) a group of 16 to 64 lanes per packed pair runs a register FFT
+// (the "group form", with the density in its own kernel before pass A); other
+// grids use one packed pair per 256-thread block and radix-4 Stockham passes
+// in shared memory.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -484,35 +485,48 @@ __global__ void __launch_bounds__(256) k_poisson_c(const __grid_constant__ PassC
 }
 
 // ---------------------------------------------------------------------------
-// Warp form for 1024 x 1024 and 512 x 512 grids.  One warp runs one N-point
-// FFT of a packed pair (two rows or two columns as real and imaginary parts)
-// with N/32 elements per lane in registers, four-step: DFTs along n2 inside
+// Group form, for grids whose counts are both 256, 512, 1024 or 2048 (256 x
+// 256 excepted).  A group of G lanes (16, 32 or 64) runs one N-point FFT of a
+// packed pair (two rows or two columns as real and imaginary parts) with
+// E = N / G elements per lane in registers, four-step: DFTs along n2 inside
 // each lane, the twiddle W^(n1 k2), one transpose through padded shared
-// memory, then 32-point DFTs along n1 (for N = 512 each of those is split
-// over a lane pair: two 16-point DFTs and one radix-2 step by shuffle).  This
-// replaces five shared-memory radix-4 passes with block barriers.
-// Independent transforms of a pair run on separate warps (the column pass's
-// two inverse transforms, the field pass's three), inputs and tables arrive
-// by cp.async so that a warp waits for memory once, and the density comes
-// from its own grid-wide kernel first (fusing it into the row pass was
-// measured slower: its long blocks overlap worse with the WA kernel).
+// memory, then G-point DFTs along n1 (for N = 512 and 2048, where G = 2 E,
+// each of those is split over a lane pair: two E-point DFTs and one radix-2
+// step by shuffle).  The block form's radix-4 passes in shared memory take
+// five or six passes with block barriers for the same transform.
+// What bounds these passes is latency and issue, not bytes, so: independent
+// transforms of a pair run on separate groups (the column pass's two inverse
+// transforms, the field pass's three); elements k and n - k, which every pre-
+// and post-processing step combines, are handled by one lane, in place, so
+// that no second copy of the rows or the spectrum is kept (at 2048 points
+// that is what lets two field blocks share an SM); and the density comes from
+// its own grid-wide kernel first (fusing it into the row pass was measured
+// slower: its long blocks overlap worse with the WA kernel).
+// Solve of a 2048 x 2048 grid with the potential: 314 us in the block form,
+// 92 us here; 512 x 256: 26.6 -> 20.5; 1024 x 1024: 34.8 -> 32.8.
 
 template <int N>
-struct WarpFft {
-  static_assert(N == 1024 || N == 512, "warp form sizes");
-  static constexpr int kE = N / 32;                     // elements per lane
-  static constexpr int kStride = kE + 1;                // padded transpose row
-  static constexpr int kBuf = 2 * N > 2 * 32 * kStride ? 2 * N : 2 * 32 * kStride;   // floats per warp buffer
+struct GroupFft {
+  static_assert(N == 256 || N == 512 || N == 1024 || N == 2048, "group form sizes");
+  static constexpr int kG = N == 256 ? 16 : N == 2048 ? 64 : 32;   // lanes per transform
+  static constexpr int kE = N / kG;                                // elements per lane
+  static constexpr int kStride = kE + 1;                           // padded transpose row
+  static constexpr int kBuf = 2 * kG * kStride;                    // floats per group buffer
+  static_assert(kBuf >= 2 * N, "the transpose holds the sequence");
 };
 
-// exp(-2 pi i n1 k2 / N) at [k2 * 32 + n1], k2 < N/32: one coalesced row per k2.
-__device__ __align__(16) float2 g_tw1024[1024];
+// exp(-2 pi i n1 k2 / N) at [k2 * G + n1], k2 < E: one coalesced row per k2.
+__device__ __align__(16) float2 g_tw256[256];
 __device__ __align__(16) float2 g_tw512[512];
+__device__ __align__(16) float2 g_tw1024[1024];
+__device__ __align__(16) float2 g_tw2048[2048];
 
 template <int N>
 __device__ __forceinline__ const float2* tw_table() {
-  if constexpr (N == 1024) return g_tw1024;
-  else return g_tw512;
+  if constexpr (N == 2048) return g_tw2048;
+  else if constexpr (N == 1024) return g_tw1024;
+  else if constexpr (N == 512) return g_tw512;
+  else return g_tw256;
 }
 
 template <int kBits>
@@ -522,38 +536,51 @@ __host__ __device__ constexpr int brev(int r) {
   return o;
 }
 
-// cos and sin of 2 pi m / 32, m = 0..8 (the other octants by symmetry).
-__host__ __device__ constexpr float cos32_oct(int m) {
-  return m == 0 ? 1.0f : m == 1 ? 0.980785280403230449f : m == 2 ? 0.923879532511286756f
-       : m == 3 ? 0.831469612302545237f : m == 4 ? 0.707106781186547524f
-       : m == 5 ? 0.555570233019602225f : m == 6 ? 0.382683432365089772f
-       : m == 7 ? 0.195090322016128268f : 0.0f;
+// cos and sin of 2 pi m / 64, m = 0..16 (the other octants by symmetry).
+__host__ __device__ constexpr float cos64_quad(int m) {
+  return m == 0 ? 1.0f
+       : m == 1 ? 0.995184726672196929f
+       : m == 2 ? 0.980785280403230431f
+       : m == 3 ? 0.956940335732208824f
+       : m == 4 ? 0.923879532511286738f
+       : m == 5 ? 0.881921264348355050f
+       : m == 6 ? 0.831469612302545236f
+       : m == 7 ? 0.773010453362736993f
+       : m == 8 ? 0.707106781186547573f
+       : m == 9 ? 0.634393284163645488f
+       : m == 10 ? 0.555570233019602289f
+       : m == 11 ? 0.471396736825997809f
+       : m == 12 ? 0.382683432365089837f
+       : m == 13 ? 0.290284677254462331f
+       : m == 14 ? 0.195090322016128331f
+       : m == 15 ? 0.098017140329560770f
+       : 0.0f;
 }
-__host__ __device__ constexpr float cos32(int m) {   // 0 <= m < 16
-  return m <= 8 ? cos32_oct(m) : -cos32_oct(16 - m);
+__host__ __device__ constexpr float cos64(int m) {   // 0 <= m < 32
+  return m <= 16 ? cos64_quad(m) : -cos64_quad(32 - m);
 }
-__host__ __device__ constexpr float sin32(int m) {   // 0 <= m < 16
-  return m <= 8 ? cos32_oct(8 - m) : cos32_oct(m - 8);
+__host__ __device__ constexpr float sin64(int m) {   // 0 <= m < 32
+  return m <= 16 ? cos64_quad(16 - m) : cos64_quad(m - 16);
 }
 
-// (re, im) times exp(kSign 2 pi i m / 32), m < 16 a compile-time constant.
+// (re, im) times exp(kSign 2 pi i m / 64), m < 32 a compile-time constant.
 template <int kSign>
-__device__ __forceinline__ void rot32(float& re, float& im, int m) {
+__device__ __forceinline__ void rot64(float& re, float& im, int m) {
   if (m == 0) return;
   const float r = re, i = im;
-  if (m == 8) {                     // exp(kSign i pi / 2) = kSign i
+  if (m == 16) {                    // exp(kSign i pi / 2) = kSign i
     re = kSign > 0 ? -i : i;
     im = kSign > 0 ? r : -r;
     return;
   }
-  const float c = cos32(m), sn = kSign > 0 ? sin32(m) : -sin32(m);
+  const float c = cos64(m), sn = kSign > 0 ? sin64(m) : -sin64(m);
   re = r * c - i * sn;
   im = r * sn + i * c;
 }
 
 // In-register M-point DFT (M = 16 or 32), radix-2 decimation in frequency:
 // natural input order, register r ends with output brev(r).  Twiddles
-// exp(kSign 2 pi i j / len) = exp(kSign 2 pi i (j 32/len) / 32) are
+// exp(kSign 2 pi i j / len) = exp(kSign 2 pi i (j 64/len) / 64) are
 // compile-time constants after unrolling.
 template <int M, int kSign>
 __device__ __forceinline__ void dft_reg(float (&re)[M], float (&im)[M]) {
@@ -570,13 +597,13 @@ __device__ __forceinline__ void dft_reg(float (&re)[M], float (&im)[M]) {
         im[a] = ai + bi;
         re[b] = ar - br;
         im[b] = ai - bi;
-        rot32<kSign>(re[b], im[b], j * (32 / len));
+        rot64<kSign>(re[b], im[b], j * (64 / len));
       }
     }
   }
 }
 
-// Asynchronous global -> shared copies (cp.async, sm_80+): a warp issues
+// Asynchronous global -> shared copies (cp.async, sm_80+): a block issues
 // all of its inputs and tables at once and waits once, so each pass pays one
 // memory latency instead of one per dependent load batch.
 __device__ __forceinline__ void cp_async4(void* dst, const void* src) {
@@ -593,94 +620,95 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// Copies n floats (n a multiple of 4 * 32, both pointers 16-byte aligned)
-// with the calling warp's 16-byte cp.async.
-__device__ __forceinline__ void warp_copy_async(float* dst, const float* src, int n) {
-  const int l = threadIdx.x & 31;
-  for (int t = 4 * l; t < n; t += 128) cp_async16(dst + t, src + t);
+// Barrier of the calling group: its warp, or for 64 lanes two warps by the
+// named barrier 1 + the group's number in the block.
+template <int G>
+__device__ __forceinline__ void group_sync() {
+  if constexpr (G <= 32) __syncwarp();
+  else asm volatile("bar.sync %0, 64;\n" ::"r"(1 + (int)(threadIdx.x >> 6)) : "memory");
 }
 
-// N-point FFT of buf (natural order in and out, [WarpFft<N>::kBuf] floats,
-// float2 view) by the calling warp; kSign -1 forward, +1 unnormalised
+// N-point FFT of buf (natural order in and out, [GroupFft<N>::kBuf] floats,
+// float2 view) by the calling group; kSign -1 forward, +1 unnormalised
 // inverse.  tws: the tw_table<N>() table in shared memory.
 template <int N, int kSign>
-__device__ __forceinline__ void warp_fft(float2* buf, const float2* tws) {
-  constexpr int E = WarpFft<N>::kE, S = WarpFft<N>::kStride;
-  constexpr int kBitsE = E == 32 ? 5 : 4;
-  const int l = threadIdx.x & 31;
-  float re[32], im[32];
-  // stage 1: lane n1 = l holds x[n1 + 32 n2], n2 < E; DFT along n2
+__device__ __forceinline__ void group_fft(float2* buf, const float2* tws) {
+  using F = GroupFft<N>;
+  constexpr int E = F::kE, S = F::kStride, G = F::kG;
+  constexpr int kBits = E == 32 ? 5 : 4;
+  const int l = threadIdx.x & (G - 1);
+  float re[E], im[E];
+  // stage 1: lane n1 = l holds x[n1 + G n2], n2 < E; DFT along n2
 #pragma unroll
   for (int j = 0; j < E; j++) {
-    const float2 v = buf[l + 32 * j];
+    const float2 v = buf[l + G * j];
     re[j] = v.x; im[j] = v.y;
   }
-  if constexpr (E == 32) {
-    dft_reg<32, kSign>(re, im);
-  } else {
-    float r16[16], i16[16];
-#pragma unroll
-    for (int j = 0; j < 16; j++) { r16[j] = re[j]; i16[j] = im[j]; }
-    dft_reg<16, kSign>(r16, i16);
-#pragma unroll
-    for (int j = 0; j < 16; j++) { re[j] = r16[j]; im[j] = i16[j]; }
-  }
+  dft_reg<E, kSign>(re, im);
   // twiddle W_N^(n1 k2), register r holding k2 = brev(r)
 #pragma unroll
   for (int r = 1; r < E; r++) {
-    float2 w = tws[brev<kBitsE>(r) * 32 + l];
+    float2 w = tws[brev<kBits>(r) * G + l];
     if (kSign > 0) w.y = -w.y;
     const float xr = re[r], xi = im[r];
     re[r] = xr * w.x - xi * w.y;
     im[r] = xr * w.y + xi * w.x;
   }
-  __syncwarp();
+  group_sync<G>();
   float* tr = reinterpret_cast<float*>(buf);
-  float* ti = tr + 32 * S;
+  float* ti = tr + G * S;
 #pragma unroll
   for (int r = 0; r < E; r++) {
-    tr[l * S + brev<kBitsE>(r)] = re[r];
-    ti[l * S + brev<kBitsE>(r)] = im[r];
+    tr[l * S + brev<kBits>(r)] = re[r];
+    ti[l * S + brev<kBits>(r)] = im[r];
   }
-  __syncwarp();
-  if constexpr (E == 32) {
-    // stage 2: lane k2 = l takes n1 = 0..31, a 32-point DFT, X[k2 + 32 k1]
+  group_sync<G>();
+  if constexpr (G == E) {
+    // stage 2: lane k2 = l takes n1 = 0..G-1, a G-point DFT, X[k2 + E k1]
 #pragma unroll
-    for (int n1 = 0; n1 < 32; n1++) {
+    for (int n1 = 0; n1 < G; n1++) {
       re[n1] = tr[n1 * S + l];
       im[n1] = ti[n1 * S + l];
     }
-    __syncwarp();
-    dft_reg<32, kSign>(re, im);
+    group_sync<G>();
+    dft_reg<E, kSign>(re, im);
 #pragma unroll
-    for (int r = 0; r < 32; r++) buf[l + 32 * brev<5>(r)] = make_float2(re[r], im[r]);
+    for (int r = 0; r < E; r++) buf[l + E * brev<kBits>(r)] = make_float2(re[r], im[r]);
   } else {
-    // stage 2 for E = 16: lane pair (2 k2, 2 k2 + 1) takes the even and odd
-    // n1 of column k2, one 16-point DFT each, then X[k] = E[k] + W^k O[k]
-    // (even lane) and X[k + 16] = E[k] - W^k O[k] (odd lane), W = W_32
+    // stage 2 for G = 2 E: lane pair (2 k2, 2 k2 + 1) takes the even and odd
+    // n1 of column k2, one E-point DFT each, then X[k] = E[k] + W^k O[k]
+    // (even lane) and X[k + E] = E[k] - W^k O[k] (odd lane), W = W_G
+    static_assert(G == 2 * E, "one or two lanes per column");
     const int k2 = l >> 1, odd = l & 1;
-    float r16[16], i16[16];
 #pragma unroll
-    for (int i = 0; i < 16; i++) {
-      r16[i] = tr[(2 * i + odd) * S + k2];
-      i16[i] = ti[(2 * i + odd) * S + k2];
+    for (int i = 0; i < E; i++) {
+      re[i] = tr[(2 * i + odd) * S + k2];
+      im[i] = ti[(2 * i + odd) * S + k2];
     }
-    __syncwarp();
-    dft_reg<16, kSign>(r16, i16);
+    group_sync<G>();
+    dft_reg<E, kSign>(re, im);
 #pragma unroll
-    for (int r = 0; r < 16; r++) {
-      const int k = brev<4>(r);
-      const float pr = __shfl_xor_sync(0xffffffffu, r16[r], 1);
-      const float pi = __shfl_xor_sync(0xffffffffu, i16[r], 1);
+    for (int r = 0; r < E; r++) {
+      const int k = brev<kBits>(r);
+      const float pr = __shfl_xor_sync(0xffffffffu, re[r], 1);
+      const float pi = __shfl_xor_sync(0xffffffffu, im[r], 1);
       // W^k O: O is the partner's value on the even lane, the own on the odd
-      float orr = odd ? r16[r] : pr, oi = odd ? i16[r] : pi;
-      rot32<kSign>(orr, oi, k);
-      const float er = odd ? pr : r16[r], ei = odd ? pi : i16[r];
+      float orr = odd ? re[r] : pr, oi = odd ? im[r] : pi;
+      rot64<kSign>(orr, oi, k * (64 / G));
+      const float er = odd ? pr : re[r], ei = odd ? pi : im[r];
       const float xr = odd ? er - orr : er + orr, xi = odd ? ei - oi : ei + oi;
-      buf[k2 + 16 * (k + 16 * odd)] = make_float2(xr, xi);
+      buf[k2 + E * (k + E * odd)] = make_float2(xr, xi);
     }
   }
-  __syncwarp();
+  group_sync<G>();
+}
+
+// c0 + i c1 of a packed pair's DCT-III coefficients (dct3_pre of each): the
+// pair's values at k and at n - k.
+__device__ __forceinline__ float2 pre_pair(float2 ak, float2 ank, float2 w4, int k) {
+  const float2 c0 = dct3_pre(ak.x, ank.x, w4, k);
+  const float2 c1 = dct3_pre(ak.y, ank.y, w4, k);
+  return make_float2(c0.x - c1.y, c0.y + c1.x);
 }
 
 // Density of every bin from the int64 areas, FP64 overflow partials (one per
@@ -713,151 +741,136 @@ __global__ void __launch_bounds__(256) k_poisson_dens(PassAArgs A) {
   if (A.part_overflow) block_reduce_add((double)ovf, &A.part_overflow[blockIdx.x], red);
 }
 
-// Pass A, warp form: DCT-II along x of row pair r (density rows 2r, 2r+1).
-// Shared memory: FFT buffer, w4 and twiddle tables.
+// Copies n floats (n a multiple of 4, both pointers 16-byte aligned) with the
+// block's 16-byte cp.async.
+__device__ __forceinline__ void block_copy_async(float* dst, const float* src, int n) {
+  for (int t = 4 * threadIdx.x; t < n; t += 4 * blockDim.x) cp_async16(dst + t, src + t);
+}
+
+// Pass A, group form: DCT-II along x of row pairs (density rows 2r, 2r + 1),
+// one pair a group, two groups of 16 lanes or one of 32 or 64 a block.
+// Shared memory: FFT buffers, the twiddle table.
 template <int N>
-__global__ void __launch_bounds__(32) k_poisson_rows_w(PassAArgs A) {
+struct RowsShape {
+  static constexpr int kT = GroupFft<N>::kG < 32 ? 32 : GroupFft<N>::kG;
+  static constexpr int kP = kT / GroupFft<N>::kG;       // row pairs per block
+  static constexpr size_t kBytes = (size_t)kP * GroupFft<N>::kBuf * 4 + N * 8;
+};
+
+template <int N>
+__global__ void __launch_bounds__(RowsShape<N>::kT) k_poisson_rows_g(PassAArgs A) {
   extern __shared__ float2 smem[];
-  float2* buf = smem;
-  float2* w4s = smem + WarpFft<N>::kBuf / 2;
-  float2* tws = w4s + N;
-  const int l = threadIdx.x;
-  const int r = blockIdx.x;
+  using F = GroupFft<N>;
+  constexpr int G = F::kG, P = RowsShape<N>::kP;
+  const int l = threadIdx.x & (G - 1), p = threadIdx.x / G;
+  float2* buf = smem + (size_t)p * (F::kBuf / 2);
+  float2* tws = smem + (size_t)P * (F::kBuf / 2);
+  const int r = blockIdx.x * P + p;
   const float* d0 = (A.density_in ? A.density_in : A.density) + (size_t)(2 * r) * N;
   const float* d1 = d0 + N;
   // Makhoul order: v[m] = x[2m], v[n-1-m] = x[2m+1]
 #pragma unroll 8
-  for (int j = 0; j < N / 32; j++) {
-    const int i = l + 32 * j;
+  for (int j = 0; j < N / G; j++) {
+    const int i = l + G * j;
     float* dst = reinterpret_cast<float*>(&buf[makhoul_pos(i, N)]);
     cp_async4(dst, d0 + i);
     cp_async4(dst + 1, d1 + i);
   }
-  warp_copy_async(reinterpret_cast<float*>(w4s), reinterpret_cast<const float*>(A.w4), 2 * N);
-  warp_copy_async(reinterpret_cast<float*>(tws), reinterpret_cast<const float*>(tw_table<N>()), 2 * N);
+  block_copy_async(reinterpret_cast<float*>(tws), reinterpret_cast<const float*>(tw_table<N>()), 2 * N);
   cp_async_wait_all();
-  __syncwarp();
-  warp_fft<N, -1>(buf, tws);
+  __syncthreads();
+  group_fft<N, -1>(buf, tws);
   float* s0 = A.spec + (size_t)(2 * r) * N;
   float* s1 = s0 + N;
 #pragma unroll 8
-  for (int j = 0; j < N / 32; j++) {
-    const int k = l + 32 * j;
-    const float2 c = dct2_post(buf[k], buf[(N - k) & (N - 1)], w4s[k]);
+  for (int j = 0; j < N / G; j++) {
+    const int k = l + G * j;
+    const float2 c = dct2_post(buf[k], buf[(N - k) & (N - 1)], __ldg(&A.w4[k]));
     s0[k] = c.x;
     s1[k] = c.y;
   }
 }
 
-// Pass B, warp form: kP column pairs per block (2 kP adjacent columns; 32-byte
-// row segments at kP = 4) and two warps per pair: warp (q, 0) takes the
-// forward transform and the spectral solve of pair q, then the two inverse
-// transforms (P1 and P2) run side by side on warps (q, 0) and (q, 1).
-template <int N>
-struct ColsShape {
-  static constexpr int kP = N == 1024 ? 4 : 2;          // column pairs per block
-  static constexpr int kThreads = 64 * kP;
-  static constexpr int kH = kP / 2;                     // float4 segments per row
-};
+// Pass B, group form: kP column pairs per block (2 kP adjacent columns; row
+// segments of 32 bytes at kP = 4, 16 at 2) and two groups per pair: group
+// (q, 0) takes the forward transform of pair q, both form the spectrum and
+// the inputs of the two inverse transforms (elements k and n - k by one lane,
+// in place), which run side by side on groups (q, 0) and (q, 1).
+template <int N, int kP>
+constexpr size_t cols_bytes() { return (size_t)2 * kP * GroupFft<N>::kBuf * 4 + N * 8; }
 
-template <int N>
-__global__ void __launch_bounds__(ColsShape<N>::kThreads) k_poisson_cols_w(PassBArgs B) {
+// phi^ of a packed column pair (u, u + 1) at row v from Z at v and n - v
+// (src/fft.cpp:117-166)
+__device__ __forceinline__ float2 solve_pair(const PassBArgs& B, float2 z, float2 zn, float2 w4, float2 wx, float wyv,
+                                             int u, int v) {
+  const float2 a = dct2_post(z, zn, w4);
+  float out[2];
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    float d = h ? a.y : a.x;
+    if (u + h == 0) d *= 0.5f;
+    if (v == 0) d *= 0.5f;
+    d *= B.scale;
+    const float wxu = h ? wx.y : wx.x;
+    const float den = __fadd_rn(__fmul_rn(wxu, wxu), __fmul_rn(wyv, wyv));
+    out[h] = (u + h != 0 || v != 0) ? __fdiv_rn(d, den) : 0.0f;
+  }
+  return make_float2(out[0], out[1]);
+}
+
+template <int N, int kP>
+__global__ void __launch_bounds__(2 * kP * GroupFft<N>::kG) k_poisson_cols_g(PassBArgs B) {
   extern __shared__ float2 smem[];
-  constexpr int kP = ColsShape<N>::kP, kT = ColsShape<N>::kThreads, kH = ColsShape<N>::kH;
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  const int q = w >> 1, role = w & 1;
-  constexpr int kBufF2 = WarpFft<N>::kBuf / 2;
-  // [pair][role] FFT buffers, [pair] spectra, then the tables
-  float2* buf = smem + (size_t)w * kBufF2;
-  float2* spc = smem + (size_t)2 * kP * kBufF2 + (size_t)q * N;
-  float2* w4s = smem + (size_t)kP * (2 * kBufF2 + N);    // [n] w4 (y)
-  float2* tws = w4s + N;                                 // [n] twiddles
-  float* wys = reinterpret_cast<float*>(tws + N);        // [n] wy
-  const int u_base = blockIdx.x * 2 * kP;
+  using F = GroupFft<N>;
+  constexpr int G = F::kG, kT = 2 * kP * G, kH = kP / 2;
+  constexpr int kBufF2 = F::kBuf / 2;
+  // groups: role-major, so that a warp's groups have one role
+  const int g = threadIdx.x / G, l = threadIdx.x & (G - 1);
+  const int role = g / kP, q = g % kP;
+  float2* buf0 = smem + (size_t)q * kBufF2;                       // forward, then P1
+  float2* buf1 = smem + (size_t)(kP + q) * kBufF2;                // P2
+  float2* tws = smem + (size_t)2 * kP * kBufF2;                   // [n] twiddles
+  const int u_base = blockIdx.x * 2 * kP, u = u_base + 2 * q;
   const int nx = B.nx;
-  // inputs: 8-byte copies of column pairs into the pairs' role-0 buffers
-  // (Makhoul order), and the block's tables
+  // inputs: 8-byte copies of column pairs into the pairs' first buffers
+  // (Makhoul order), and the twiddles
   for (int idx = threadIdx.x; idx < N * kP; idx += kT) {
     const int v = idx / kP, c = idx % kP;       // row v, pair c
-    cp_async8(smem + (size_t)(2 * c) * kBufF2 + makhoul_pos(v, N), B.spec + (size_t)v * nx + u_base + 2 * c);
+    cp_async8(smem + (size_t)c * kBufF2 + makhoul_pos(v, N), B.spec + (size_t)v * nx + u_base + 2 * c);
   }
-  for (int t = 4 * threadIdx.x; t < 2 * N; t += 4 * kT) {
-    cp_async16(reinterpret_cast<float*>(w4s) + t, reinterpret_cast<const float*>(B.w4) + t);
-    cp_async16(reinterpret_cast<float*>(tws) + t, reinterpret_cast<const float*>(tw_table<N>()) + t);
-  }
-  for (int t = 4 * threadIdx.x; t < N; t += 4 * kT) cp_async16(wys + t, B.wy + t);
-  const float wx0 = __ldg(&B.wx[u_base + 2 * q]), wx1 = __ldg(&B.wx[u_base + 2 * q + 1]);
+  block_copy_async(reinterpret_cast<float*>(tws), reinterpret_cast<const float*>(tw_table<N>()), 2 * N);
+  const float2 wx = make_float2(__ldg(&B.wx[u]), __ldg(&B.wx[u + 1]));
   cp_async_wait_all();
   __syncthreads();
-  if (role == 0) {
-    warp_fft<N, -1>(buf, tws);
-    // DCT-II along y, then the spectral solve (src/fft.cpp:117-166)
-#pragma unroll 4
-    for (int j = 0; j < N / 32; j++) {
-      const int v = l + 32 * j;
-      const float2 a = dct2_post(buf[v], buf[(N - v) & (N - 1)], w4s[v]);
-      const float wyv = wys[v];
-      float out[2];
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int u = u_base + 2 * q + h;
-        float d = h ? a.y : a.x;
-        if (u == 0) d *= 0.5f;
-        if (v == 0) d *= 0.5f;
-        d *= B.scale;
-        float ph = 0.0f;
-        if (u != 0 || v != 0) {
-          const float wxu = h ? wx1 : wx0;
-          ph = __fdiv_rn(d, __fadd_rn(__fmul_rn(wxu, wxu), __fmul_rn(wyv, wyv)));
-        }
-        out[h] = ph;
-      }
-      spc[v] = make_float2(out[0], out[1]);
-    }
+  if (role == 0) group_fft<N, -1>(buf0, tws);
+  __syncthreads();
+  // spectrum, then P1 = IDCT_y(phi^) and P2 = IDST_y(wy phi^), a DCT-III of
+  // b[k] = wy[n-k] phi^[n-k] (b[0] = 0): rows k and n - k of the pair
+#pragma unroll 2
+  for (int k = role * G + l; k < N / 2; k += 2 * G) {
+    const int m = k ? N - k : N / 2;            // (0 and n / 2 stand alone)
+    const float2 zk = buf0[k], zm = buf0[m];
+    const float2 w4k = __ldg(&B.w4[k]), w4m = __ldg(&B.w4[m]);
+    const float wk = __ldg(&B.wy[k]), wm = __ldg(&B.wy[m]);
+    const float2 pk = solve_pair(B, zk, k ? zm : zk, w4k, wx, wk, u, k);
+    const float2 pm = solve_pair(B, zm, k ? zk : zm, w4m, wx, wm, u, m);
+    const float2 sk = make_float2(__fmul_rn(pk.x, wk), __fmul_rn(pk.y, wk));
+    const float2 sm = make_float2(__fmul_rn(pm.x, wm), __fmul_rn(pm.y, wm));
+    buf0[k] = pre_pair(pk, pm, w4k, k);
+    buf0[m] = pre_pair(pm, k ? pk : pm, w4m, m);
+    buf1[k] = k ? pre_pair(sm, sk, w4k, k) : make_float2(0.0f, 0.0f);
+    buf1[m] = pre_pair(k ? sk : sm, sm, w4m, m);
   }
   __syncthreads();
-  if (role == 0) {
-    // P1 = IDCT_y(phi^) of both columns (one complex inverse FFT)
-#pragma unroll 4
-    for (int j = 0; j < N / 32; j++) {
-      const int k = l + 32 * j;
-      const float2 w4 = w4s[k];
-      const float2 ak = spc[k], ank = k ? spc[N - k] : make_float2(0.f, 0.f);
-      const float2 c0 = dct3_pre(ak.x, ank.x, w4, k);
-      const float2 c1 = dct3_pre(ak.y, ank.y, w4, k);
-      buf[k] = make_float2(c0.x - c1.y, c0.y + c1.x);
-    }
-  } else {
-    // P2 = IDST_y(wy * phi^): DCT-III of b[k] = wy[n-k] phi^[n-k] (b[0] = 0)
-#pragma unroll 4
-    for (int j = 0; j < N / 32; j++) {
-      const int k = l + 32 * j;
-      const float2 w4 = w4s[k];
-      float2 bk = make_float2(0.f, 0.f), bnk = make_float2(0.f, 0.f);
-      if (k) {
-        const float wa = wys[N - k];
-        const float2 a = spc[N - k];
-        bk = make_float2(__fmul_rn(a.x, wa), __fmul_rn(a.y, wa));
-        const float wb = wys[k];
-        const float2 b = spc[k];
-        bnk = make_float2(__fmul_rn(b.x, wb), __fmul_rn(b.y, wb));
-      }
-      const float2 c0 = dct3_pre(bk.x, bnk.x, w4, k);
-      const float2 c1 = dct3_pre(bk.y, bnk.y, w4, k);
-      buf[k] = make_float2(c0.x - c1.y, c0.y + c1.x);
-    }
-  }
-  __syncwarp();
-  warp_fft<N, 1>(buf, tws);
+  group_fft<N, 1>(role ? buf1 : buf0, tws);
   __syncthreads();
-  // stores: P1 from the role-0 buffers, P2 (signs alternating in v) from
-  // the role-1 buffers; a thread writes four columns (two pairs) as a float4
+  // stores: P1 from the first buffers, P2 (signs alternating in v) from the
+  // second ones; a thread writes four columns (two pairs) as a float4
   for (int idx = threadIdx.x; idx < N * kH * 2; idx += kT) {
     const int h = idx % kH, out = (idx / kH) & 1, v = idx / (2 * kH);
     const int m = makhoul_pos(v, N);
-    const float2* b0 = smem + (size_t)(2 * (2 * h) + out) * kBufF2;   // pair 2h, role out
-    const float2* b1 = b0 + 2 * kBufF2;                               // pair 2h + 1
-    const float2 x0 = b0[m], x1 = b1[m];
+    const float2* b0 = smem + (size_t)(out * kP + 2 * h) * kBufF2;    // pair 2h
+    const float2 x0 = b0[m], x1 = b0[kBufF2 + m];
     const float sg = (out && (v & 1)) ? -1.0f : 1.0f;
     float* dst = out ? B.p2 : B.p1;
     *reinterpret_cast<float4*>(dst + (size_t)v * nx + u_base + 4 * h) =
@@ -865,77 +878,73 @@ __global__ void __launch_bounds__(ColsShape<N>::kThreads) k_poisson_cols_w(PassB
   }
 }
 
-// Pass C, warp form: two row pairs per block and one warp per transform of
-// a pair (Ex = IDST_x(wx * P1), Ey = IDCT_x(P2), phi = IDCT_x(P1)); the
-// block writes the field (Ex, Ey per bin) once all transforms are done.
-constexpr int kWFieldPairs = 2;
-constexpr int kWFieldThreads = 96 * kWFieldPairs;
+// Pass C, group form: kP row pairs per block and one group per transform of a
+// pair (Ex = IDST_x(wx * P1), Ey = IDCT_x(P2) and, where it is wanted, phi =
+// IDCT_x(P1)); the block writes the field (Ex, Ey per bin) once all
+// transforms are done.
+template <int N>
+struct FieldShape {
+  static constexpr int kP = N == 2048 ? 1 : N == 256 ? 4 : 2;
+  static constexpr int threads(int roles) { return roles * kP * GroupFft<N>::kG; }
+  static constexpr size_t bytes(int roles) { return (size_t)roles * kP * GroupFft<N>::kBuf * 4 + N * 8; }
+};
 
 template <int N>
-__global__ void __launch_bounds__(kWFieldThreads) k_poisson_field_w(PassCArgs C) {
+__global__ void __launch_bounds__(FieldShape<N>::threads(3)) k_poisson_field_g(PassCArgs C) {
   extern __shared__ float2 smem[];
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  const int p = w / 3, role = w % 3;            // role 0 Ex, 1 Ey, 2 phi
-  constexpr int kBufF2 = WarpFft<N>::kBuf / 2;
-  float2* buf = smem + (size_t)w * kBufF2;
-  float* rows_all = reinterpret_cast<float*>(smem + (size_t)3 * kWFieldPairs * kBufF2);  // [pair][4][n]
-  float2* w4s = reinterpret_cast<float2*>(rows_all + (size_t)kWFieldPairs * 4 * N);
-  float2* tws = w4s + N;
-  float* wxs = reinterpret_cast<float*>(tws + N);
-  const int r0 = blockIdx.x * kWFieldPairs;
-  // inputs: P1 and P2 rows of both pairs (contiguous per array), tables
+  using F = GroupFft<N>;
+  constexpr int G = F::kG, kP = FieldShape<N>::kP;
+  constexpr int kBufF2 = F::kBuf / 2;
+  const int g = threadIdx.x / G, l = threadIdx.x & (G - 1);
+  const int role = g / kP, p = g % kP;          // role 0 Ex, 1 Ey, 2 phi
+  float2* buf = smem + (size_t)g * kBufF2;
+  float2* tws = smem + (size_t)(blockDim.x / G) * kBufF2;
+  const int r0 = blockIdx.x * kP;
+  block_copy_async(reinterpret_cast<float*>(tws), reinterpret_cast<const float*>(tw_table<N>()), 2 * N);
   {
-    const size_t base = (size_t)(2 * r0) * N;
-    const int n = 2 * N * kWFieldPairs;       // floats per array
-    for (int t = 4 * threadIdx.x; t < n; t += 4 * kWFieldThreads) {
-      const int pp = t / (2 * N), o = t - pp * 2 * N;
-      cp_async16(rows_all + (size_t)pp * 4 * N + o, C.p1 + base + t);
-      cp_async16(rows_all + (size_t)pp * 4 * N + 2 * N + o, C.p2 + base + t);
+    const float* __restrict__ a0 = (role == 1 ? C.p2 : C.p1) + (size_t)(2 * (r0 + p)) * N;
+    const float* __restrict__ a1 = a0 + N;
+    constexpr int U = 4;                        // element pairs in flight per lane
+    for (int k0 = l; k0 < N / 2; k0 += U * G) {
+      float2 xk[U], xm[U], w4k[U], w4m[U];
+      float wk[U], wm[U];
+#pragma unroll
+      for (int j = 0; j < U; j++) {
+        const int k = k0 + j * G, m = k ? N - k : N / 2;
+        xk[j] = make_float2(__ldg(a0 + k), __ldg(a1 + k));
+        xm[j] = make_float2(__ldg(a0 + m), __ldg(a1 + m));
+        w4k[j] = __ldg(&C.w4[k]);
+        w4m[j] = __ldg(&C.w4[m]);
+        if (role == 0) { wk[j] = __ldg(&C.wx[k]); wm[j] = __ldg(&C.wx[m]); }
+      }
+#pragma unroll
+      for (int j = 0; j < U; j++) {
+        const int k = k0 + j * G, m = k ? N - k : N / 2;
+        if (role != 0) {
+          buf[k] = pre_pair(xk[j], xm[j], w4k[j], k);
+          buf[m] = pre_pair(xm[j], k ? xk[j] : xm[j], w4m[j], m);
+        } else {
+          // b[k] = wx[n-k] a[n-k] for k >= 1, b[0] = 0
+          const float2 sk = make_float2(__fmul_rn(xk[j].x, wk[j]), __fmul_rn(xk[j].y, wk[j]));
+          const float2 sm = make_float2(__fmul_rn(xm[j].x, wm[j]), __fmul_rn(xm[j].y, wm[j]));
+          buf[k] = k ? pre_pair(sm, sk, w4k[j], k) : make_float2(0.0f, 0.0f);
+          buf[m] = pre_pair(k ? sk : sm, sm, w4m[j], m);
+        }
+      }
     }
-    for (int t = 4 * threadIdx.x; t < 2 * N; t += 4 * kWFieldThreads) {
-      cp_async16(reinterpret_cast<float*>(w4s) + t, reinterpret_cast<const float*>(C.w4) + t);
-      cp_async16(reinterpret_cast<float*>(tws) + t, reinterpret_cast<const float*>(tw_table<N>()) + t);
-    }
-    for (int t = 4 * threadIdx.x; t < N; t += 4 * kWFieldThreads) cp_async16(wxs + t, C.wx + t);
   }
   cp_async_wait_all();
   __syncthreads();
-  const float* rows = rows_all + (size_t)p * 4 * N;
-  if (role != 2 || C.phi) {
-    const float* a0 = rows + (role == 1 ? 2 : 0) * N;
-    const float* a1 = a0 + N;
-#pragma unroll 4
-    for (int j = 0; j < N / 32; j++) {
-      const int k = l + 32 * j;
-      float x0k, x0nk, x1k, x1nk;
-      if (role != 0) {
-        x0k = a0[k]; x1k = a1[k];
-        x0nk = k ? a0[N - k] : 0.f; x1nk = k ? a1[N - k] : 0.f;
-      } else if (k) {
-        // b[k] = wx[n-k] a[n-k] for k >= 1, b[0] = 0
-        const float wa = wxs[N - k], wb = wxs[k];
-        x0k = __fmul_rn(a0[N - k], wa); x1k = __fmul_rn(a1[N - k], wa);
-        x0nk = __fmul_rn(a0[k], wb); x1nk = __fmul_rn(a1[k], wb);
-      } else {
-        x0k = x1k = x0nk = x1nk = 0.f;
-      }
-      const float2 w4 = w4s[k];
-      const float2 c0 = dct3_pre(x0k, x0nk, w4, k);
-      const float2 c1 = dct3_pre(x1k, x1nk, w4, k);
-      buf[k] = make_float2(c0.x - c1.y, c0.y + c1.x);
-    }
-    __syncwarp();
-    warp_fft<N, 1>(buf, tws);
-  }
+  group_fft<N, 1>(buf, tws);
   __syncthreads();
-  // outputs, bin m of rows 2r and 2r + 1 of both pairs (IDST signs alternate)
-  for (int idx = threadIdx.x; idx < kWFieldPairs * N; idx += kWFieldThreads) {
+  // outputs, bin m of rows 2r and 2r + 1 of every pair (IDST signs alternate)
+  for (int idx = threadIdx.x; idx < kP * N; idx += blockDim.x) {
     const int pp = idx / N, m = idx - pp * N;
     const size_t b0 = (size_t)(2 * (r0 + pp)) * N;
     const int mp = makhoul_pos(m, N);
-    const float2* bp = smem + (size_t)(3 * pp) * kBufF2;
+    const float2* bp = smem + (size_t)pp * kBufF2;
     float2 ex = bp[mp];
-    const float2 ey = bp[kBufF2 + mp];
+    const float2 ey = bp[kP * kBufF2 + mp];
     if (m & 1) { ex.x = -ex.x; ex.y = -ex.y; }
     if (C.field) {
       C.field[b0 + m] = make_float2(ex.x, ey.x);
@@ -945,26 +954,45 @@ __global__ void __launch_bounds__(kWFieldThreads) k_poisson_field_w(PassCArgs C)
       C.fy[b0 + m] = ey.x; C.fy[b0 + N + m] = ey.y;
     }
     if (C.phi) {
-      const float2 ph = bp[2 * kBufF2 + mp];
+      const float2 ph = bp[2 * kP * kBufF2 + mp];
       C.phi[b0 + m] = ph.x; C.phi[b0 + N + m] = ph.y;
     }
   }
 }
 
-template <int N>
-constexpr size_t smem_rows_w() { return (size_t)WarpFft<N>::kBuf * 4 + 2 * N * 8; }
-template <int N>
-constexpr size_t smem_cols_w() {
-  return (size_t)ColsShape<N>::kP * (2 * WarpFft<N>::kBuf * 4 + N * 8) + 2 * N * 8 + N * 4;
-}
-template <int N>
-constexpr size_t smem_field_w() {
-  return (size_t)kWFieldPairs * (3 * WarpFft<N>::kBuf * 4 + 4 * N * 4) + 2 * N * 8 + N * 4;
+// Whether the group form takes this grid.
+bool group_form(int nx, int ny) {
+  auto in = [](int n) { return n == 256 || n == 512 || n == 1024 || n == 2048; };
+  return in(nx) && in(ny) && !(nx == 256 && ny == 256);
 }
 
-// The sequence length of the warp form for this grid, or 0 (block form).
-int warp_form(int nx, int ny) { return nx == ny && (nx == 1024 || nx == 512) ? nx : 0; }
+template <int N>
+void launch_rows_g(const PassAArgs& A, int ny, cudaStream_t s) {
+  using R = RowsShape<N>;
+  k_poisson_rows_g<N><<<ny / 2 / R::kP, R::kT, R::kBytes, s>>>(A);
+}
+template <int N>
+void launch_cols_g(const PassBArgs& B, int nx, cudaStream_t s) {
+  // 32-byte row segments where that leaves 128 blocks (most of the SMs)
+  if (nx >= 1024) k_poisson_cols_g<N, 4><<<nx / 8, 8 * GroupFft<N>::kG, cols_bytes<N, 4>(), s>>>(B);
+  else k_poisson_cols_g<N, 2><<<nx / 4, 4 * GroupFft<N>::kG, cols_bytes<N, 2>(), s>>>(B);
+}
+template <int N>
+void launch_field_g(const PassCArgs& C, int ny, cudaStream_t s) {
+  using S = FieldShape<N>;
+  const int roles = C.phi ? 3 : 2;
+  k_poisson_field_g<N><<<ny / 2 / S::kP, S::threads(roles), S::bytes(roles), s>>>(C);
+}
 
+template <int N>
+cudaError_t group_prepare() {
+  const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  cudaError_t e = cudaFuncSetAttribute(k_poisson_rows_g<N>, a, (int)RowsShape<N>::kBytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_poisson_cols_g<N, 4>, a, (int)cols_bytes<N, 4>());
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_poisson_cols_g<N, 2>, a, (int)cols_bytes<N, 2>());
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_poisson_field_g<N>, a, (int)FieldShape<N>::bytes(3));
+  return e;
+}
 
 int ilog2(int v) { int l = 0; while ((1 << l) < v) l++; return l; }
 
@@ -985,10 +1013,11 @@ size_t smem_a(int nx, int ny) { return ((size_t)2 * pairs_a(nx, ny) * nx + nx / 
 size_t smem_b(int nx, int ny) { return ((size_t)3 * pairs_b(nx, ny) * ny + ny / 2) * sizeof(float2); }
 size_t smem_c(int nx, int ny) { return ((size_t)4 * pairs_c(nx, ny) * nx + nx / 2) * sizeof(float2); }
 
-// Blocks of the density pass (one FP64 overflow partial each): the warp
-// form's grid-wide density kernel takes four bins per thread.
+// Blocks of the density pass (one FP64 overflow partial each): the group
+// form's grid-wide density kernel takes four bins per thread, more on grids
+// of over a million bins (a partial per block has to fit part_stride).
 int poisson_blocks_a(int nx, int ny) {
-  if (warp_form(nx, ny)) return nx * ny / 1024;
+  if (group_form(nx, ny)) return min(nx * ny / 1024, 1024);
   int r = pairs_a(nx, ny);
   return (ny / 2 + r - 1) / r;
 }
@@ -1006,24 +1035,25 @@ int poisson_prepare_device() {
   GPL_CUDA(cudaFuncSetAttribute(k_poisson_a, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   GPL_CUDA(cudaFuncSetAttribute(k_poisson_b, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   GPL_CUDA(cudaFuncSetAttribute(k_poisson_c, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  GPL_CUDA(cudaFuncSetAttribute(k_poisson_cols_w<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem_cols_w<1024>()));
-  GPL_CUDA(cudaFuncSetAttribute(k_poisson_field_w<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem_field_w<1024>()));
-  GPL_CUDA(cudaFuncSetAttribute(k_poisson_cols_w<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem_cols_w<512>()));
-  GPL_CUDA(cudaFuncSetAttribute(k_poisson_field_w<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem_field_w<512>()));
-  for (int n : {1024, 512}) {
-    // the warp form's twiddles, [k2 * 32 + n1] = exp(-2 pi i n1 k2 / n)
+  GPL_CUDA(group_prepare<256>());
+  GPL_CUDA(group_prepare<512>());
+  GPL_CUDA(group_prepare<1024>());
+  GPL_CUDA(group_prepare<2048>());
+  for (int n : {256, 512, 1024, 2048}) {
+    // the group form's twiddles, [k2 * G + n1] = exp(-2 pi i n1 k2 / n)
+    const int g = n == 256 ? GroupFft<256>::kG : n == 2048 ? GroupFft<2048>::kG : GroupFft<512>::kG;
+    static_assert(GroupFft<512>::kG == GroupFft<1024>::kG, "one width");
     std::vector<float2> t(n);
-    for (int k2 = 0; k2 < n / 32; k2++)
-      for (int n1 = 0; n1 < 32; n1++) {
+    for (int k2 = 0; k2 < n / g; k2++)
+      for (int n1 = 0; n1 < g; n1++) {
         const double a = -2.0 * M_PI * (double)(n1 * k2) / (double)n;
-        t[k2 * 32 + n1] = make_float2((float)cos(a), (float)sin(a));
+        t[k2 * g + n1] = make_float2((float)cos(a), (float)sin(a));
       }
-    if (n == 1024) GPL_CUDA(cudaMemcpyToSymbol(g_tw1024, t.data(), n * sizeof(float2)));
-    else GPL_CUDA(cudaMemcpyToSymbol(g_tw512, t.data(), n * sizeof(float2)));
+    const size_t bytes = n * sizeof(float2);
+    if (n == 256) GPL_CUDA(cudaMemcpyToSymbol(g_tw256, t.data(), bytes));
+    else if (n == 512) GPL_CUDA(cudaMemcpyToSymbol(g_tw512, t.data(), bytes));
+    else if (n == 1024) GPL_CUDA(cudaMemcpyToSymbol(g_tw1024, t.data(), bytes));
+    else GPL_CUDA(cudaMemcpyToSymbol(g_tw2048, t.data(), bytes));
   }
   done[dev] = true;
   return GPL_OK;
@@ -1112,7 +1142,7 @@ size_t poisson_batch_args_bytes(int pass) {
 
 bool write_poisson_batch_args(const DeviceModel& d, void* dst_a, void* dst_b, void* dst_c, int grid[3],
                               size_t smem[3]) {
-  if (d.poisson_path != 1 || warp_form(d.cnt_x, d.cnt_y)) return false;
+  if (d.poisson_path != 1 || group_form(d.cnt_x, d.cnt_y)) return false;
   const PoissonGrid g = job_grid(d);
   const PassAArgs A = pass_a_args(g, d.area, d.ctl, d.nonplace, d.target_density, nullptr, d.density,
                                   d.part + (size_t)kPartOverflow * d.part_stride, d.spec);
@@ -1161,35 +1191,34 @@ int poisson_passes(const PoissonGrid& g, unsigned long long* const* area_pair,
   if (rc) return rc;
   const int nx = g.nx, ny = g.ny;
   const PassAArgs A = pass_a_args(g, area_pair, ctl, nonplace, td, density_in, density, part_overflow, spec);
-  if (const int wn = warp_form(nx, ny)) {
+  if (group_form(nx, ny)) {
     const bool areas = area_pair && ctl;
     PassBArgs B;
-    B.nx = nx; B.ny = ny; B.logn = ilog2(ny);
+    B.nx = nx; B.ny = ny; B.logn = ilog2(ny); B.col_pairs = 0;
     B.spec = spec; B.p1 = p1; B.p2 = p2; B.wx = g.wx; B.wy = g.wy; B.tw = g.tw; B.w4 = g.w4y;
     B.scale = 4.0f / (float)nx / (float)ny;
     PassCArgs C;
-    C.nx = nx; C.ny = ny; C.logn = ilog2(nx); C.pairs_per_block = kWFieldPairs;
+    C.nx = nx; C.ny = ny; C.logn = ilog2(nx); C.pairs_per_block = 0;
     C.p1 = p1; C.p2 = p2; C.field = field; C.fx = fx; C.fy = fy; C.phi = phi;
     C.wx = g.wx; C.tw = g.tw; C.w4 = g.w4x;
     if (t) t->begin(kKPoissonA);
     if (areas) k_poisson_dens<<<poisson_blocks_a(nx, ny), 256, 0, s>>>(A);
-    if (wn == 1024) k_poisson_rows_w<1024><<<ny / 2, 32, smem_rows_w<1024>(), s>>>(A);
-    else k_poisson_rows_w<512><<<ny / 2, 32, smem_rows_w<512>(), s>>>(A);
+    if (nx == 256) launch_rows_g<256>(A, ny, s);
+    else if (nx == 512) launch_rows_g<512>(A, ny, s);
+    else if (nx == 1024) launch_rows_g<1024>(A, ny, s);
+    else launch_rows_g<2048>(A, ny, s);
     if (t) t->end(kKPoissonA);
     if (t) t->begin(kKPoissonB);
-    if (wn == 1024) {
-      B.col_pairs = ColsShape<1024>::kP;
-      k_poisson_cols_w<1024><<<nx / (2 * ColsShape<1024>::kP), ColsShape<1024>::kThreads,
-                               smem_cols_w<1024>(), s>>>(B);
-    } else {
-      B.col_pairs = ColsShape<512>::kP;
-      k_poisson_cols_w<512><<<nx / (2 * ColsShape<512>::kP), ColsShape<512>::kThreads,
-                              smem_cols_w<512>(), s>>>(B);
-    }
+    if (ny == 256) launch_cols_g<256>(B, nx, s);
+    else if (ny == 512) launch_cols_g<512>(B, nx, s);
+    else if (ny == 1024) launch_cols_g<1024>(B, nx, s);
+    else launch_cols_g<2048>(B, nx, s);
     if (t) t->end(kKPoissonB);
     if (t) t->begin(kKPoissonC);
-    if (wn == 1024) k_poisson_field_w<1024><<<ny / 2 / kWFieldPairs, kWFieldThreads, smem_field_w<1024>(), s>>>(C);
-    else k_poisson_field_w<512><<<ny / 2 / kWFieldPairs, kWFieldThreads, smem_field_w<512>(), s>>>(C);
+    if (nx == 256) launch_field_g<256>(C, ny, s);
+    else if (nx == 512) launch_field_g<512>(C, ny, s);
+    else if (nx == 1024) launch_field_g<1024>(C, ny, s);
+    else launch_field_g<2048>(C, ny, s);
     if (t) t->end(kKPoissonC);
     if (t) t->count(areas ? 4 : 3);
     GPL_CUDA(cudaGetLastError());
