@@ -23,21 +23,20 @@ namespace gpl {
 namespace {
 
 constexpr int kBlock = 256;
-constexpr int kBigBins = 64;          // cells covering more bins go to the big-cell kernels
 constexpr int kCellBlocksPerSm = 6;   // the gcell kernel's residency (40 registers, a few spilled)
 
 struct ScatterArgs {
   BinGeom geo;
   int n_g;
   float td;
-  const int2* half;
-  const float* scale;
-  const uint8_t* kind;
+  const int4* geo_g;            // per gcell (GCellGeo)
   float2* slp[4];
   float2* sum[4];
   float2* coordi[2];
   unsigned long long* area[2];  // two sets of inst [nb], filler [nb]
   const EvalCtl* ctl;
+  int one_word;                 // a window's sums fit 32 bits (scatter_one_word)
+  int fits32;                   // so does every single value
 };
 
 __device__ __forceinline__ float2 predict_one(const ScatterArgs& A, const EvalCtl& C, int g, int2 h) {
@@ -83,8 +82,8 @@ struct OrderArgs {
 
 __device__ __forceinline__ int tile_of(const OrderArgs& O, float2 c) {
   const BinGeom& G = O.geo;
-  const int bx = min(max((__float2int_rz(c.x) - G.core_lx) / G.size_x, 0), G.cnt_x - 1);
-  const int by = min(max((__float2int_rz(c.y) - G.core_ly) / G.size_y, 0), G.cnt_y - 1);
+  const int bx = min(G.div_x(max(__float2int_rz(c.x) - G.core_lx, 0)), G.cnt_x - 1);
+  const int by = min(G.div_y(max(__float2int_rz(c.y) - G.core_ly, 0)), G.cnt_y - 1);
   return (by / O.tile_h) * O.tiles_x + bx / O.tile_w;
 }
 
@@ -132,7 +131,13 @@ __global__ void __launch_bounds__(kOrderScanT) k_order_scan(OrderArgs O) {
     const int c = O.tile_count[t];
     O.tile_start[t] = at;
     O.tile_count[t] = at;
-    for (int f = 0; f < c; f += O.chunk) O.chunks[ck++] = make_int4(t, at + f, at + min(f + O.chunk, c), 0);
+    // equal chunks: a short last one would cost a block's window all the same
+    const int n_ch = (c + O.chunk - 1) / O.chunk;
+    for (int f = 0, k = 0; k < n_ch; k++) {
+      const int e = (int)(((long long)c * (k + 1)) / n_ch);
+      O.chunks[ck++] = make_int4(t, at + f, at + e, 0);
+      f = e;
+    }
     at += c;
   }
   if (threadIdx.x == kOrderScanT - 1) {
@@ -156,6 +161,7 @@ __global__ void __launch_bounds__(kBlock) k_order_fill(OrderArgs O) {
 
 struct TileArgs {
   int tile_w, tile_h, tiles_x;
+  FastDiv div_wx;               // by the window's width
   const int32_t* order;
   const int4* chunks;
   const int32_t* n_chunks;
@@ -168,6 +174,16 @@ struct TileArgs {
 // every gcell (big ones included; their bins are left to k_scatter_big).
 // The body of one block (chunk vb); `win` is the block's dynamic shared
 // window.  Shared by the per-job launch and the batched one.
+//
+// What bounds it is instruction issue (60 % of the slots at a million cells),
+// so: bin ranges by multiplication (FastDiv), a gcell's overlap widths once
+// per column and row, its up to 3 x 3 bins without loops or range tests when
+// they lie inside the window, and one 32-bit window word per bin where the
+// chunk's sums cannot pass 2^32 (two 16-bit halves in two words otherwise).
+// 12.5k gcells 17.5 -> 9.8 us, 250k with 40 macros 28.9 -> 24, 1.25M 64.0 ->
+// 42.8 (in the loop, events around the launch); a 1024-gcell block used to
+// run 1800 instructions a warp of gcells.
+template <bool kOneWord>
 __device__ __forceinline__ void scatter_body(const ScatterArgs& A, const TileArgs& T, int vb, unsigned* win) {
   if (vb >= *T.n_chunks) return;                   // block-uniform
   const EvalCtl C = *A.ctl;
@@ -175,57 +191,86 @@ __device__ __forceinline__ void scatter_body(const ScatterArgs& A, const TileArg
   const BinGeom& G = A.geo;
   const int nb = G.cnt_x * G.cnt_y;
   const int4 ch = T.chunks[vb];
-  const int ox = (ch.x % T.tiles_x) * T.tile_w - kTileMargin;
-  const int oy = (ch.x / T.tiles_x) * T.tile_h - kTileMargin;
+  const int tile_y = ch.x / T.tiles_x, tile_x = ch.x - tile_y * T.tiles_x;
+  const int ox = tile_x * T.tile_w - kTileMargin;
+  const int oy = tile_y * T.tile_h - kTileMargin;
   const int wx = T.tile_w + 2 * kTileMargin, wy = T.tile_h + 2 * kTileMargin, wn = wx * wy;
-  unsigned* win_hi = win + 2 * wn;
-  for (int i = threadIdx.x; i < 4 * wn; i += blockDim.x) win[i] = 0u;
+  unsigned* win_hi = win + 2 * wn;                 // (two-word form)
+  constexpr int kWords = kOneWord ? 2 : 4;
+  // (wn is even, the window 16-byte aligned)
+  for (int i = threadIdx.x; i < kWords * wn / 4; i += blockDim.x) reinterpret_cast<uint4*>(win)[i] = make_uint4(0u, 0u, 0u, 0u);
   __syncthreads();
+  // adds v at window index i: the sums return nothing and neither word can
+  // wrap (one word: see scatter_one_word; two: a chunk has fewer than 2^16
+  // gcells, one addition of a 16-bit half each per bin)
+  auto add = [&](int i, unsigned v) {
+    if (v == 0u) return;
+    if constexpr (kOneWord) {
+      atomicAdd(&win[i], v);
+    } else {
+      atomicAdd(&win[i], v & 0xffffu);
+      atomicAdd(&win_hi[i], v >> 16);
+    }
+  };
   for (int idx = ch.y + threadIdx.x; idx < ch.z; idx += blockDim.x) {
     const int g = T.order[idx];
-    const int2 h = A.half[g];
-    const float2 c = C.predict ? predict_one(A, C, g, h) : pick4(A.slp, C.i_eval)[g];
-    const int k = A.kind[g];
-    if (k & 4) continue;                           // big cell: k_scatter_big
+    const GCellGeo q = gcell_geo(A.geo_g[g]);
+    const float2 c = C.predict ? predict_one(A, C, g, q.half) : pick4(A.slp, C.i_eval)[g];
+    if (q.big()) continue;                         // k_scatter_big
     int lx, ux, ly, uy, x0, x1, y0, y1;
-    density_rect(c, h, lx, ux, ly, uy);
+    density_rect(c, q.half, lx, ux, ly, uy);
     G.range(lx, ux, ly, uy, x0, x1, y0, y1);
-    const float sc = A.scale[g];
-    const int half = (k & 3) == 2 ? 1 : 0;
+    const int half = q.type() == 2 ? 1 : 0;
+    const bool macro = q.type() == 1;              // scaled down by the target density
+    const int u0 = x0 - ox, w0 = y0 - oy;
+    const int nx = x1 - x0, ny = y1 - y0;
+    if (A.fits32 && q.scale <= 1.0f && nx <= 3 && ny <= 3 && u0 >= 0 && u0 + nx <= wx && w0 >= 0 && w0 + ny <= wy) {
+      float fx[3], fy[3];
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        fx[k] = k < nx ? G.overlap_x(x0 + k, lx, ux) : 0.0f;
+        fy[k] = k < ny ? G.overlap_y(y0 + k, ly, uy) : 0.0f;
+      }
+      const int i0 = half * wn + w0 * wx + u0;
+#pragma unroll
+      for (int r = 0; r < 3; r++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+          float f = __fmul_rn(__fmul_rn(fx[k], fy[r]), q.scale);
+          if (macro) f = __fmul_rn(f, A.td);
+          add(i0 + r * wx + k, __float2uint_rz(f));
+        }
+      continue;
+    }
     for (int cc = y0; cc < y1; cc++) {
       for (int a = x0; a < x1; a++) {
-        const float ov = G.overlap(a, cc, lx, ux, ly, uy);
-        float f = __fmul_rn(ov, sc);
-        if ((k & 3) == 1) f = __fmul_rn(f, A.td);          // macro: scale down by target density
+        float f = __fmul_rn(G.overlap(a, cc, lx, ux, ly, uy), q.scale);
+        if (macro) f = __fmul_rn(f, A.td);
         const unsigned long long v = trunc_u64(f);
         if (!v) continue;
         const int u = a - ox, w = cc - oy;
-        if (u >= 0 && u < wx && w >= 0 && w < wy && v < (1ull << 32)) {
-          // v < 2^32 split into 16-bit halves added to two 32-bit words: a
-          // chunk has fewer than 2^16 gcells (set_scatter_shape), one addition
-          // each per bin, so neither word can wrap; the adds return nothing
-          const int i = half * wn + w * wx + u;
-          atomicAdd(&win[i], (unsigned)(v & 0xffffu));
-          atomicAdd(&win_hi[i], (unsigned)(v >> 16));
-        } else {
-          atomicAdd(&area[half * nb + cc * G.cnt_x + a], v);
-        }
+        if (A.fits32 && q.scale <= 1.0f && u >= 0 && u < wx && w >= 0 && w < wy) add(half * wn + w * wx + u, (unsigned)v);
+        else atomicAdd(&area[half * nb + cc * G.cnt_x + a], v);
       }
     }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < 2 * wn; i += blockDim.x) {
-    const unsigned long long v = (unsigned long long)win[i] + ((unsigned long long)win_hi[i] << 16);
+    unsigned long long v = win[i];
+    if constexpr (!kOneWord) v += (unsigned long long)win_hi[i] << 16;
     if (!v) continue;
     const int half = i >= wn ? 1 : 0, r = i - half * wn;
-    const int a = ox + r % wx, cc = oy + r / wx;      // inside the grid: only in-grid bins were added
+    const int w = T.div_wx(r);
+    const int a = ox + r - w * wx, cc = oy + w;       // inside the grid: only in-grid bins were added
     atomicAdd(&area[half * nb + cc * G.cnt_x + a], v);
   }
 }
 
-__global__ void __launch_bounds__(kBlock, 5) k_scatter(ScatterArgs A, TileArgs T) {
-  extern __shared__ unsigned win[];                // [2][wy][wx] low 16-bit sums, then high 16-bit sums
-  scatter_body(A, T, (int)blockIdx.x, win);
+template <bool kOneWord>
+__global__ void __launch_bounds__(kBlock, 5) k_scatter(const __grid_constant__ ScatterArgs A,
+                                                       const __grid_constant__ TileArgs T) {
+  extern __shared__ __align__(16) unsigned win[];  // [words][2][wy][wx]: sums, or low 16-bit then high 16-bit sums
+  scatter_body<kOneWord>(A, T, (int)blockIdx.x, win);
 }
 
 // One block per big cell (macros): threads stride over its bins.
@@ -235,7 +280,8 @@ __device__ __forceinline__ void scatter_big_body(const ScatterArgs& A, const int
   const int g = big[vb];
   const BinGeom& G = A.geo;
   const int nb = G.cnt_x * G.cnt_y;
-  const int2 h = A.half[g];
+  const GCellGeo geo = gcell_geo(A.geo_g[g]);
+  const int2 h = geo.half;
   // k_scatter has already written this cell's predicted coordinates; the
   // block recomputes them with the same arithmetic instead of reading them
   float2 c;
@@ -252,8 +298,8 @@ __device__ __forceinline__ void scatter_big_body(const ScatterArgs& A, const int
   G.range(lx, ux, ly, uy, x0, x1, y0, y1);
   if (x1 <= x0 || y1 <= y0) return;
   const int nbx = x1 - x0, total = nbx * (y1 - y0);
-  const int k = A.kind[g];
-  const float sc = A.scale[g];
+  const int k = geo.kind;
+  const float sc = geo.scale;
   for (int t = threadIdx.x; t < total; t += blockDim.x) {
     const int a = x0 + t % nbx, cc = y0 + t / nbx;
     float f = __fmul_rn(G.overlap(a, cc, lx, ux, ly, uy), sc);
@@ -270,9 +316,7 @@ __global__ void __launch_bounds__(kBlock) k_scatter_big(ScatterArgs A, const int
 struct CellArgs {
   BinGeom geo;
   int n_g;
-  const int2* half;
-  const float* scale;
-  const uint8_t* kind;
+  const int4* geo_g;          // per gcell (GCellGeo)
   float2* slp[4];
   float2* sum[4];
   const EvalCtl* ctl;
@@ -280,8 +324,7 @@ struct CellArgs {
   const int32_t* g_pin_start;
   const int32_t* g_pins;      // device pin index of each gcell pin slot
   const float2* pin_grad;     // device pin order
-  const float2* precond;      // (#pins, dx*dy)
-  const int32_t* big_idx;
+  const float* area_g;        // dx*dy of each gcell (the pin count comes from its slots)
   float2* d_big;
   float min_precond;
   float2* wl_out;
@@ -302,10 +345,11 @@ __device__ __forceinline__ void dgrad_big_body(const CellArgs& A, const int32_t*
   const BinGeom& G = A.geo;
   const EvalCtl C = *A.ctl;
   int lx, ux, ly, uy, x0, x1, y0, y1;
-  density_rect(pick4(A.slp, C.i_eval)[g], A.half[g], lx, ux, ly, uy);
+  const GCellGeo geo = gcell_geo(A.geo_g[g]);
+  density_rect(pick4(A.slp, C.i_eval)[g], geo.half, lx, ux, ly, uy);
   G.range(lx, ux, ly, uy, x0, x1, y0, y1);
   const int nbx = max(x1 - x0, 0), total = nbx * max(y1 - y0, 0);
-  const float sc = A.scale[g];
+  const float sc = geo.scale;
   float ex = 0.0f, ey = 0.0f;
   for (int t = threadIdx.x; t < total; t += blockDim.x) {
     const int a = x0 + t % nbx, cc = y0 + t / nbx;
@@ -354,10 +398,8 @@ __device__ __forceinline__ void cell_body(const CellArgs& A, int vb, int vgrid) 
   const int32_t* __restrict__ g_pins = A.g_pins;
   const int32_t* __restrict__ g_pin_start = A.g_pin_start;
   const float2* __restrict__ field = A.field;
-  const int2* __restrict__ half = A.half;
-  const uint8_t* __restrict__ kind = A.kind;
-  const float* __restrict__ scale = A.scale;
-  const float2* __restrict__ precond = A.precond;
+  const int4* __restrict__ geo_g = A.geo_g;
+  const float* __restrict__ area_g = A.area_g;
   const float lam = C.density_penalty;
   const int lane = threadIdx.x & 31;
   // warp-uniform grid-stride loop: the warps gather the pins of cells with
@@ -410,16 +452,16 @@ __device__ __forceinline__ void cell_body(const CellArgs& A, int vb, int vgrid) 
     }
     if (!valid) continue;
     const float2 c = slp[g];
-    const int k = kind[g];
+    const GCellGeo geo = gcell_geo(geo_g[g]);
     // density gradient: sum over covered bins of overlap * scale * field
     float2 d = make_float2(0.0f, 0.0f);
-    if (k & 4) {
-      d = A.d_big[A.big_idx[g]];
+    if (geo.big()) {
+      d = A.d_big[geo.big_index()];
     } else {
       int lx, ux, ly, uy, x0, x1, y0, y1;
-      density_rect(c, half[g], lx, ux, ly, uy);
+      density_rect(c, geo.half, lx, ux, ly, uy);
       G.range(lx, ux, ly, uy, x0, x1, y0, y1);
-      const float sc = scale[g];
+      const float sc = geo.scale;
       for (int a = x0; a < x1; a++) {
         for (int cc = y0; cc < y1; cc++) {
           const float ov = __fmul_rn(G.overlap(a, cc, lx, ux, ly, uy), sc);
@@ -430,8 +472,8 @@ __device__ __forceinline__ void cell_body(const CellArgs& A, int vb, int vgrid) 
       }
     }
     float2 s = make_float2(__fadd_rn(w.x, __fmul_rn(lam, d.x)), __fadd_rn(w.y, __fmul_rn(lam, d.y)));
-    const float2 pc = precond[g];
-    float px = __fadd_rn(pc.x, __fmul_rn(lam, pc.y));
+    // getWireLengthPreconditioner / getDensityPreconditioner (src/nesterovBase.cpp:1442-1454)
+    float px = __fadd_rn((float)(pe - ps), __fmul_rn(lam, area_g[g]));
     float py = px;
     if (px <= A.min_precond) px = A.min_precond;
     if (py <= A.min_precond) py = A.min_precond;
@@ -548,6 +590,7 @@ BinGeom geom(const DeviceModel& d) {
   BinGeom G;
   G.core_lx = d.core_lx; G.core_ly = d.core_ly; G.core_ux = d.core_ux; G.core_uy = d.core_uy;
   G.size_x = d.size_x; G.size_y = d.size_y; G.cnt_x = d.cnt_x; G.cnt_y = d.cnt_y;
+  G.div_x = FastDiv(d.size_x); G.div_y = FastDiv(d.size_y);
   return G;
 }
 
@@ -556,12 +599,22 @@ BinGeom geom(const DeviceModel& d) {
 int cell_blocks(const DeviceModel& d) { return (d.n_g + kBlock - 1) / kBlock; }
 
 namespace {
+// The largest value a gcell of scale at most 1 adds to a bin, as the float
+// product rounds (the factors are at most the bin's sides).
+double scatter_max_value(const DeviceModel& d) {
+  return 1.000001 * (double)d.size_x * (double)d.size_y * std::max(1.0, (double)d.target_density);
+}
+// One window word per bin: a chunk adds at most `piece` values to it.
+bool scatter_one_word(const DeviceModel& d) { return scatter_max_value(d) * d.piece < 4294967295.0; }
+
 ScatterArgs scatter_args(const DeviceModel& d) {
   ScatterArgs A;
   A.geo = geom(d);
   A.n_g = d.n_g;
   A.td = d.target_density;
-  A.half = d.g_half; A.scale = d.g_scale; A.kind = d.g_kind;
+  A.geo_g = d.g_geo;
+  A.one_word = scatter_one_word(d) ? 1 : 0;
+  A.fits32 = scatter_max_value(d) < 4294967295.0 ? 1 : 0;
   for (int k = 0; k < 4; k++) { A.slp[k] = d.slp[k]; A.sum[k] = d.sum[k]; }
   A.coordi[0] = d.coordi[0]; A.coordi[1] = d.coordi[1];
   A.area[0] = d.area[0]; A.area[1] = d.area[1];
@@ -572,6 +625,7 @@ ScatterArgs scatter_args(const DeviceModel& d) {
 TileArgs tile_args(const DeviceModel& d) {
   TileArgs T;
   T.tile_w = d.tile_w; T.tile_h = d.tile_h; T.tiles_x = d.tiles_x;
+  T.div_wx = FastDiv(d.tile_w + 2 * kTileMargin);
   T.order = d.order; T.chunks = d.chunks; T.n_chunks = d.n_chunks;
   return T;
 }
@@ -580,15 +634,15 @@ CellArgs cell_args(const DeviceModel& d, const EvalArgs& a, int n_phi_blocks) {
   CellArgs A;
   A.geo = geom(d);
   A.n_g = d.n_g;
-  A.half = d.g_half; A.scale = d.g_scale; A.kind = d.g_kind;
+  A.geo_g = d.g_geo;
   for (int k = 0; k < 4; k++) { A.slp[k] = d.slp[k]; A.sum[k] = d.sum[k]; }
   A.ctl = d.ctl;
   A.field = d.field;
   A.g_pin_start = d.g_pin_start;
   A.g_pins = d.g_pins;
   A.pin_grad = d.pin_grad;
-  A.precond = d.g_precond;
-  A.big_idx = d.g_big_idx; A.d_big = d.d_big;
+  A.area_g = d.g_area;
+  A.d_big = d.d_big;
   A.min_precond = a.min_precond;
   A.wl_out = d.wl_out; A.d_out = d.d_out;
   A.part = d.part;
@@ -608,7 +662,8 @@ int launch_scatter(DeviceModel& d, const EvalArgs& a, cudaStream_t s, Timer& t) 
   const TileArgs T = tile_args(d);
   (void)a;
   t.begin(kKScatter);
-  k_scatter<<<d.max_chunks, kBlock, scatter_smem(d), s>>>(A, T);
+  if (A.one_word) k_scatter<true><<<d.max_chunks, kBlock, scatter_smem(d), s>>>(A, T);
+  else k_scatter<false><<<d.max_chunks, kBlock, scatter_smem(d), s>>>(A, T);
   if (d.n_big) k_scatter_big<<<d.n_big, kBlock, 0, s>>>(A, d.big_cells, d.n_big);
   t.end(kKScatter);
   t.count(d.n_big ? 2 : 1);
@@ -630,17 +685,24 @@ int scatter_max_chunks(int n_g, int tiles, int chunk) { return tiles + (n_g + ch
 bool set_scatter_shape(DeviceModel& d, int side, int chunk) {
   int tw, th, tx, ty;
   tile_grid(d.cnt_x, d.cnt_y, side, &tw, &th, &tx, &ty);
-  const int mc = scatter_max_chunks(d.n_g, tx * ty, chunk);
+  // a design of fewer chunks than resident blocks (five per SM) takes smaller
+  // ones: at 12.5k gcells 49 blocks instead of 17
+  int piece = std::min(chunk, std::max(kScatterPieceMin, (d.n_g + 5 * d.sm_count - 1) / (5 * d.sm_count)));
+  const double one = 4294967294.0 / scatter_max_value(d);    // up to here one window word will do
+  if (one < piece && one >= std::max(0.75 * piece, (double)kScatterPieceMin)) piece = (int)one;
+  const int mc = scatter_max_chunks(d.n_g, tx * ty, piece);
   if (tx * ty > d.tile_cap || mc > d.chunk_cap || chunk <= 0 || chunk >= 65536) return false;
   d.tile_w = tw; d.tile_h = th; d.tiles_x = tx; d.tiles_y = ty;
   d.chunk = chunk;
+  d.piece = piece;
   d.max_chunks = mc;
   return true;
 }
 
-// the window: two 32-bit words (16-bit split) per bin of the tile and its margin
+// the window: one 32-bit word, or two (16-bit split), per bin of the tile and
+// its margin, for the inst and the filler set
 size_t scatter_smem(const DeviceModel& d) {
-  return (size_t)4 * (d.tile_w + 2 * kTileMargin) * (d.tile_h + 2 * kTileMargin) * 4;
+  return (size_t)(scatter_one_word(d) ? 2 : 4) * (d.tile_w + 2 * kTileMargin) * (d.tile_h + 2 * kTileMargin) * 4;
 }
 
 int scatter_prepare_device() {
@@ -648,7 +710,8 @@ int scatter_prepare_device() {
   if (done) return GPL_OK;
   const int side = kTileSides[sizeof(kTileSides) / sizeof(kTileSides[0]) - 1];
   const int smem = 4 * (side + 2 * kTileMargin) * (side + 2 * kTileMargin) * 4;
-  GPL_CUDA(cudaFuncSetAttribute(k_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  GPL_CUDA(cudaFuncSetAttribute(k_scatter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  GPL_CUDA(cudaFuncSetAttribute(k_scatter<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   done = 1;
   return GPL_OK;
 }
@@ -662,7 +725,7 @@ int launch_tile_order(DeviceModel& d, int slot, cudaStream_t s, Timer& t) {
   O.slp = slot >= 0 ? d.slp[slot] : nullptr;
   for (int k = 0; k < 4; k++) O.slp_all[k] = d.slp[k];
   O.ctl = d.ctl;
-  O.chunk = d.chunk;
+  O.chunk = d.piece;
   O.tile_count = d.tile_count; O.tile_start = d.tile_start; O.order = d.order;
   O.chunks = d.chunks; O.n_chunks = d.n_chunks;
   t.begin(kKOther);
@@ -695,12 +758,12 @@ int launch_cell(DeviceModel& d, const EvalArgs& a, int n_phi_blocks, cudaStream_
 namespace {
 // updateInitialPrevSLPCoordi (src/nesterovPlace.cpp:492-512):
 // prev = inside(cur + coef * sum), one clamp per axis.
-__global__ void __launch_bounds__(kBlock) k_initial_prev(BinGeom G, int n_g, const int2* half,
+__global__ void __launch_bounds__(kBlock) k_initial_prev(BinGeom G, int n_g, const int4* geo,
                                                          const float2* cur, const float2* sum, float coef,
                                                          float2* out) {
   const int g = blockIdx.x * kBlock + threadIdx.x;
   if (g >= n_g) return;
-  const int2 h = half[g];
+  const int2 h = gcell_geo(geo[g]).half;
   const float2 c = cur[g], s = sum[g];
   const float x = __fadd_rn(c.x, __fmul_rn(coef, s.x));
   const float y = __fadd_rn(c.y, __fmul_rn(coef, s.y));
@@ -711,7 +774,7 @@ __global__ void __launch_bounds__(kBlock) k_initial_prev(BinGeom G, int n_g, con
 int launch_initial_prev(DeviceModel& d, const float2* cur_slp, const float2* cur_sum, float coef,
                         float2* out, cudaStream_t s, Timer& t) {
   t.begin(kKOther);
-  k_initial_prev<<<cell_blocks(d), kBlock, 0, s>>>(geom(d), d.n_g, d.g_half, cur_slp, cur_sum, coef, out);
+  k_initial_prev<<<cell_blocks(d), kBlock, 0, s>>>(geom(d), d.n_g, d.g_geo, cur_slp, cur_sum, coef, out);
   t.end(kKOther);
   t.count(1);
   GPL_CUDA(cudaGetLastError());
@@ -752,12 +815,13 @@ struct CellBatchArgs {
 
 __global__ void __launch_bounds__(kBlock, 5) k_scatter_batch(const ScatterBatchArgs* args, const int4* items,
                                                              const int* count) {
-  extern __shared__ unsigned win[];
+  extern __shared__ __align__(16) unsigned win[];
   const int n = *count;
   for (int w = blockIdx.x; w < n; w += gridDim.x) {
     const int4 it = items[w];
     const ScatterBatchArgs& a = args[it.x];
-    scatter_body(a.A, a.T, it.y, win);
+    if (a.A.one_word) scatter_body<true>(a.A, a.T, it.y, win);
+    else scatter_body<false>(a.A, a.T, it.y, win);
     __syncthreads();                  // the window is the next item's
   }
 }

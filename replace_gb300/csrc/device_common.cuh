@@ -7,26 +7,53 @@
 
 namespace gpl {
 
+// Division of 0 <= n < 2^31 by a fixed d >= 1 by a multiplication: with
+// 2^(l-1) < d <= 2^l, q = n ceil(2^(31+l) / d) / 2^(31+l) is exact (Granlund
+// and Montgomery, PLDI'94).  Integer division is some 25 instructions here,
+// and the scatter and gcell kernels need four per gcell.
+struct FastDiv {
+  unsigned m = 0;
+  int d = 1, s = 0;
+  FastDiv() = default;
+  __host__ explicit FastDiv(int div) : d(div) {
+    int l = 0;
+    while ((1ll << l) < d) l++;
+    s = l - 1;
+    if (d > 1) m = (unsigned)(((1ull << (31 + l)) + (unsigned)d - 1) / (unsigned)d);
+  }
+  __device__ __forceinline__ int operator()(int n) const {
+    return d == 1 ? n : (int)(__umulhi((unsigned)n, m) >> s);
+  }
+};
+
 // Bin column/row bounds of the reference's BinGrid (src/nesterovBase.cpp:684-711):
 // uniform binSize steps from the core corner, the last one clipped.
 struct BinGeom {
   int core_lx, core_ly, core_ux, core_uy, size_x, size_y, cnt_x, cnt_y;
+  FastDiv div_x, div_y;
   __device__ __forceinline__ int lo_x(int a) const { return core_lx + a * size_x; }
   __device__ __forceinline__ int hi_x(int a) const { return min(core_lx + (a + 1) * size_x, core_ux); }
   __device__ __forceinline__ int lo_y(int c) const { return core_ly + c * size_y; }
   __device__ __forceinline__ int hi_y(int c) const { return min(core_ly + (c + 1) * size_y, core_uy); }
+  // first and past-the-last bin of [l, u) (offsets from the core corner):
+  // l / size and u / size, rounded up when it does not divide (as C divides:
+  // towards zero), clamped to the grid
+  static __device__ __forceinline__ void span(int l, int u, int size, int cnt, const FastDiv& div, int& i0, int& i1) {
+    i0 = l > 0 ? div(l) : 0;
+    if (u >= 0) {
+      const int q = div(u);
+      i1 = q + (u - q * size != 0 ? 1 : 0);
+    } else {
+      i1 = u > -size ? 1 : 0;
+    }
+    i1 = min(i1, cnt);
+  }
   // getDensityMinMaxIdxX/Y (src/nesterovBase.cpp:822-841), clamped to the
   // grid so that a coordinate outside the core cannot index outside it.
   __device__ __forceinline__ void range(int lx, int ux, int ly, int uy, int& x0, int& x1, int& y0,
                                         int& y1) const {
-    const int dl = lx - core_lx, du = ux - core_lx;
-    x0 = dl / size_x;
-    x1 = ((du >= size_x ? du % size_x : du) == 0) ? du / size_x : du / size_x + 1;
-    const int el = ly - core_ly, eu = uy - core_ly;
-    y0 = el / size_y;
-    y1 = ((eu >= size_y ? eu % size_y : eu) == 0) ? eu / size_y : eu / size_y + 1;
-    x0 = max(x0, 0); y0 = max(y0, 0);
-    x1 = min(x1, cnt_x); y1 = min(y1, cnt_y);
+    span(lx - core_lx, ux - core_lx, size_x, cnt_x, div_x, x0, x1);
+    span(ly - core_ly, uy - core_ly, size_y, cnt_y, div_y, y0, y1);
   }
   // getOverlapDensityArea (src/nesterovBase.cpp:1533-1547)
   __device__ __forceinline__ float overlap(int a, int c, int lx, int ux, int ly, int uy) const {
@@ -35,7 +62,33 @@ struct BinGeom {
     if (rlx >= rux || rly >= ruy) return 0.0f;
     return __fmul_rn((float)(rux - rlx), (float)(ruy - rly));
   }
+  // the overlap's two factors; 0 where there is none
+  __device__ __forceinline__ float overlap_x(int a, int lx, int ux) const {
+    return (float)max(min(hi_x(a), ux) - max(lo_x(a), lx), 0);
+  }
+  __device__ __forceinline__ float overlap_y(int c, int ly, int uy) const {
+    return (float)max(min(hi_y(c), uy) - max(lo_y(c), ly), 0);
+  }
 };
+
+// A gcell's fixed geometry: half density size, scale (bits), and its kind in
+// the low byte (0 standard cell, 1 macro, 2 filler; bit 2: covers many bins)
+// with a big cell's index above.
+struct GCellGeo {
+  int2 half;
+  float scale;
+  int kind;
+  __device__ __forceinline__ int type() const { return kind & 3; }
+  __device__ __forceinline__ bool big() const { return kind & 4; }
+  __device__ __forceinline__ int big_index() const { return kind >> 8; }
+};
+__device__ __forceinline__ GCellGeo gcell_geo(int4 g) {
+  GCellGeo q;
+  q.half = make_int2(g.x, g.y);
+  q.scale = __int_as_float(g.z);
+  q.kind = g.w;
+  return q;
+}
 
 // GCell::setDensityCenterLocation: float centre truncated to int, then the
 // density rectangle is centre -/+ half size (src/nesterovBase.cpp:164-179).

@@ -114,10 +114,8 @@ constexpr int kWaBuckets = 8;
 struct DeviceModel {
   // static gcell data
   int n_g = 0, n_place = 0;
-  int2* g_half = nullptr;          // half density size (dDx/2, dDy/2)
-  float* g_scale = nullptr;
-  uint8_t* g_kind = nullptr;
-  float2* g_precond = nullptr;     // (#pins, real dx*dy)
+  int4* g_geo = nullptr;           // half density size, scale, kind (GCellGeo)
+  float* g_area = nullptr;         // real dx*dy (the density preconditioner)
   int32_t* g_pin_start = nullptr;  // CSR of each gcell's pin slots
   int32_t* g_pins = nullptr;       // device pin index of each slot
   int32_t* big_cells = nullptr;    // gcells covering many bins (macros)
@@ -151,7 +149,6 @@ struct DeviceModel {
   float2* w4x = nullptr;           // [cnt_x]
   float2* w4y = nullptr;           // [cnt_y]
   float2* twiddle = nullptr;       // exp(-2 pi i k / kFftMax), k < kFftMax/2
-  int32_t* g_big_idx = nullptr;    // index into big_cells or -1
   float2* d_big = nullptr;         // density gradient of big cells
   // Nesterov vectors (float2 per gcell): slots 0-2 rotate as prev/cur/next,
   // slot 3 holds the coordinates of the gradient-check hook (gpl_eval)
@@ -173,6 +170,7 @@ struct DeviceModel {
   // evaluations; any order gives the same int64 areas)
   int tile_w = 32, tile_h = 32, tiles_x = 1, tiles_y = 1, max_chunks = 1;
   int chunk = 2048;                // gcells per scatter chunk (at most)
+  int piece = 2048;                // the same, less on small designs (set_scatter_shape)
   int tile_cap = 1, chunk_cap = 1; // capacity of the tile and chunk tables
   int32_t* order = nullptr;        // [n_g] gcell indices, tile by tile
   int32_t* tile_count = nullptr;   // [tiles] counts, then fill cursors
@@ -357,7 +355,7 @@ int launch_loop_step(NesterovState* S, EvalCtl* ctl, const EvalResult* res, Iter
 constexpr int kScatterChunk = 2048;               // the default chunk
 constexpr int kTileSides[] = {16, 32, 64};
 constexpr int kScatterChunks[] = {1024, 2048};
-constexpr int kTileSideMin = 16, kScatterChunkMin = 1024;
+constexpr int kTileSideMin = 16, kScatterPieceMin = 256;
 static_assert(kScatterChunk < 65536 && kScatterChunks[1] < 65536,
               "the scatter's 16-bit split window sums need < 2^16 gcells per chunk");
 void tile_grid(int cnt_x, int cnt_y, int side, int* tw, int* th, int* tx, int* ty);

@@ -85,10 +85,9 @@ using namespace gpl;
 
 // Host arrays of a job's device model (see stage_device_model).
 struct DevStage {
-  std::vector<int2> half;
-  std::vector<uint8_t> kind;
-  std::vector<float2> precond;
-  std::vector<int32_t> big, big_idx;
+  std::vector<int4> geo;               // GCellGeo records
+  std::vector<float> area;
+  std::vector<int32_t> big;
   std::vector<int4> pins;
   std::vector<int32_t> dnet_start, g_dpins;
   std::vector<float2> tw, w4x, w4y;
@@ -192,9 +191,9 @@ size_t arena_bytes(size_t ng, size_t n_pins, size_t n_nets, size_t n_gpins, size
   const size_t tiles = (size_t)tx * ty;
   Sizer S;
   S.add(ng, 4); S.add(tiles, 4); S.add(tiles + 1, 4);
-  S.add(scatter_max_chunks((int)ng, (int)tiles, kScatterChunkMin), 16); S.add(1, 4);
-  S.add(ng, sizeof(int2)); S.add(ng, 4); S.add(ng, 1); S.add(ng, 8); S.add(ng + 1, 4);
-  S.add(n_big, 4); S.add(ng, 4); S.add(n_big, 8);
+  S.add(scatter_max_chunks((int)ng, (int)tiles, kScatterPieceMin), 16); S.add(1, 4);
+  S.add(ng, sizeof(int4)); S.add(ng, 4); S.add(ng + 1, 4);
+  S.add(n_big, 4); S.add(n_big, 8);
   S.add(n_pins, 16); S.add(n_nets + 1, 4);
   S.add(n_pins, 8); S.add(n_nets, 4); S.add(n_gpins, 4);
   S.add(2 * nb, 8); S.add(2 * nb, 8); S.add(nb, 8);
@@ -214,24 +213,24 @@ size_t arena_bytes(size_t ng, size_t n_pins, size_t n_nets, size_t n_gpins, size
 // positions, so that it can be built beside the initial place.
 int stage_device_model(const HostModel& m, DevStage& st) {
   const size_t ng = m.n_g;
-  st.half.resize(ng);
-  st.kind.resize(ng);
-  st.precond.resize(ng);
+  st.geo.resize(ng);
+  st.area.resize(ng);
   st.big.clear();
-  st.big_idx.assign(ng, -1);
   for (size_t g = 0; g < ng; g++) {
-    st.half[g] = make_int2((m.gdux[g] - m.gdlx[g]) / 2, (m.gduy[g] - m.gdly[g]) / 2);
-    st.kind[g] = m.gkind[g];
+    const int2 half = make_int2((m.gdux[g] - m.gdlx[g]) / 2, (m.gduy[g] - m.gdly[g]) / 2);
+    int kind = m.gkind[g];
     // bins a cell can touch per axis: its extent in bins plus one for a straddle
-    const long long bx = (2LL * st.half[g].x) / m.size_x + 2, by = (2LL * st.half[g].y) / m.size_y + 2;
+    const long long bx = (2LL * half.x) / m.size_x + 2, by = (2LL * half.y) / m.size_y + 2;
     if (bx * by > 64) {
-      st.kind[g] |= 4;
-      st.big_idx[g] = (int)st.big.size();
+      kind |= 4 | (int)st.big.size() << 8;
       st.big.push_back((int)g);
     }
-    // getWireLengthPreconditioner / getDensityPreconditioner (src/nesterovBase.cpp:1442-1454)
-    st.precond[g] = make_float2((float)(m.g_pin_start[g + 1] - m.g_pin_start[g]),
-                                (float)(m.gux[g] - m.glx[g]) * (float)(m.guy[g] - m.gly[g]));
+    int scale;
+    static_assert(sizeof(scale) == sizeof(m.gscale[g]), "float bits");
+    memcpy(&scale, &m.gscale[g], sizeof(scale));
+    st.geo[g] = make_int4(half.x, half.y, scale, kind);
+    // getDensityPreconditioner (src/nesterovBase.cpp:1442-1454)
+    st.area[g] = (float)(m.gux[g] - m.glx[g]) * (float)(m.guy[g] - m.gly[g]);
   }
   // WA buckets by degree: group widths 2, 4, 8, 16, 32 lanes, then a warp per net
   std::vector<int32_t> net_order;
@@ -427,7 +426,7 @@ int ensure_nb(gpl_job* j) {
     int tw, th, tx, ty;
     tile_grid(m.cnt_x, m.cnt_y, kTileSideMin, &tw, &th, &tx, &ty);
     d.tile_cap = tx * ty;
-    d.chunk_cap = scatter_max_chunks((int)ng, d.tile_cap, kScatterChunkMin);
+    d.chunk_cap = scatter_max_chunks((int)ng, d.tile_cap, kScatterPieceMin);
   }
   set_scatter_shape(d, 32, kScatterChunk);        // until the autotuner picks
   d.order = C.take<int32_t>(ng);
@@ -435,10 +434,9 @@ int ensure_nb(gpl_job* j) {
   d.tile_start = C.take<int32_t>((size_t)d.tile_cap + 1);
   d.chunks = C.take<int4>(d.chunk_cap);
   d.n_chunks = C.take<int32_t>(1);
-  d.g_half = C.take<int2>(ng); d.g_scale = C.take<float>(ng); d.g_kind = C.take<uint8_t>(ng);
-  d.g_precond = C.take<float2>(ng); d.g_pin_start = C.take<int32_t>(ng + 1);
+  d.g_geo = C.take<int4>(ng); d.g_area = C.take<float>(ng); d.g_pin_start = C.take<int32_t>(ng + 1);
   d.big_cells = C.take<int32_t>(st.big.size());
-  d.g_big_idx = C.take<int32_t>(ng); d.d_big = C.take<float2>(st.big.size());
+  d.d_big = C.take<float2>(st.big.size());
   d.pins = C.take<int4>(m.n_pins);
   d.net_start = C.take<int32_t>(m.n_nets + 1);
   d.pin_grad = C.take<float2>(m.n_pins);
@@ -465,13 +463,10 @@ int ensure_nb(gpl_job* j) {
   j->log_cap = (int)log_cap;
   cudaStream_t s = j->stream;
   int rc2 = GPL_OK;
-  rc2 = rc2 ? rc2 : upload(d.g_half, st.half.data(), ng * sizeof(int2), s);
-  rc2 = rc2 ? rc2 : upload(d.g_scale, m.gscale.data(), ng * 4, s);
-  rc2 = rc2 ? rc2 : upload(d.g_kind, st.kind.data(), ng, s);
-  rc2 = rc2 ? rc2 : upload(d.g_precond, st.precond.data(), ng * sizeof(float2), s);
+  rc2 = rc2 ? rc2 : upload(d.g_geo, st.geo.data(), ng * sizeof(int4), s);
+  rc2 = rc2 ? rc2 : upload(d.g_area, st.area.data(), ng * 4, s);
   rc2 = rc2 ? rc2 : upload(d.g_pin_start, m.g_pin_start.data(), (ng + 1) * 4, s);
   rc2 = rc2 ? rc2 : upload(d.big_cells, st.big.data(), st.big.size() * 4, s);
-  rc2 = rc2 ? rc2 : upload(d.g_big_idx, st.big_idx.data(), ng * 4, s);
   rc2 = rc2 ? rc2 : upload(d.pins, st.pins.data(), (size_t)m.n_pins * sizeof(int4), s);
   rc2 = rc2 ? rc2 : upload(d.g_pins, st.g_dpins.data(), st.g_dpins.size() * 4, s);
   rc2 = rc2 ? rc2 : upload(d.net_start, st.dnet_start.data(), (size_t)(m.n_nets + 1) * 4, s);
@@ -763,9 +758,9 @@ int choose_scatter_shape(gpl_job* j, int slot) {
       if ((want_side && side != want_side) || (want_chunk && chunk != want_chunk)) continue;
       if (!set_scatter_shape(d, side, chunk)) continue;
       bool dup = false;
-      for (int k = 0; k < n_seen; k++) dup |= seen[k][0] == d.tile_w && seen[k][1] == d.tile_h && seen[k][2] == chunk;
+      for (int k = 0; k < n_seen; k++) dup |= seen[k][0] == d.tile_w && seen[k][1] == d.tile_h && seen[k][2] == d.piece;
       if (dup || n_seen >= 16) continue;
-      seen[n_seen][0] = d.tile_w; seen[n_seen][1] = d.tile_h; seen[n_seen][2] = chunk;
+      seen[n_seen][0] = d.tile_w; seen[n_seen][1] = d.tile_h; seen[n_seen][2] = d.piece;
       n_seen++;
       rc = launch_tile_order(d, slot, j->stream, quiet);
       if (!rc) rc = launch_scatter(d, base_args(j), j->stream, quiet);    // warm-up
