@@ -37,6 +37,15 @@ GPL_HD bool diverged_result(const EvalResult& r) {
   return bad_value((float)r.wl_sum) || bad_value((float)r.d_sum) || r.nan_flag != 0.0;
 }
 
+// getStepLength / getDistance (src/nesterovPlace.cpp:555-571, 598-607).  Taken
+// where the result is read: on the device the two FP64 divisions and square
+// roots were 2 us at the end of every evaluation.
+GPL_HD float new_step_length(const EvalResult& r) {
+  const float cd = (float)sqrt(r.coord_dist / (2.0 * r.n_g));
+  const float gd = (float)sqrt(r.grad_dist / (2.0 * r.n_g));
+  return cd / gd;
+}
+
 // sumOverflow_ (src/nesterovPlace.cpp:112-115, 529-532)
 GPL_HD float overflow_ratio_of(const NesterovState& S, double overflow) {
   return (float)(int64_t)overflow / S.ovf_den;
@@ -151,7 +160,7 @@ GPL_HD int after_eval(NesterovState& S, const EvalResult& r, IterEntry* entry, b
   if (diverged_result(r)) {
     S.is_diverged = 1;
   } else {
-    const float ns = r.new_step_length;
+    const float ns = new_step_length(r);
     if (ns > S.step_length * 0.95) {
       S.step_length = ns;
     } else {

@@ -23,7 +23,10 @@ namespace gpl {
 namespace {
 
 constexpr int kBlock = 256;
-constexpr int kCellBlocksPerSm = 6;   // the gcell kernel's residency (40 registers, a few spilled)
+// The gcell kernel's residency (48 registers): at six blocks the loads moved
+// ahead of the pin gathers spill (10k / 200k / 1M cells: 12.2 / 28.6 / 54.1 us
+// against 11.3 / 24.6 / 55.0 at five and 10.9 / 24.6 / 58.6 at four).
+constexpr int kCellBlocksPerSm = 5;
 
 struct ScatterArgs {
   BinGeom geo;
@@ -334,7 +337,6 @@ struct CellArgs {
   int n_ovf_blocks, n_phi_blocks;
   unsigned* counters;
   long long* hpwl_total;
-  double* part_total;         // [kPartSlots] scratch of the final reduction
   EvalResult* out;
 };
 
@@ -377,7 +379,8 @@ __global__ void __launch_bounds__(kBlock) k_dgrad_big(CellArgs A, const int32_t*
 // the result is the same run to run.
 // Block vb of a launch of vgrid blocks.
 __device__ __forceinline__ void cell_body(const CellArgs& A, int vb, int vgrid) {
-  __shared__ double sh[32 * kPartSlots];
+  __shared__ float sh[32];
+  __shared__ int sh_bad[8];
   __shared__ bool last;
   // per-thread sums in float over the thread's few gcells; FP64 from the
   // warp sums on (the FP64 pipe is narrow on this part)
@@ -410,6 +413,9 @@ __device__ __forceinline__ void cell_body(const CellArgs& A, int vb, int vgrid) 
     const bool valid = g < A.n_g;
     int ps = 0, pe = 0;
     float2 w = make_float2(0.0f, 0.0f);
+    const int gg = valid ? g : A.n_g - 1;          // (loaded ahead of the pin gathers)
+    const float2 c = slp[gg];
+    const int4 gi = geo_g[gg];
     if (valid) {
       ps = g_pin_start[g];
       pe = g_pin_start[g + 1];
@@ -451,8 +457,7 @@ __device__ __forceinline__ void cell_body(const CellArgs& A, int vb, int vgrid) 
       if (lane == src) w = part;
     }
     if (!valid) continue;
-    const float2 c = slp[g];
-    const GCellGeo geo = gcell_geo(geo_g[g]);
+    const GCellGeo geo = gcell_geo(gi);
     // density gradient: sum over covered bins of overlap * scale * field
     float2 d = make_float2(0.0f, 0.0f);
     if (geo.big()) {
@@ -462,12 +467,35 @@ __device__ __forceinline__ void cell_body(const CellArgs& A, int vb, int vgrid) 
       density_rect(c, geo.half, lx, ux, ly, uy);
       G.range(lx, ux, ly, uy, x0, x1, y0, y1);
       const float sc = geo.scale;
-      for (int a = x0; a < x1; a++) {
-        for (int cc = y0; cc < y1; cc++) {
-          const float ov = __fmul_rn(G.overlap(a, cc, lx, ux, ly, uy), sc);
-          const float2 f = field[cc * G.cnt_x + a];
-          d.x = __fadd_rn(d.x, __fmul_rn(ov, f.x));
-          d.y = __fadd_rn(d.y, __fmul_rn(ov, f.y));
+      const int ny = y1 - y0;
+      if (ny <= 3) {
+        // the usual cell: its row widths once, a column's field loads together
+        float fy[3];
+#pragma unroll
+        for (int r = 0; r < 3; r++) fy[r] = r < ny ? G.overlap_y(y0 + r, ly, uy) : 0.0f;
+        const float2* fp = field + y0 * G.cnt_x;
+        for (int a = x0; a < x1; a++) {
+          const float fx = G.overlap_x(a, lx, ux);
+          float2 f[3];
+#pragma unroll
+          for (int r = 0; r < 3; r++) f[r] = r < ny ? fp[r * G.cnt_x + a] : make_float2(0.0f, 0.0f);
+#pragma unroll
+          for (int r = 0; r < 3; r++) {
+            if (r < ny) {
+              const float ov = __fmul_rn(__fmul_rn(fx, fy[r]), sc);
+              d.x = __fadd_rn(d.x, __fmul_rn(ov, f[r].x));
+              d.y = __fadd_rn(d.y, __fmul_rn(ov, f[r].y));
+            }
+          }
+        }
+      } else {
+        for (int a = x0; a < x1; a++) {
+          for (int cc = y0; cc < y1; cc++) {
+            const float ov = __fmul_rn(G.overlap(a, cc, lx, ux, ly, uy), sc);
+            const float2 f = field[cc * G.cnt_x + a];
+            d.x = __fadd_rn(d.x, __fmul_rn(ov, f.x));
+            d.y = __fadd_rn(d.y, __fmul_rn(ov, f.y));
+          }
         }
       }
     }
@@ -493,81 +521,86 @@ __device__ __forceinline__ void cell_body(const CellArgs& A, int vb, int vgrid) 
       const float gx = s.x - q.x, gy = s.y - q.y;
       // rounding spelled out: the per-job and the batched kernel inline
       // this body, and must not fuse differently
-      acc[2] = __fadd_rn(acc[2], __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)));
-      acc[3] = __fadd_rn(acc[3], __fadd_rn(__fmul_rn(gx, gx), __fmul_rn(gy, gy)));
+      acc[2] = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, acc[2]));
+      acc[3] = __fmaf_rn(gx, gx, __fmaf_rn(gy, gy, acc[3]));
     }
     if (!isfinite(aw) || !isfinite(ad)) bad = 1;
   }
+  // The FP64 pipe takes 15 cycles a warp instruction here, so the sums across
+  // warps and blocks are laid out to need few: each instruction serves all
+  // slots at once (block), or one slot a warp (final).
+  const int wid = threadIdx.x >> 5;
+  static_assert(kBlock == 256, "eight warps");
   {
-    // warp sums (float, fixed xor tree), then the block's warps in order in FP64
+    // warp sums (float, fixed xor tree), then the block's eight warps in FP64
 #pragma unroll
     for (int k = 0; k < 4; k++)
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
     const int any_bad = __any_sync(0xffffffffu, bad);
-    const int wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     if (lane == 0) {
 #pragma unroll
-      for (int k = 0; k < 4; k++) sh[k * 32 + wid] = (double)acc[k];
-      sh[4 * 32 + wid] = any_bad ? 1.0 : 0.0;
+      for (int k = 0; k < 4; k++) sh[k * 8 + wid] = acc[k];
+      sh_bad[wid] = any_bad;
     }
     __syncthreads();
-    if (threadIdx.x < 5) {
-      double t = 0.0;
-      for (int w8 = 0; w8 < nw; w8++) t += sh[threadIdx.x * 32 + w8];
-      A.part[(size_t)(kPartWl + threadIdx.x) * A.stride + vb] = t;
+    if (threadIdx.x < 32) {
+      // lane 8 k + w: slot k of warp w
+      double t = (double)sh[lane];
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      const int bads = __popc(__ballot_sync(0xffffffffu, lane < 8 && sh_bad[lane & 7]));
+      static_assert(kPartD == kPartWl + 1 && kPartCoordDist == kPartWl + 2 && kPartGradDist == kPartWl + 3 &&
+                        kPartNan == kPartWl + 4, "slot order");
+      if ((lane & 7) == 0) A.part[(size_t)(kPartWl + (lane >> 3)) * A.stride + vb] = t;
+      if (lane == 0) A.part[(size_t)kPartNan * A.stride + vb] = (double)bads;
+      __threadfence();
+      __syncwarp();
+      if (lane == 0) last = atomicAdd(&A.counters[0], 1u) == (unsigned)vgrid - 1;
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(&A.counters[0], 1u) == (unsigned)vgrid - 1;
-  }
-  __syncthreads();
   if (!last) return;
-  // final reduction (the last block): every partial is visible after the
-  // fence; all slots are loaded in one pass so the loads overlap
-  double tot[kPartSlots];
+  // final reduction (the last block), a slot per warp: every partial is
+  // visible after the fence; four loads in flight per lane
+  __threadfence();
+  static_assert(kPartSlots <= 7, "a slot per warp, HPWL on the last");
+  if (wid < kPartSlots) {
+    const int n = wid == kPartOverflow ? A.n_ovf_blocks : (wid == kPartPhi ? A.n_phi_blocks : vgrid);
+    const double* p = A.part + (size_t)wid * A.stride;
+    double t = 0.0;
+    for (int i = lane; i < n; i += 128) {
+      double x[4];
 #pragma unroll
-  for (int slot = 0; slot < kPartSlots; slot++) tot[slot] = 0.0;
-  const int n_max = max(max(vgrid, A.n_ovf_blocks), A.n_phi_blocks);
-  for (int i = threadIdx.x; i < n_max; i += blockDim.x) {
+      for (int u = 0; u < 4; u++) x[u] = i + 32 * u < n ? __ldcg(p + i + 32 * u) : 0.0;
 #pragma unroll
-    for (int slot = 0; slot < kPartSlots; slot++) {
-      const int n = slot == kPartOverflow ? A.n_ovf_blocks
-                                          : (slot == kPartPhi ? A.n_phi_blocks : vgrid);
-      if (i < n) tot[slot] += __ldcg(A.part + (size_t)slot * A.stride + i);
+      for (int u = 0; u < 4; u++)
+        if (i + 32 * u < n) t += x[u];
     }
-  }
-  // the WA kernel's HPWL accumulators: one per lane of the first warp,
-  // summed by shuffles and cleared for the next evaluation
-  static_assert(kHpwlLanes == 32, "one HPWL accumulator per lane");
-  long long hpwl = 0;
-  if (threadIdx.x < 32) {
-    hpwl = __ldcg(A.hpwl_total + threadIdx.x * kHpwlStride);
-    A.hpwl_total[threadIdx.x * kHpwlStride] = 0;
+    if (n > 0) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    }
+    if (lane == 0) {
+      EvalResult* r = A.out;
+      double* dst = wid == kPartOverflow ? &r->overflow : wid == kPartWl ? &r->wl_sum : wid == kPartD ? &r->d_sum
+                    : wid == kPartCoordDist ? &r->coord_dist : wid == kPartGradDist ? &r->grad_dist
+                    : wid == kPartNan ? &r->nan_flag : &r->sum_phi;
+      *dst = t;
+    }
+  } else {
+    // the WA kernel's HPWL accumulators: one per lane, summed by shuffles and
+    // cleared for the next evaluation
+    static_assert(kHpwlLanes == 32, "one HPWL accumulator per lane");
+    long long hpwl = __ldcg(A.hpwl_total + lane * kHpwlStride);
+    A.hpwl_total[lane * kHpwlStride] = 0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) hpwl += __shfl_xor_sync(0xffffffffu, hpwl, o);
-  }
-  block_reduce_n<kPartSlots>(tot, A.part_total, 1, sh, 0);   // thread 0 writes part_total[k]
-  if (threadIdx.x == 0) {
-    for (int slot = 0; slot < kPartSlots; slot++) tot[slot] = A.part_total[slot];
-    EvalResult r;
-    r.overflow = tot[kPartOverflow];
-    r.wl_sum = tot[kPartWl];
-    r.d_sum = tot[kPartD];
-    r.coord_dist = tot[kPartCoordDist];
-    r.grad_dist = tot[kPartGradDist];
-    r.sum_phi = tot[kPartPhi];
-    r.nan_flag = tot[kPartNan];
-    r.hpwl = hpwl;
-    // getStepLength / getDistance (src/nesterovPlace.cpp:555-571, 598-607)
-    const float cd = (float)sqrt(r.coord_dist / (2.0 * A.n_g));
-    const float gd = (float)sqrt(r.grad_dist / (2.0 * A.n_g));
-    r.new_step_length = cd / gd;
-    r.pad = 0;
-    *A.out = r;
-    A.counters[0] = 0u;
+    if (lane == 0) {
+      A.out->hpwl = hpwl;
+      A.out->n_g = A.n_g;
+      A.counters[0] = 0u;
+    }
   }
 }
 
@@ -651,7 +684,6 @@ CellArgs cell_args(const DeviceModel& d, const EvalArgs& a, int n_phi_blocks) {
   A.n_phi_blocks = n_phi_blocks;
   A.counters = d.counters;
   A.hpwl_total = d.hpwl_total;
-  A.part_total = d.part_total;
   A.out = d.result;
   return A;
 }

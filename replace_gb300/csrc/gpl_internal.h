@@ -163,7 +163,6 @@ struct DeviceModel {
   double* part = nullptr;          // [kPartSlots * part_stride]
   int part_stride = 0;
   long long* hpwl_total = nullptr; // HPWL accumulators (WA warps add, the gcell kernel sums and clears)
-  double* part_total = nullptr;    // [kPartSlots] final sums
   unsigned* counters = nullptr;    // [2] last-block counters (gcell kernel, WA kernel)
   int sm_count = 0;
   // gcells ordered by bin tile for the scatter (refreshed every few
@@ -219,7 +218,7 @@ struct EvalResult {
   double sum_phi;
   double nan_flag;
   long long hpwl;
-  float new_step_length;
+  int n_g;                // gcells (the distances' count)
   int pad;
 };
 

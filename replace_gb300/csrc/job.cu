@@ -204,7 +204,6 @@ size_t arena_bytes(size_t ng, size_t n_pins, size_t n_nets, size_t n_gpins, size
   S.add(ng, 8); S.add(ng, 8);                 // hook outputs: wl / density gradients
   S.add(1, sizeof(EvalCtl));
   S.add(ps, 8); S.add(1, sizeof(EvalResult)); S.add(kHpwlLanes * kHpwlStride, 8); S.add(4, 4);
-  S.add(kPartSlots, 8);
   S.add(1, sizeof(NesterovState)); S.add(log_cap, sizeof(IterEntry));   // device loop
   return S.bytes;
 }
@@ -457,7 +456,6 @@ int ensure_nb(gpl_job* j) {
   d.result = C.take<EvalResult>(1);
   d.hpwl_total = C.take<long long>(kHpwlLanes * kHpwlStride);
   d.counters = C.take<unsigned>(4);
-  d.part_total = C.take<double>(kPartSlots);
   j->d_state = C.take<NesterovState>(1);
   j->d_log = C.take<IterEntry>(log_cap);
   j->log_cap = (int)log_cap;
@@ -869,7 +867,7 @@ int nesterov_init(gpl_job* j) {
   }
   j->S.density_penalty = ((float)j->S.last.wl_sum / (float)j->S.last.d_sum) * m.p.init_density_penalty;
   j->S.sum_overflow = overflow_ratio(j);
-  j->S.step_length = j->S.last.new_step_length;
+  j->S.step_length = new_step_length(j->S.last);
   j->S.cur_a = 1.0f;
   j->S.min_sum_overflow = 1e30f;
   j->S.hpwl_with_min = 1e30f;
