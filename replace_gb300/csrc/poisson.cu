@@ -23,6 +23,7 @@
 // (the "group form", with the density in its own kernel before pass A); other
 // grids use one packed pair per 256-thread block and radix-4 Stockham passes
 // in shared memory.
+#include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -39,6 +40,8 @@
 namespace gpl {
 
 namespace {
+
+namespace cg = cooperative_groups;
 
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
@@ -507,8 +510,8 @@ __global__ void __launch_bounds__(256) k_poisson_c(const __grid_constant__ PassC
 
 template <int N>
 struct GroupFft {
-  static_assert(N == 256 || N == 512 || N == 1024 || N == 2048, "group form sizes");
-  static constexpr int kG = N == 256 ? 16 : N == 2048 ? 64 : 32;   // lanes per transform
+  static_assert(N >= 64 && N <= 2048 && (N & (N - 1)) == 0, "group form sizes");
+  static constexpr int kG = N <= 128 ? 8 : N == 256 ? 16 : N == 2048 ? 64 : 32;   // lanes per transform
   static constexpr int kE = N / kG;                                // elements per lane
   static constexpr int kStride = kE + 1;                           // padded transpose row
   static constexpr int kBuf = 2 * kG * kStride;                    // floats per group buffer
@@ -516,6 +519,8 @@ struct GroupFft {
 };
 
 // exp(-2 pi i n1 k2 / N) at [k2 * G + n1], k2 < E: one coalesced row per k2.
+__device__ __align__(16) float2 g_tw64[64];
+__device__ __align__(16) float2 g_tw128[128];
 __device__ __align__(16) float2 g_tw256[256];
 __device__ __align__(16) float2 g_tw512[512];
 __device__ __align__(16) float2 g_tw1024[1024];
@@ -526,7 +531,9 @@ __device__ __forceinline__ const float2* tw_table() {
   if constexpr (N == 2048) return g_tw2048;
   else if constexpr (N == 1024) return g_tw1024;
   else if constexpr (N == 512) return g_tw512;
-  else return g_tw256;
+  else if constexpr (N == 256) return g_tw256;
+  else if constexpr (N == 128) return g_tw128;
+  else return g_tw64;
 }
 
 template <int kBits>
@@ -578,7 +585,7 @@ __device__ __forceinline__ void rot64(float& re, float& im, int m) {
   im = r * sn + i * c;
 }
 
-// In-register M-point DFT (M = 16 or 32), radix-2 decimation in frequency:
+// In-register M-point DFT (M = 8, 16 or 32), radix-2 decimation in frequency:
 // natural input order, register r ends with output brev(r).  Twiddles
 // exp(kSign 2 pi i j / len) = exp(kSign 2 pi i (j 64/len) / 64) are
 // compile-time constants after unrolling.
@@ -620,11 +627,12 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// Barrier of the calling group: its warp, or for 64 lanes two warps by the
-// named barrier 1 + the group's number in the block.
+// Barrier of the calling group: its lanes of the warp, or for 64 lanes two
+// warps by the named barrier 1 + the group's number in the block.
 template <int G>
 __device__ __forceinline__ void group_sync() {
-  if constexpr (G <= 32) __syncwarp();
+  if constexpr (G == 32) __syncwarp();
+  else if constexpr (G < 32) __syncwarp(((1u << G) - 1u) << (threadIdx.x & 31 & ~(G - 1)));
   else asm volatile("bar.sync %0, 64;\n" ::"r"(1 + (int)(threadIdx.x >> 6)) : "memory");
 }
 
@@ -635,7 +643,7 @@ template <int N, int kSign>
 __device__ __forceinline__ void group_fft(float2* buf, const float2* tws) {
   using F = GroupFft<N>;
   constexpr int E = F::kE, S = F::kStride, G = F::kG;
-  constexpr int kBits = E == 32 ? 5 : 4;
+  constexpr int kBits = E == 32 ? 5 : E == 16 ? 4 : 3;
   const int l = threadIdx.x & (G - 1);
   float re[E], im[E];
   // stage 1: lane n1 = l holds x[n1 + G n2], n2 < E; DFT along n2
@@ -674,11 +682,29 @@ __device__ __forceinline__ void group_fft(float2* buf, const float2* tws) {
     dft_reg<E, kSign>(re, im);
 #pragma unroll
     for (int r = 0; r < E; r++) buf[l + E * brev<kBits>(r)] = make_float2(re[r], im[r]);
+  } else if constexpr (E == 2 * G) {
+    // stage 2: lane l takes columns k2 = l and l + G, a G-point DFT each
+    constexpr int kBitsG = kBits - 1;
+    float r2[2][G], i2[2][G];
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int n1 = 0; n1 < G; n1++) {
+        r2[h][n1] = tr[n1 * S + l + G * h];
+        i2[h][n1] = ti[n1 * S + l + G * h];
+      }
+    group_sync<G>();
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      dft_reg<G, kSign>(r2[h], i2[h]);
+#pragma unroll
+      for (int r = 0; r < G; r++) buf[l + G * h + E * brev<kBitsG>(r)] = make_float2(r2[h][r], i2[h][r]);
+    }
   } else {
     // stage 2 for G = 2 E: lane pair (2 k2, 2 k2 + 1) takes the even and odd
     // n1 of column k2, one E-point DFT each, then X[k] = E[k] + W^k O[k]
     // (even lane) and X[k + E] = E[k] - W^k O[k] (odd lane), W = W_G
-    static_assert(G == 2 * E, "one or two lanes per column");
+    static_assert(G == 2 * E, "one or two lanes or columns");
     const int k2 = l >> 1, odd = l & 1;
 #pragma unroll
     for (int i = 0; i < E; i++) {
@@ -960,6 +986,191 @@ __global__ void __launch_bounds__(FieldShape<N>::threads(3)) k_poisson_field_g(P
   }
 }
 
+// ---------------------------------------------------------------------------
+// Cluster form, for 64 x 64, 128 x 128 and 256 x 256 grids given as densities
+// (gpl_poisson_solve): the whole solve in one launch of one cluster of 16
+// CTAs.  On these grids each of the three passes is bound by its launch and
+// one round trip to memory (7 us a pass whatever the size, for 0.04 us of
+// bytes), so the passes become phases of one kernel and the transposes
+// between them go through distributed shared memory: CTA c transforms rows
+// [c N/16, (c + 1) N/16), writes each spectrum element into the shared memory
+// of its column's owner, that CTA solves its columns and writes P1 and P2
+// back to the rows' owners.  Group FFTs as above (8 or 16 lanes a pair);
+// elements k and n - k by one thread, in place.
+// Solve with the potential: 64 x 64 19.5 -> 8.2 us, 128 x 128 20.5 -> 10.3,
+// 256 x 256 22.6 -> 18.4.  Jobs keep the block form on these grids: the other
+// rounding, amplified over a loop's iterations, moved single cells of 10k-cell
+// designs by up to 1e-3 of the core in 64 iterations.
+constexpr int kClCtas = 16;
+
+template <int N>
+struct ClusterShape {
+  static constexpr int kT = N >= 128 ? 512 : 256;          // threads per CTA
+  static constexpr int kP = N / (2 * kClCtas);             // row pairs, and column pairs, per CTA
+  static constexpr int kBufF2 = GroupFft<N>::kBuf / 2;
+  // three row buffers (Ex, P1, P2) and two column buffers a pair, twiddles
+  static constexpr size_t kBytes = ((size_t)5 * kP * kBufF2 + N) * sizeof(float2);
+};
+
+// f(task) for task < n by the block's groups of G lanes
+template <int G, int kT, class F>
+__device__ __forceinline__ void group_tasks(int n, F f) {
+  for (int t = threadIdx.x / G; t < n; t += kT / G) f(t);
+}
+
+template <int N>
+__global__ void __cluster_dims__(kClCtas, 1, 1) __launch_bounds__(ClusterShape<N>::kT)
+    k_poisson_cluster(const __grid_constant__ PassAArgs A, const __grid_constant__ PassBArgs B,
+                      const __grid_constant__ PassCArgs C) {
+  extern __shared__ float2 smem[];
+  using F = GroupFft<N>;
+  constexpr int G = F::kG, kP = ClusterShape<N>::kP, kBufF2 = ClusterShape<N>::kBufF2;
+  constexpr int kT = ClusterShape<N>::kT;
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank(), tid = threadIdx.x;
+  float2* rowx = smem;                                     // [kP] density pairs, then Ex
+  float2* row1 = rowx + kP * kBufF2;                       // [kP] P1 of row pairs
+  float2* row2 = row1 + kP * kBufF2;                       // [kP] P2
+  float2* col0 = row2 + kP * kBufF2;                       // [kP] spectrum of column pairs, then P1
+  float2* col1 = col0 + kP * kBufF2;                       // [kP] P2
+  float2* tws = col1 + kP * kBufF2;
+  for (int t = tid; t < N; t += kT) tws[t] = __ldg(tw_table<N>() + t);
+  // rows in Makhoul order
+  const int j0 = rank * 2 * kP;
+  for (int idx = tid; idx < 2 * kP * N; idx += kT) {
+    const int h = idx / N, i = idx & (N - 1);
+    float* slot = reinterpret_cast<float*>(&rowx[(h >> 1) * kBufF2 + makhoul_pos(i, N)]);
+    slot[h & 1] = __ldg(&A.density_in[(j0 + h) * N + i]);
+  }
+  // every CTA of the cluster has started (its shared memory may be written)
+  cl.sync();
+  group_tasks<G, kT>(kP, [&](int p) { group_fft<N, -1>(rowx + p * kBufF2, tws); });
+  __syncthreads();
+  // DCT-II along x, each column pair to its owner (Makhoul order along y)
+  for (int idx = tid; idx < kP * N; idx += kT) {
+    const int p = idx / N, k = idx & (N - 1);
+    const float2* z = rowx + p * kBufF2;
+    const float2 c = dct2_post(z[k], z[(N - k) & (N - 1)], __ldg(&A.w4[k]));
+    float2* col = cl.map_shared_rank(col0, k / (2 * kP)) + ((k >> 1) & (kP - 1)) * kBufF2;
+    // a lane pair holds columns k, k + 1 of rows v, v + 1: one row each
+    const int odd = k & 1, v = j0 + 2 * p + odd;
+    const float got = __shfl_xor_sync(0xffffffffu, odd ? c.x : c.y, 1);
+    col[makhoul_pos(v, N)] = odd ? make_float2(got, c.y) : make_float2(c.x, got);
+  }
+  cl.sync();
+  // columns: DCT-II along y, the spectral solve, P1 = IDCT_y(phi^) and P2 =
+  // IDST_y(wy phi^), as in the group form's pass B
+  group_tasks<G, kT>(kP, [&](int q) { group_fft<N, -1>(col0 + q * kBufF2, tws); });
+  __syncthreads();
+  const int u0 = rank * 2 * kP;
+  for (int idx = tid; idx < kP * (N / 2); idx += kT) {
+    const int q = idx / (N / 2), k = idx & (N / 2 - 1), m = k ? N - k : N / 2, u = u0 + 2 * q;
+    float2* buf0 = col0 + q * kBufF2;
+    float2* buf1 = col1 + q * kBufF2;
+    const float2 zk = buf0[k], zm = buf0[m];
+    const float2 wx = make_float2(__ldg(&B.wx[u]), __ldg(&B.wx[u + 1]));
+    const float2 w4k = __ldg(&B.w4[k]), w4m = __ldg(&B.w4[m]);
+    const float wk = __ldg(&B.wy[k]), wm = __ldg(&B.wy[m]);
+    const float2 pk = solve_pair(B, zk, k ? zm : zk, w4k, wx, wk, u, k);
+    const float2 pm = solve_pair(B, zm, k ? zk : zm, w4m, wx, wm, u, m);
+    const float2 sk = make_float2(__fmul_rn(pk.x, wk), __fmul_rn(pk.y, wk));
+    const float2 sm = make_float2(__fmul_rn(pm.x, wm), __fmul_rn(pm.y, wm));
+    buf0[k] = pre_pair(pk, pm, w4k, k);
+    buf0[m] = pre_pair(pm, k ? pk : pm, w4m, m);
+    buf1[k] = k ? pre_pair(sm, sk, w4k, k) : make_float2(0.0f, 0.0f);
+    buf1[m] = pre_pair(k ? sk : sm, sm, w4m, m);
+  }
+  __syncthreads();
+  group_tasks<G, kT>(2 * kP, [&](int t) { group_fft<N, 1>(col0 + t * kBufF2, tws); });   // col1 follows col0
+  __syncthreads();
+  for (int idx = tid; idx < kP * N; idx += kT) {
+    const int q = idx & (kP - 1), v = idx / kP, m = makhoul_pos(v, N), u = u0 + 2 * q;
+    const float2 a = col0[q * kBufF2 + m];
+    float2 b = col1[q * kBufF2 + m];
+    if (v & 1) { b.x = -b.x; b.y = -b.y; }
+    // lanes kP apart hold rows v, v + 1 of columns u, u + 1: one column each
+    const int odd = v & 1, owner = v / (2 * kP), at = ((v >> 1) & (kP - 1)) * kBufF2 + u + odd;
+    const float ga = __shfl_xor_sync(0xffffffffu, odd ? a.x : a.y, kP);
+    const float gb = __shfl_xor_sync(0xffffffffu, odd ? b.x : b.y, kP);
+    cl.map_shared_rank(row1, owner)[at] = odd ? make_float2(ga, a.y) : make_float2(a.x, ga);
+    cl.map_shared_rank(row2, owner)[at] = odd ? make_float2(gb, b.y) : make_float2(b.x, gb);
+  }
+  cl.sync();
+  // rows: Ex = IDST_x(wx P1), Ey = IDCT_x(P2), phi = IDCT_x(P1)
+  for (int idx = tid; idx < kP * (N / 2); idx += kT) {
+    const int p = idx / (N / 2), k = idx & (N / 2 - 1), m = k ? N - k : N / 2;
+    const float2 w4k = __ldg(&C.w4[k]), w4m = __ldg(&C.w4[m]);
+    const float wk = __ldg(&C.wx[k]), wm = __ldg(&C.wx[m]);
+    const float2 pk = row1[p * kBufF2 + k], pm = row1[p * kBufF2 + m];
+    const float2 yk = row2[p * kBufF2 + k], ym = row2[p * kBufF2 + m];
+    const float2 sk = make_float2(__fmul_rn(pk.x, wk), __fmul_rn(pk.y, wk));
+    const float2 sm = make_float2(__fmul_rn(pm.x, wm), __fmul_rn(pm.y, wm));
+    rowx[p * kBufF2 + k] = k ? pre_pair(sm, sk, w4k, k) : make_float2(0.0f, 0.0f);
+    rowx[p * kBufF2 + m] = pre_pair(k ? sk : sm, sm, w4m, m);
+    row2[p * kBufF2 + k] = pre_pair(yk, ym, w4k, k);
+    row2[p * kBufF2 + m] = pre_pair(ym, k ? yk : ym, w4m, m);
+    if (C.phi) {
+      row1[p * kBufF2 + k] = pre_pair(pk, pm, w4k, k);
+      row1[p * kBufF2 + m] = pre_pair(pm, k ? pk : pm, w4m, m);
+    }
+  }
+  __syncthreads();
+  // tasks: Ex and Ey of every pair, then phi
+  group_tasks<G, kT>(C.phi ? 3 * kP : 2 * kP, [&](int t) {
+    float2* buf = t < kP ? rowx + t * kBufF2 : t < 2 * kP ? row2 + (t - kP) * kBufF2 : row1 + (t - 2 * kP) * kBufF2;
+    group_fft<N, 1>(buf, tws);
+  });
+  __syncthreads();
+  for (int idx = tid; idx < kP * N; idx += kT) {
+    const int p = idx / N, i = idx & (N - 1), m = makhoul_pos(i, N);
+    const int b = (j0 + 2 * p) * N + i;
+    float2 ex = rowx[p * kBufF2 + m];
+    const float2 ey = row2[p * kBufF2 + m];
+    if (i & 1) { ex.x = -ex.x; ex.y = -ex.y; }
+    if (C.field) {
+      C.field[b] = make_float2(ex.x, ey.x);
+      C.field[b + N] = make_float2(ex.y, ey.y);
+    } else {
+      C.fx[b] = ex.x; C.fx[b + N] = ex.y;
+      C.fy[b] = ey.x; C.fy[b + N] = ey.y;
+    }
+    if (C.phi) {
+      const float2 ph = row1[p * kBufF2 + m];
+      C.phi[b] = ph.x; C.phi[b + N] = ph.y;
+    }
+  }
+}
+
+template <int N>
+bool cluster_prepare() {
+  const int bytes = (int)ClusterShape<N>::kBytes;
+  const void* f = (const void*)k_poisson_cluster<N>;
+  bool ok = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess &&
+            cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(kClCtas);
+  c.blockDim = dim3(ClusterShape<N>::kT);
+  c.dynamicSmemBytes = bytes;
+  int num = 0;
+  ok = ok && cudaOccupancyMaxActiveClusters(&num, k_poisson_cluster<N>, &c) == cudaSuccess && num > 0;
+  if (!ok) cudaGetLastError();
+  return ok;
+}
+
+// Whether the cluster form takes this grid on the current device (16 CTAs are
+// above the portable cluster size; a device that cannot place them keeps the
+// block form).
+bool cluster_form(int nx, int ny) {
+  if (nx != ny || (nx != 64 && nx != 128 && nx != 256)) return false;
+  static std::mutex mu;
+  static signed char state[64] = {0};                      // per device: 0 unknown, 1 yes, -1 no
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  std::lock_guard<std::mutex> lk(mu);
+  if (state[dev] == 0) state[dev] = cluster_prepare<64>() && cluster_prepare<128>() && cluster_prepare<256>() ? 1 : -1;
+  return state[dev] > 0;
+}
+
 // Whether the group form takes this grid.
 bool group_form(int nx, int ny) {
   auto in = [](int n) { return n == 256 || n == 512 || n == 1024 || n == 2048; };
@@ -1039,10 +1250,10 @@ int poisson_prepare_device() {
   GPL_CUDA(group_prepare<512>());
   GPL_CUDA(group_prepare<1024>());
   GPL_CUDA(group_prepare<2048>());
-  for (int n : {256, 512, 1024, 2048}) {
+  for (int n : {64, 128, 256, 512, 1024, 2048}) {
     // the group form's twiddles, [k2 * G + n1] = exp(-2 pi i n1 k2 / n)
-    const int g = n == 256 ? GroupFft<256>::kG : n == 2048 ? GroupFft<2048>::kG : GroupFft<512>::kG;
-    static_assert(GroupFft<512>::kG == GroupFft<1024>::kG, "one width");
+    const int g = n <= 128 ? GroupFft<64>::kG : n == 256 ? GroupFft<256>::kG : n == 2048 ? GroupFft<2048>::kG : GroupFft<512>::kG;
+    static_assert(GroupFft<512>::kG == GroupFft<1024>::kG && GroupFft<64>::kG == GroupFft<128>::kG, "one width");
     std::vector<float2> t(n);
     for (int k2 = 0; k2 < n / g; k2++)
       for (int n1 = 0; n1 < g; n1++) {
@@ -1050,7 +1261,9 @@ int poisson_prepare_device() {
         t[k2 * g + n1] = make_float2((float)cos(a), (float)sin(a));
       }
     const size_t bytes = n * sizeof(float2);
-    if (n == 256) GPL_CUDA(cudaMemcpyToSymbol(g_tw256, t.data(), bytes));
+    if (n == 64) GPL_CUDA(cudaMemcpyToSymbol(g_tw64, t.data(), bytes));
+    else if (n == 128) GPL_CUDA(cudaMemcpyToSymbol(g_tw128, t.data(), bytes));
+    else if (n == 256) GPL_CUDA(cudaMemcpyToSymbol(g_tw256, t.data(), bytes));
     else if (n == 512) GPL_CUDA(cudaMemcpyToSymbol(g_tw512, t.data(), bytes));
     else if (n == 1024) GPL_CUDA(cudaMemcpyToSymbol(g_tw1024, t.data(), bytes));
     else GPL_CUDA(cudaMemcpyToSymbol(g_tw2048, t.data(), bytes));
@@ -1221,6 +1434,21 @@ int poisson_passes(const PoissonGrid& g, unsigned long long* const* area_pair,
     else launch_field_g<2048>(C, ny, s);
     if (t) t->end(kKPoissonC);
     if (t) t->count(areas ? 4 : 3);
+    GPL_CUDA(cudaGetLastError());
+    return GPL_OK;
+  }
+  if (density_in && cluster_form(nx, ny)) {
+    PassBArgs B;
+    PassCArgs C;
+    int grid[3];
+    size_t smem[3];
+    block_form_bc(g, spec, p1, p2, field, fx, fy, phi, B, C, grid, smem);
+    if (t) t->begin(kKPoissonB);
+    if (nx == 64) k_poisson_cluster<64><<<kClCtas, ClusterShape<64>::kT, ClusterShape<64>::kBytes, s>>>(A, B, C);
+    else if (nx == 128) k_poisson_cluster<128><<<kClCtas, ClusterShape<128>::kT, ClusterShape<128>::kBytes, s>>>(A, B, C);
+    else k_poisson_cluster<256><<<kClCtas, ClusterShape<256>::kT, ClusterShape<256>::kBytes, s>>>(A, B, C);
+    if (t) t->end(kKPoissonB);
+    if (t) t->count(1);
     GPL_CUDA(cudaGetLastError());
     return GPL_OK;
   }
