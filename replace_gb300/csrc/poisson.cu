@@ -997,7 +997,7 @@ __global__ void __launch_bounds__(FieldShape<N>::threads(3)) k_poisson_field_g(P
 // of its column's owner, that CTA solves its columns and writes P1 and P2
 // back to the rows' owners.  Group FFTs as above (8 or 16 lanes a pair);
 // elements k and n - k by one thread, in place.
-// Solve with the potential: 64 x 64 19.5 -> 8.2 us, 128 x 128 20.5 -> 10.3,
+// Solve with the potential: 64 x 64 19.5 -> 6.2 us, 128 x 128 20.5 -> 10.3,
 // 256 x 256 22.6 -> 18.4.  Jobs keep the block form on these grids: the other
 // rounding, amplified over a loop's iterations, moved single cells of 10k-cell
 // designs by up to 1e-3 of the core in 64 iterations.
