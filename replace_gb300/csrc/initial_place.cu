@@ -1001,19 +1001,22 @@ struct BlockRows {
 // (A x)_i of the block's rows when it has a window: fills the window (ld(j):
 // the operands of x_j as loaded; cb(raw): x_j from them; scalars(): run by
 // one thread before any cb), then sums the rows into vs; ends with a block
-// barrier (false: `stop`, nothing done).  What bounds it is latency: a load
+// barrier (false: stopped, nothing done).  What bounds it is latency: a load
 // from L2 takes about 850 cycles, and a block's chain of them sets the
 // kernel's time.  So the first groups of the warp's stream, its first rows
-// and the first staged entries load before the window, the window's operands
-// four at a time, and then a ring of two groups a warp (48 bytes a lane) runs
+// and the first staged entries, which depend on nothing the solve changes,
+// load before the solver's state is read (head(): the state's scalars and
+// buffers; true: stop) and before the window (400k cells 145.9 -> 140.3 ms
+// against the state first; with the state read first but tested here it
+// costs registers: 143.5), the window's operands four at a time, and then a ring of two groups a warp (48 bytes a lane) runs
 // ahead of the sums over all its slices; four groups cost spills and measured
 // 1 % slower.  The ring's loads are unconditional and of one size: behind
 // conditions the compiler waits for each (5.4 thousand cycles for the slices
 // of a 256-row block instead of 2.7).  Against the form that staged every
 // product and summed 32 neighbouring rows a warp, the initial place of 400k
 // cells went 183 -> 148 ms, of 1M cells 369 -> 320, of 30k 65.6 -> 62.3.
-template <class Ld, class Cb, class Sc>
-__device__ __forceinline__ bool block_product(const IpDev& D, int axis, int vb, int stop, Ld ld, Cb cb, Sc scalars,
+template <class Head, class Ld, class Cb, class Sc>
+__device__ __forceinline__ bool block_product(const IpDev& D, int axis, int vb, Head head, Ld ld, Cb cb, Sc scalars,
                                               BlockRows& b) {
   extern __shared__ float stage_all[];
   static_assert(kXWin + kSliceTable <= (kB / 32) * kStage, "a windowed block's rows and table fit the stages");
@@ -1034,16 +1037,12 @@ __device__ __forceinline__ bool block_product(const IpDev& D, int axis, int vb, 
   b.vs = stage_all;
   float* xs = stage_all + nw * kStage;
   b.xs = xs;
-  if (stop) return false;                            // (with the table's loads under way)
   if (b.span == 0) {
+    if (head()) return false;
     if (threadIdx.x == 0) scalars();
     __syncthreads();
     return true;
   }
-  // the window's first operands, four elements of each
-  decltype(ld(0)) raw[4];
-#pragma unroll
-  for (int u = 0; u < 4; u++) raw[u] = ld(b.lo + min((int)threadIdx.x + u * kB, b.span - 1));
   float* stage = stage_all + D.rows_blk;
   uint32_t* tab = reinterpret_cast<uint32_t*>(stage_all + nw * kStage - kSliceTable);
   const int own = b.r0 - b.lo;
@@ -1070,6 +1069,14 @@ __device__ __forceinline__ bool block_product(const IpDev& D, int axis, int vb, 
   uint2 pc = make_uint2(0u, 0u);
   if ((int)threadIdx.x < n4) { pv = __ldg(sv + threadIdx.x); pc = __ldg(sc4 + threadIdx.x); }
   if ((int)threadIdx.x < n_tab) tab[threadIdx.x] = width_t;
+  // (the compiler would put the state's loads first, and the block wait for
+  // them before its matrix loads)
+  asm volatile("" ::: "memory");
+  if (head()) return false;
+  // the window's first operands, four elements of each
+  decltype(ld(0)) raw[4];
+#pragma unroll
+  for (int u = 0; u < 4; u++) raw[u] = ld(b.lo + min((int)threadIdx.x + u * kB, b.span - 1));
   if (threadIdx.x == 0) scalars();
   __syncthreads();
   for (int k = threadIdx.x;;) {
@@ -1183,16 +1190,16 @@ __device__ __forceinline__ bool block_product(const IpDev& D, int axis, int vb, 
 }
 
 // op of the thread's first row of block vb (loaded ahead of the products)
-__device__ __forceinline__ float first_row_operand(const IpDev& D, int vb, const float* __restrict__ op) {
+__device__ __forceinline__ float first_row_operand(const IpDev& D, int vb, const float* op) {
   const int i = vb * D.rows_blk + (int)threadIdx.x;
-  return (int)threadIdx.x < D.rows_blk && i < D.n_mov ? __ldg(op + i) : 0.0f;
+  return (int)threadIdx.x < D.rows_blk && i < D.n_mov ? op[i] : 0.0f;
 }
 
 // f(i, (A x)_i, op[i]) for the block's rows in the thread's order: first is
 // op of its first row; the others' load four at a time before the f that use
 // them (whose stores the loads could not pass).
 template <class F>
-__device__ __forceinline__ void for_block_rows(const BlockRows& b, const float* __restrict__ op, float first, F f) {
+__device__ __forceinline__ void for_block_rows(const BlockRows& b, const float* op, float first, F f) {
   int i = b.r0 + threadIdx.x;
   if (i < b.r1) f(i, b.vs[i - b.r0], first);
   for (i += kB; i < b.r1; i += 4 * kB) {
@@ -1280,9 +1287,13 @@ __device__ __forceinline__ void bi_residual_body(const IpDev& D, int init, int m
   float* r0 = D.r0 + axis * n;
   float v[2] = {0.0f, 0.0f};
   auto gx = [&](int j) { return x[j]; };
-  const float first = first_row_operand(D, vb, bb);
+  float first = 0.0f;
   BlockRows br;
-  if (!block_product(D, axis, vb, !init && (S.done || !S.need_restart), gx, [](float v) { return v; }, [] {}, br)) return;
+  auto head = [&] {
+    first = first_row_operand(D, vb, bb);
+    return !init && (S.done || !S.need_restart);
+  };
+  if (!block_product(D, axis, vb, head, gx, [](float v) { return v; }, [] {}, br)) return;
   auto epi = [&](int i, float ax, float bi) {
     const float ri = bi - ax;
     r[i] = ri;
@@ -1322,12 +1333,18 @@ __device__ __forceinline__ void bi_pv_body(const IpDev& D, int vb, int vgrid, in
   float* stage = warp_stage();
   const BiState& S = D.st[axis];
   __shared__ float sc[2];
-  const int par = S.par, stop = S.done | S.need_restart;
-  const float first = first_row_operand(D, vb, D.r0 + axis * D.n_mov);
-  const float* po = pv_buf(D.p, D, par, axis);
-  const float* vo = pv_buf(D.v, D, par, axis);
-  float* pn = pv_buf(D.p, D, par ^ 1, axis);
-  float* vn = pv_buf(D.v, D, par ^ 1, axis);
+  float first = 0.0f;
+  const float *po = nullptr, *vo = nullptr;
+  float *pn = nullptr, *vn = nullptr;
+  auto head = [&] {
+    const int par = S.par, stop = S.done | S.need_restart;
+    first = first_row_operand(D, vb, D.r0 + axis * D.n_mov);
+    po = pv_buf(D.p, D, par, axis);
+    vo = pv_buf(D.v, D, par, axis);
+    pn = pv_buf(D.p, D, par ^ 1, axis);
+    vn = pv_buf(D.v, D, par ^ 1, axis);
+    return stop;
+  };
   const float* r = D.r + axis * D.n_mov;
   const float* r0 = D.r0 + axis * D.n_mov;
   struct Raw { float p, v, r; };
@@ -1336,7 +1353,7 @@ __device__ __forceinline__ void bi_pv_body(const IpDev& D, int vb, int vgrid, in
   auto gx = [&](int j) { return cb(ld(j)); };
   // beta once per block: FP64 division is slow on this part
   BlockRows br;
-  if (!block_product(D, axis, vb, stop, ld, cb, [&] {
+  if (!block_product(D, axis, vb, head, ld, cb, [&] {
         const double beta = (S.rho / S.rho_old) * (S.alpha / S.w);
         sc[0] = (float)beta;            // Eigen's scalars are float
         sc[1] = (float)S.w;
@@ -1364,9 +1381,13 @@ __device__ __forceinline__ void bi_pv_body(const IpDev& D, int vb, int vgrid, in
 __device__ __forceinline__ void bi_st_body(const IpDev& D, int vb, int vgrid, int axis) {
   float* stage = warp_stage();
   const BiState& S = D.st[axis];
-  const int stop = S.done | S.need_restart;
-  const float af = (float)S.alpha;
-  const float* vn = pv_buf(D.v, D, S.par ^ 1, axis);
+  float af = 0.0f;
+  const float* vn = nullptr;
+  auto head = [&] {
+    af = (float)S.alpha;
+    vn = pv_buf(D.v, D, S.par ^ 1, axis);
+    return S.done | S.need_restart;
+  };
   const float* r = D.r + axis * D.n_mov;
   float* s = D.s + axis * D.n_mov;
   float* t = D.t + axis * D.n_mov;
@@ -1375,7 +1396,7 @@ __device__ __forceinline__ void bi_st_body(const IpDev& D, int vb, int vgrid, in
   auto cb = [&](const Raw& x) { return __fmaf_rn(-af, x.v, x.r); };
   auto gx = [&](int j) { return cb(ld(j)); };
   BlockRows br;
-  if (!block_product(D, axis, vb, stop, ld, cb, [] {}, br)) return;
+  if (!block_product(D, axis, vb, head, ld, cb, [] {}, br)) return;
   float acc[2] = {0.0f, 0.0f};
   auto epi = [&](int i, float ti, float si) {
     t[i] = ti;
