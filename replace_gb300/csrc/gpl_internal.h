@@ -366,7 +366,7 @@ bool set_scatter_shape(DeviceModel& d, int side, int chunk);
 size_t scatter_smem(const DeviceModel& d);
 int scatter_prepare_device();
 int launch_wa(DeviceModel& d, const EvalArgs& a, cudaStream_t s, Timer& t);
-int launch_cell(DeviceModel& d, const EvalArgs& a, int n_phi_blocks, cudaStream_t s, Timer& t);
+int launch_cell(DeviceModel& d, const EvalArgs& a, int n_phi_blocks, bool to_host, cudaStream_t s, Timer& t);
 // the Poisson passes of a job evaluation (area set chosen by EvalCtl)
 int launch_poisson_job(DeviceModel& d, bool want_phi, cudaStream_t s, Timer& t);
 // The tensor-core GEMM form of the Poisson solve (poisson_gemm.cu).

@@ -506,8 +506,8 @@ int put_ctl(gpl_job* j, const EvalCtl& c) {
 }
 
 // WA forces, per-gcell gradients and reductions again (the gcell kernel's
-// last block writes the result record), then the record's copy to the host:
-// a second pass over the same coordinates and bins with new coefficients.
+// last block writes the result record, here and on the host): a second pass
+// over the same coordinates and bins with new coefficients.
 int launch_phase2(gpl_job* j, bool want_phi, int area_set) {
   DeviceModel& d = j->d;
   int rc = launch_wa(d, base_args(j), j->stream, j->timer);
@@ -517,20 +517,18 @@ int launch_phase2(gpl_job* j, bool want_phi, int area_set) {
     rc = launch_sum_phi(d, area_set, j->stream, j->timer, &phi_blocks);
     if (rc) return rc;
   }
-  rc = launch_cell(d, base_args(j), phi_blocks, j->stream, j->timer);
-  if (rc) return rc;
-  GPL_CUDA(cudaMemcpyAsync(d.result_h, d.result, sizeof(EvalResult), cudaMemcpyDeviceToHost, j->stream));
-  return GPL_OK;
+  return launch_cell(d, base_args(j), phi_blocks, true, j->stream, j->timer);
 }
 
 // One evaluation's launches: scatter (with the predictor), then the Poisson
 // passes with the WA kernel on the side stream beside them (WA needs only
 // the predicted coordinates, Poisson only the areas), joined before the gcell
-// kernel, and the result record's copy to the host.  The Poisson passes are
-// the longer chain and go first: launched after WA, their first blocks wait
-// for its (loop of 10k cells 42.1 -> 40.6 us an iteration, 1M 204 -> 199).  With kernel timing on,
-// everything stays on the job's stream so that each class is timed alone.
-int launch_eval(gpl_job* j, bool want_phi, int area_set, bool copy_result = true) {
+// kernel, whose last block writes the result record, on the host too.  The
+// Poisson passes are the longer chain and go first: launched after WA, their
+// first blocks wait for its (loop of 10k cells 42.1 -> 40.6 us an iteration,
+// 1M 204 -> 199).  With kernel timing on, everything stays on the job's stream
+// so that each class is timed alone.
+int launch_eval(gpl_job* j, bool want_phi, int area_set, bool to_host = true) {
   DeviceModel& d = j->d;
   int rc = launch_scatter(d, base_args(j), j->stream, j->timer);
   if (rc) return rc;
@@ -550,11 +548,7 @@ int launch_eval(gpl_job* j, bool want_phi, int area_set, bool copy_result = true
     rc = launch_sum_phi(d, area_set, j->stream, j->timer, &phi_blocks);
     if (rc) return rc;
   }
-  rc = launch_cell(d, base_args(j), phi_blocks, j->stream, j->timer);
-  if (rc) return rc;
-  if (copy_result)
-    GPL_CUDA(cudaMemcpyAsync(d.result_h, d.result, sizeof(EvalResult), cudaMemcpyDeviceToHost, j->stream));
-  return GPL_OK;
+  return launch_cell(d, base_args(j), phi_blocks, to_host, j->stream, j->timer);
 }
 
 int finish(gpl_job* j) {
@@ -634,8 +628,8 @@ int choose_poisson_path(gpl_job* j) {
   return GPL_OK;
 }
 
-// The whole evaluation as one CUDA graph (control-record upload, kernels,
-// result download); every evaluation of the job replays it.
+// The whole evaluation as one CUDA graph (control-record upload, kernels);
+// every evaluation of the job replays it.
 int build_graph(gpl_job* j) {
   if (!j->m.p.use_graph || j->graph_exec) return GPL_OK;
   int rc0 = poisson_prepare_device();
