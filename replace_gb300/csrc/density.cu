@@ -38,6 +38,7 @@ struct ScatterArgs {
   float2* coordi[2];
   unsigned long long* area[2];  // two sets of inst [nb], filler [nb]
   const EvalCtl* ctl;
+  EvalCtl* ctl_dev;           // copy of ctl for the evaluation's other kernels (null: ctl is it)
   int one_word;                 // a window's sums fit 32 bits (scatter_one_word)
   int fits32;                   // so does every single value
 };
@@ -314,6 +315,8 @@ template <bool kOneWord>
 __global__ void __launch_bounds__(kBlock, 5) k_scatter(const __grid_constant__ ScatterArgs A,
                                                        const __grid_constant__ TileArgs T, const int32_t* big, int n_big) {
   extern __shared__ __align__(16) unsigned win[];  // [words][2][wy][wx]: sums, or low 16-bit then high 16-bit sums
+  if (A.ctl_dev && blockIdx.x == 0 && threadIdx.x < sizeof(EvalCtl) / 4)
+    reinterpret_cast<unsigned*>(A.ctl_dev)[threadIdx.x] = reinterpret_cast<const unsigned*>(A.ctl)[threadIdx.x];
   if ((int)blockIdx.x < n_big) scatter_big_body(A, big, (int)blockIdx.x);
   else scatter_body<kOneWord>(A, T, (int)blockIdx.x - n_big, win);
 }
@@ -669,6 +672,7 @@ ScatterArgs scatter_args(const DeviceModel& d) {
   A.coordi[0] = d.coordi[0]; A.coordi[1] = d.coordi[1];
   A.area[0] = d.area[0]; A.area[1] = d.area[1];
   A.ctl = d.ctl;
+  A.ctl_dev = nullptr;
   return A;
 }
 
@@ -707,8 +711,9 @@ CellArgs cell_args(const DeviceModel& d, const EvalArgs& a, int n_phi_blocks) {
 }
 }  // namespace
 
-int launch_scatter(DeviceModel& d, const EvalArgs& a, cudaStream_t s, Timer& t) {
-  const ScatterArgs A = scatter_args(d);
+int launch_scatter(DeviceModel& d, const EvalArgs& a, bool ctl_from_host, cudaStream_t s, Timer& t) {
+  ScatterArgs A = scatter_args(d);
+  if (ctl_from_host) { A.ctl = d.ctl_h; A.ctl_dev = d.ctl; }
   const TileArgs T = tile_args(d);
   (void)a;
   t.begin(kKScatter);

@@ -336,7 +336,7 @@ int poisson_passes(const PoissonGrid& g, unsigned long long* const* area_pair,
 int poisson_blocks_a(int nx, int ny);
 void make_w4(int n, std::vector<float2>& w);
 
-int launch_scatter(DeviceModel& d, const EvalArgs& a, cudaStream_t s, Timer& t);
+int launch_scatter(DeviceModel& d, const EvalArgs& a, bool ctl_from_host, cudaStream_t s, Timer& t);
 // Orders the gcells by the bin tile of their centres in slp[slot] (counting
 // sort) and builds the scatter's chunk table; slot < 0: the slot the device
 // control record's predictor starts from (ctl->i_src).

@@ -528,9 +528,9 @@ int launch_phase2(gpl_job* j, bool want_phi, int area_set) {
 // first blocks wait for its (loop of 10k cells 42.1 -> 40.6 us an iteration,
 // 1M 204 -> 199).  With kernel timing on, everything stays on the job's stream
 // so that each class is timed alone.
-int launch_eval(gpl_job* j, bool want_phi, int area_set, bool to_host = true) {
+int launch_eval(gpl_job* j, bool want_phi, int area_set, bool to_host = true, bool ctl_from_host = false) {
   DeviceModel& d = j->d;
-  int rc = launch_scatter(d, base_args(j), j->stream, j->timer);
+  int rc = launch_scatter(d, base_args(j), ctl_from_host, j->stream, j->timer);
   if (rc) return rc;
   const bool fork = j->side && !j->timer.enabled;
   if (fork) {
@@ -628,8 +628,8 @@ int choose_poisson_path(gpl_job* j) {
   return GPL_OK;
 }
 
-// The whole evaluation as one CUDA graph (control-record upload, kernels);
-// every evaluation of the job replays it.
+// The whole evaluation as one CUDA graph (the scatter takes the control record
+// from the host); every evaluation of the job replays it.
 int build_graph(gpl_job* j) {
   if (!j->m.p.use_graph || j->graph_exec) return GPL_OK;
   int rc0 = poisson_prepare_device();
@@ -644,8 +644,7 @@ int build_graph(gpl_job* j) {
     j->timer.enabled = te;
     return GPL_OK;                       // stream cannot be captured: direct launches
   }
-  cudaMemcpyAsync(j->d.ctl, j->d.ctl_h, sizeof(EvalCtl), cudaMemcpyHostToDevice, j->stream);
-  rc = launch_eval(j, false, 0);
+  rc = launch_eval(j, false, 0, true, true);
   cudaError_t e = cudaStreamEndCapture(j->stream, &g);
   j->graph_kernels = j->timer.kernels - k0;
   j->timer.kernels = k0;
@@ -757,10 +756,10 @@ int choose_scatter_shape(gpl_job* j, int slot) {
       seen[n_seen][0] = d.tile_w; seen[n_seen][1] = d.tile_h; seen[n_seen][2] = d.piece;
       n_seen++;
       rc = launch_tile_order(d, slot, j->stream, quiet);
-      if (!rc) rc = launch_scatter(d, base_args(j), j->stream, quiet);    // warm-up
+      if (!rc) rc = launch_scatter(d, base_args(j), false, j->stream, quiet);    // warm-up
       if (rc) break;
       cudaEventRecord(a, j->stream);
-      for (int r = 0; r < kReps && !rc; r++) rc = launch_scatter(d, base_args(j), j->stream, quiet);
+      for (int r = 0; r < kReps && !rc; r++) rc = launch_scatter(d, base_args(j), false, j->stream, quiet);
       cudaEventRecord(b, j->stream);
       if (rc) break;
       float ms = 0.0f;
