@@ -140,6 +140,37 @@ __device__ __forceinline__ float fast_exp(float a) {
   return a;
 }
 
+// Two floats in one 64-bit register: one packed instruction, each element
+// rounded like the scalar operation.
+struct F2 { unsigned long long v; };
+__device__ __forceinline__ F2 pack2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(F2 p, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v));
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+
+// fast_exp of two values: equal to it bit for bit (the product with 2^-10 is
+// exact, or too small to change 1).
+__device__ __forceinline__ F2 fast_exp2(F2 a) {
+  a = fma2(a, pack2(0.0009765625f, 0.0009765625f), pack2(1.0f, 1.0f));
+#pragma unroll
+  for (int i = 0; i < 10; i++) a = mul2(a, a);
+  return a;
+}
+
 // Block sums of N values; thread 0 writes out_base[k * stride + index]
 // (index defaults to the block index).
 template <int N>

@@ -79,11 +79,15 @@ __device__ __forceinline__ int2 pin_pos(const WaEval<kW>& V, const int4& r) {
 }
 
 // The four WA exponentials of one pin (src/nesterovBase.cpp:1320-1355);
-// a direction whose exponent is not above minWireLengthForceBar contributes 0
-// and has its flag cleared.
+// a direction whose exponent is not above minWireLengthForceBar contributes 0.
+// The kernel is bound by the instructions it issues (57 million a million
+// cells): two exponentials go through each packed multiply, computed for both
+// sides of the bar and selected (12.5k gcells 8.1 -> 7.4 us, 1.25M 66.5 ->
+// 63.7).  The sums are not packed: a packed multiply and add is fused by the
+// compiler whatever the rounding asked for, and with separate adds the packing
+// costs spills at 32 registers (63.5).
 struct PinExp {
   float e[4];      // min x, max x, min y, max y
-  unsigned flags;  // bit k set: e[k] is used
 };
 
 __device__ __forceinline__ PinExp pin_exps(int2 p, int lx, int ux, int ly, int uy, float cx, float cy,
@@ -91,12 +95,11 @@ __device__ __forceinline__ PinExp pin_exps(int2 p, int lx, int ux, int ly, int u
   PinExp r;
   const float a[4] = {__fmul_rn((float)(lx - p.x), cx), __fmul_rn((float)(p.x - ux), cx),
                       __fmul_rn((float)(ly - p.y), cy), __fmul_rn((float)(p.y - uy), cy)};
-  r.flags = 0;
+  float v[4];
+  unpack2(fast_exp2(pack2(a[0], a[1])), v[0], v[1]);
+  unpack2(fast_exp2(pack2(a[2], a[3])), v[2], v[3]);
 #pragma unroll
-  for (int k = 0; k < 4; k++) {
-    r.e[k] = 0.0f;
-    if (a[k] > bar) { r.e[k] = fast_exp(a[k]); r.flags |= 1u << k; }
-  }
+  for (int k = 0; k < 4; k++) r.e[k] = a[k] > bar ? v[k] : 0.0f;
   return r;
 }
 
@@ -201,16 +204,17 @@ __device__ __forceinline__ void pair_exps(int2 p0, int2 p1, int lx, int ux, int 
                        __fmul_rn((float)(ly - p0.y), cy), __fmul_rn((float)(p0.y - uy), cy)};
   const float a1[4] = {__fmul_rn((float)(lx - p1.x), cx), __fmul_rn((float)(p1.x - ux), cx),
                        __fmul_rn((float)(ly - p1.y), cy), __fmul_rn((float)(p1.y - uy), cy)};
-  E0.flags = E1.flags = 0;
+  // the smaller exponent is the non-extreme pin's (or 0 for a tie)
+  float am[4], v[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) am[k] = fminf(a0[k], a1[k]);
+  unpack2(fast_exp2(pack2(am[0], am[1])), v[0], v[1]);
+  unpack2(fast_exp2(pack2(am[2], am[3])), v[2], v[3]);
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    // the smaller exponent is the non-extreme pin's (or 0 for a tie)
-    const float am = fminf(a0[k], a1[k]);
-    const float v = am > bar ? fast_exp(am) : 0.0f;
-    E0.e[k] = 0.0f;
-    E1.e[k] = 0.0f;
-    if (a0[k] > bar) { E0.e[k] = a0[k] == am ? v : 1.0f; E0.flags |= 1u << k; }
-    if (a1[k] > bar) { E1.e[k] = a1[k] == am ? v : 1.0f; E1.flags |= 1u << k; }
+    const float u = am[k] > bar ? v[k] : 0.0f;
+    E0.e[k] = a0[k] > bar ? (a0[k] == am[k] ? u : 1.0f) : 0.0f;
+    E1.e[k] = a1[k] > bar ? (a1[k] == am[k] ? u : 1.0f) : 0.0f;
   }
 }
 
@@ -286,7 +290,6 @@ __device__ __forceinline__ long long wa_group(const WaArgs& A, const WaEval<kW>&
     E = pin_exps(p, lx, ux, ly, uy, V.cx, V.cy, A.bar);
     sums_of(p, E, S);
   } else {
-    E.flags = 0;
 #pragma unroll
     for (int t = 0; t < 4; t++) E.e[t] = 0.0f;
 #pragma unroll
