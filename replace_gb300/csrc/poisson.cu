@@ -585,26 +585,48 @@ __device__ __forceinline__ void rot64(float& re, float& im, int m) {
   im = r * sn + i * c;
 }
 
-// In-register M-point DFT (M = 8, 16 or 32), radix-2 decimation in frequency:
-// natural input order, register r ends with output brev(r).  Twiddles
-// exp(kSign 2 pi i j / len) = exp(kSign 2 pi i (j 64/len) / 64) are
-// compile-time constants after unrolling.
+// (re, im) times exp(kSign 2 pi i m / 64), m < 64 a compile-time constant.
+template <int kSign>
+__device__ __forceinline__ void rot64_full(float& re, float& im, int m) {
+  if (m >= 32) { re = -re; im = -im; m -= 32; }
+  rot64<kSign>(re, im, m);
+}
+
+// In-register M-point DFT (M = 8, 16 or 32), decimation in frequency: natural
+// input order, register r ends with output brev(r).  Two radix-2 stages at a
+// time, so that a value meets one twiddle where two stages would give it two
+// (an odd last stage has none): fewer roundings and fewer instructions than
+// stage by stage.  Twiddles exp(kSign 2 pi i j / len) = exp(kSign 2 pi i
+// (j 64/len) / 64) are compile-time constants after unrolling.
 template <int M, int kSign>
 __device__ __forceinline__ void dft_reg(float (&re)[M], float (&im)[M]) {
 #pragma unroll
-  for (int len = M; len >= 2; len >>= 1) {
-    const int half = len >> 1;
+  for (int len = M; len >= 4; len >>= 2) {
+    const int q = len >> 2;
 #pragma unroll
     for (int start = 0; start < M; start += len) {
 #pragma unroll
-      for (int j = 0; j < half; j++) {
-        const int a = start + j, b = a + half;
-        const float ar = re[a], ai = im[a], br = re[b], bi = im[b];
-        re[a] = ar + br;
-        im[a] = ai + bi;
-        re[b] = ar - br;
-        im[b] = ai - bi;
-        rot64<kSign>(re[b], im[b], j * (64 / len));
+      for (int j = 0; j < q; j++) {
+        const int a = start + j, b = a + q, c = b + q, d = c + q;
+        const float sr = re[a] + re[c], si = im[a] + im[c], tr = re[a] - re[c], ti = im[a] - im[c];
+        const float ur = re[b] + re[d], ui = im[b] + im[d], vr = re[b] - re[d], vi = im[b] - im[d];
+        // kSign i (b - d)
+        const float wr = kSign > 0 ? -vi : vi, wi = kSign > 0 ? vr : -vr;
+        re[a] = sr + ur; im[a] = si + ui;
+        re[b] = sr - ur; im[b] = si - ui;
+        re[c] = tr + wr; im[c] = ti + wi;
+        re[d] = tr - wr; im[d] = ti - wi;
+        rot64_full<kSign>(re[b], im[b], 2 * j * (64 / len));
+        rot64_full<kSign>(re[c], im[c], j * (64 / len));
+        rot64_full<kSign>(re[d], im[d], 3 * j * (64 / len));
+      }
+    }
+    if (len == 8) {                   // the last stage, of pairs
+#pragma unroll
+      for (int a = 0; a < M; a += 2) {
+        const float ar = re[a], ai = im[a];
+        re[a] = ar + re[a + 1]; im[a] = ai + im[a + 1];
+        re[a + 1] = ar - re[a + 1]; im[a + 1] = ai - im[a + 1];
       }
     }
   }
