@@ -133,13 +133,6 @@ __device__ __forceinline__ float ll_to_float(long long v) {
   return (v >= 0 && v < 2147483648ll) ? __int2float_rn((int)v) : __ll2float_rn(v);
 }
 
-__device__ __forceinline__ float fast_exp(float a) {
-  a = __fadd_rn(1.0f, __fmul_rn(a, 0.0009765625f));
-#pragma unroll
-  for (int i = 0; i < 10; i++) a = __fmul_rn(a, a);
-  return a;
-}
-
 // Two floats in one 64-bit register: one packed instruction, each element
 // rounded like the scalar operation.
 struct F2 { unsigned long long v; };
@@ -162,8 +155,9 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
   return r;
 }
 
-// fast_exp of two values: equal to it bit for bit (the product with 2^-10 is
-// exact, or too small to change 1).
+// fastExp (src/nesterovBase.cpp:1568-1582) of two values: (1 + a / 1024)^1024
+// by ten squarings.  The first step fused rounds as a product and a sum would:
+// the product with 2^-10 is exact, or too small to change 1.
 __device__ __forceinline__ F2 fast_exp2(F2 a) {
   a = fma2(a, pack2(0.0009765625f, 0.0009765625f), pack2(1.0f, 1.0f));
 #pragma unroll

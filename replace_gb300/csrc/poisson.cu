@@ -601,8 +601,9 @@ __device__ __forceinline__ void rot64_full(float& re, float& im, int m) {
 // 2.25 and 2.03, 2048 x 2048 2.40 and 2.17, 512 x 2048 3.24 and 2.97; the block
 // form's is 1.86 and 2.61 on the last two, so these grids pay 14 to 17 % of error
 // for a solve of 92 us instead of 315 (decimation in time with the products
-// fused into the additions was worse: 2.56 at 2048 x 2048).  Twiddles exp(kSign 2 pi i j / len) = exp(kSign 2 pi i
-// (j 64/len) / 64) are compile-time constants after unrolling.
+// fused into the additions was worse: 2.56 at 2048 x 2048).  Twiddles
+// exp(kSign 2 pi i j / len) = exp(kSign 2 pi i (j 64/len) / 64) are compile-time
+// constants after unrolling.
 template <int M, int kSign>
 __device__ __forceinline__ void dft_reg(float (&re)[M], float (&im)[M]) {
 #pragma unroll

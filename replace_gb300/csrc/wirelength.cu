@@ -196,8 +196,8 @@ __device__ __forceinline__ void group_sum8(float (&S)[8]) {
 
 // The exponentials of both pins of a two-pin net, equal to pin_exps of each
 // pin: in every direction one pin is the extreme (exponent exactly 0, and
-// fast_exp(0) = 1 exactly), so only the other pin's exponential is computed,
-// one fast_exp per direction instead of two.
+// its exponential exactly 1), so only the other pin's exponential is computed,
+// one per direction instead of two.
 __device__ __forceinline__ void pair_exps(int2 p0, int2 p1, int lx, int ux, int ly, int uy, float cx, float cy,
                                           float bar, PinExp& E0, PinExp& E1) {
   const float a0[4] = {__fmul_rn((float)(lx - p0.x), cx), __fmul_rn((float)(p0.x - ux), cx),
