@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -489,6 +490,39 @@ int batch_member_status(gpl_job* j, gpl_nesterov_stats* stats);
 // device addresses are keyed on it: after cudaDeviceReset the device gets a
 // new primary context, whose memory and symbol addresses are new.
 unsigned long long current_context_id();
+
+// What a piece of code prepares once per context (function attributes and the
+// contents of __device__ arrays go with the context): T as the preparation
+// left it.  A process makes few contexts, so the entries stay.
+template <class T>
+class PerContext {
+  struct Entry { int dev; unsigned long long ctx; T value; };
+  std::mutex mu_;
+  std::vector<Entry> entries_;
+
+ public:
+  // Runs prepare(T&) in the calling thread's current context unless it has
+  // succeeded there before; *out receives the value.
+  template <class F>
+  int get(T* out, F prepare) {
+    int dev = 0;
+    GPL_CUDA(cudaGetDevice(&dev));
+    unsigned long long ctx = current_context_id();
+    if (!ctx) {                          // no context yet, or one that was reset
+      GPL_CUDA(cudaSetDevice(dev));
+      ctx = current_context_id();
+    }
+    std::lock_guard<std::mutex> lk(mu_);
+    for (const Entry& e : entries_)
+      if (e.dev == dev && e.ctx == ctx) { *out = e.value; return GPL_OK; }
+    T value{};
+    const int rc = prepare(value);
+    if (rc) return rc;
+    entries_.push_back({dev, ctx, value});
+    *out = value;
+    return GPL_OK;
+  }
+};
 void make_freq(int nx, int ny, int bsx, int bsy, std::vector<float>& wx, std::vector<float>& wy);
 
 }  // namespace gpl

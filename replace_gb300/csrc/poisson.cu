@@ -1185,19 +1185,8 @@ bool cluster_prepare() {
   return ok;
 }
 
-// Whether the cluster form takes this grid on the current device (16 CTAs are
-// above the portable cluster size; a device that cannot place them keeps the
-// block form).
-bool cluster_form(int nx, int ny) {
-  if (nx != ny || (nx != 64 && nx != 128 && nx != 256)) return false;
-  static std::mutex mu;
-  static signed char state[64] = {0};                      // per device: 0 unknown, 1 yes, -1 no
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-  std::lock_guard<std::mutex> lk(mu);
-  if (state[dev] == 0) state[dev] = cluster_prepare<64>() && cluster_prepare<128>() && cluster_prepare<256>() ? 1 : -1;
-  return state[dev] > 0;
-}
+// Whether the cluster form takes this grid, where it can be placed at all.
+bool cluster_grid(int nx, int ny) { return nx == ny && (nx == 64 || nx == 128 || nx == 256); }
 
 // Whether the group form takes this grid.
 bool group_form(int nx, int ny) {
@@ -1261,43 +1250,54 @@ int poisson_blocks_a(int nx, int ny) {
   return (ny / 2 + r - 1) / r;
 }
 
-// The dynamic shared-memory limit is a per-device function attribute.
+namespace {
+// What a context holds for the Poisson kernels besides their shared-memory
+// limits and twiddle tables.
+struct PoissonContext {
+  bool cluster = false;   // 16 CTAs (above the portable size) can be placed; otherwise the block form stays
+};
+
+int poisson_context(PoissonContext* out) {
+  static PerContext<PoissonContext> contexts;
+  return contexts.get(out, [](PoissonContext& pc) -> int {
+    const int big = 200 * 1024;
+    GPL_CUDA(cudaFuncSetAttribute(k_poisson_a, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    GPL_CUDA(cudaFuncSetAttribute(k_poisson_b, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    GPL_CUDA(cudaFuncSetAttribute(k_poisson_c, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    GPL_CUDA(group_prepare<256>());
+    GPL_CUDA(group_prepare<512>());
+    GPL_CUDA(group_prepare<1024>());
+    GPL_CUDA(group_prepare<2048>());
+    pc.cluster = cluster_prepare<64>() && cluster_prepare<128>() && cluster_prepare<256>();
+    for (int n : {64, 128, 256, 512, 1024, 2048}) {
+      // the group form's twiddles, [k2 * G + n1] = exp(-2 pi i n1 k2 / n)
+      const int g = n <= 128 ? GroupFft<64>::kG : n == 256 ? GroupFft<256>::kG : n == 2048 ? GroupFft<2048>::kG : GroupFft<512>::kG;
+      static_assert(GroupFft<512>::kG == GroupFft<1024>::kG && GroupFft<64>::kG == GroupFft<128>::kG, "one width");
+      std::vector<float2> t(n);
+      for (int k2 = 0; k2 < n / g; k2++)
+        for (int n1 = 0; n1 < g; n1++) {
+          const double a = -2.0 * M_PI * (double)(n1 * k2) / (double)n;
+          t[k2 * g + n1] = make_float2((float)cos(a), (float)sin(a));
+        }
+      const size_t bytes = n * sizeof(float2);
+      if (n == 64) GPL_CUDA(cudaMemcpyToSymbol(g_tw64, t.data(), bytes));
+      else if (n == 128) GPL_CUDA(cudaMemcpyToSymbol(g_tw128, t.data(), bytes));
+      else if (n == 256) GPL_CUDA(cudaMemcpyToSymbol(g_tw256, t.data(), bytes));
+      else if (n == 512) GPL_CUDA(cudaMemcpyToSymbol(g_tw512, t.data(), bytes));
+      else if (n == 1024) GPL_CUDA(cudaMemcpyToSymbol(g_tw1024, t.data(), bytes));
+      else GPL_CUDA(cudaMemcpyToSymbol(g_tw2048, t.data(), bytes));
+    }
+    // (a copy from pageable memory may return before it has arrived, and a
+    // caller's non-blocking stream does not wait for it)
+    GPL_CUDA(cudaStreamSynchronize(nullptr));
+    return GPL_OK;
+  });
+}
+}  // namespace
+
 int poisson_prepare_device() {
-  static std::mutex mu;
-  static bool done[64] = {false};
-  int dev = 0;
-  GPL_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64) { set_error("device ordinal out of range"); return GPL_ERR_INVALID_ARG; }
-  std::lock_guard<std::mutex> lk(mu);
-  if (done[dev]) return GPL_OK;
-  const int big = 200 * 1024;
-  GPL_CUDA(cudaFuncSetAttribute(k_poisson_a, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  GPL_CUDA(cudaFuncSetAttribute(k_poisson_b, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  GPL_CUDA(cudaFuncSetAttribute(k_poisson_c, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  GPL_CUDA(group_prepare<256>());
-  GPL_CUDA(group_prepare<512>());
-  GPL_CUDA(group_prepare<1024>());
-  GPL_CUDA(group_prepare<2048>());
-  for (int n : {64, 128, 256, 512, 1024, 2048}) {
-    // the group form's twiddles, [k2 * G + n1] = exp(-2 pi i n1 k2 / n)
-    const int g = n <= 128 ? GroupFft<64>::kG : n == 256 ? GroupFft<256>::kG : n == 2048 ? GroupFft<2048>::kG : GroupFft<512>::kG;
-    static_assert(GroupFft<512>::kG == GroupFft<1024>::kG && GroupFft<64>::kG == GroupFft<128>::kG, "one width");
-    std::vector<float2> t(n);
-    for (int k2 = 0; k2 < n / g; k2++)
-      for (int n1 = 0; n1 < g; n1++) {
-        const double a = -2.0 * M_PI * (double)(n1 * k2) / (double)n;
-        t[k2 * g + n1] = make_float2((float)cos(a), (float)sin(a));
-      }
-    const size_t bytes = n * sizeof(float2);
-    if (n == 64) GPL_CUDA(cudaMemcpyToSymbol(g_tw64, t.data(), bytes));
-    else if (n == 128) GPL_CUDA(cudaMemcpyToSymbol(g_tw128, t.data(), bytes));
-    else if (n == 256) GPL_CUDA(cudaMemcpyToSymbol(g_tw256, t.data(), bytes));
-    else if (n == 512) GPL_CUDA(cudaMemcpyToSymbol(g_tw512, t.data(), bytes));
-    else if (n == 1024) GPL_CUDA(cudaMemcpyToSymbol(g_tw1024, t.data(), bytes));
-    else GPL_CUDA(cudaMemcpyToSymbol(g_tw2048, t.data(), bytes));
-  }
-  done[dev] = true;
-  return GPL_OK;
+  PoissonContext pc;
+  return poisson_context(&pc);
 }
 
 namespace {
@@ -1397,19 +1397,15 @@ bool write_poisson_batch_args(const DeviceModel& d, void* dst_a, void* dst_b, vo
 }
 
 int poisson_batch_prepare_device() {
-  static std::mutex mu;
-  static bool done[64] = {false};
-  int dev = 0;
-  GPL_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64) { set_error("device ordinal out of range"); return GPL_ERR_INVALID_ARG; }
-  std::lock_guard<std::mutex> lk(mu);
-  if (done[dev]) return GPL_OK;
-  const int big = 200 * 1024;
-  GPL_CUDA(cudaFuncSetAttribute(k_poisson_a_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  GPL_CUDA(cudaFuncSetAttribute(k_poisson_b_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  GPL_CUDA(cudaFuncSetAttribute(k_poisson_c_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  done[dev] = true;
-  return GPL_OK;
+  static PerContext<char> contexts;
+  char done;
+  return contexts.get(&done, [](char&) -> int {
+    const int big = 200 * 1024;
+    GPL_CUDA(cudaFuncSetAttribute(k_poisson_a_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    GPL_CUDA(cudaFuncSetAttribute(k_poisson_b_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    GPL_CUDA(cudaFuncSetAttribute(k_poisson_c_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    return GPL_OK;
+  });
 }
 
 int launch_poisson_batch(int pass, const void* args, const int4* items, const int* count, int grid, size_t smem,
@@ -1428,7 +1424,8 @@ int poisson_passes(const PoissonGrid& g, unsigned long long* const* area_pair,
                    const float* density_in, float* density, double* part_overflow,
                    float* spec, float* p1, float* p2, float2* field, float* fx, float* fy,
                    float* phi, cudaStream_t s, Timer* t) {
-  int rc = poisson_prepare_device();
+  PoissonContext pc;
+  int rc = poisson_context(&pc);
   if (rc) return rc;
   const int nx = g.nx, ny = g.ny;
   const PassAArgs A = pass_a_args(g, area_pair, ctl, nonplace, td, density_in, density, part_overflow, spec);
@@ -1465,7 +1462,7 @@ int poisson_passes(const PoissonGrid& g, unsigned long long* const* area_pair,
     GPL_CUDA(cudaGetLastError());
     return GPL_OK;
   }
-  if (density_in && cluster_form(nx, ny)) {
+  if (density_in && pc.cluster && cluster_grid(nx, ny)) {
     PassBArgs B;
     PassCArgs C;
     int grid[3];
