@@ -776,14 +776,15 @@ size_t scatter_smem(const DeviceModel& d) {
 }
 
 int scatter_prepare_device() {
-  static int done = 0;   // per process (one device in use)
-  if (done) return GPL_OK;
-  const int side = kTileSides[sizeof(kTileSides) / sizeof(kTileSides[0]) - 1];
-  const int smem = 4 * (side + 2 * kTileMargin) * (side + 2 * kTileMargin) * 4;
-  GPL_CUDA(cudaFuncSetAttribute(k_scatter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  GPL_CUDA(cudaFuncSetAttribute(k_scatter<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  done = 1;
-  return GPL_OK;
+  static PerContext<char> contexts;
+  char done;
+  return contexts.get(&done, [](char&) -> int {
+    const int side = kTileSides[sizeof(kTileSides) / sizeof(kTileSides[0]) - 1];
+    const int smem = 4 * (side + 2 * kTileMargin) * (side + 2 * kTileMargin) * 4;
+    GPL_CUDA(cudaFuncSetAttribute(k_scatter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    GPL_CUDA(cudaFuncSetAttribute(k_scatter<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    return GPL_OK;
+  });
 }
 
 int launch_tile_order(DeviceModel& d, int slot, cudaStream_t s, Timer& t) {
@@ -950,13 +951,14 @@ void write_cell_batch_args(const DeviceModel& d, const EvalArgs& a, void* dst) {
 }
 
 int scatter_batch_prepare_device() {
-  static int done = 0;
-  if (done) return GPL_OK;
-  const int side = kTileSides[sizeof(kTileSides) / sizeof(kTileSides[0]) - 1];
-  const int smem = 4 * (side + 2 * kTileMargin) * (side + 2 * kTileMargin) * 4;
-  GPL_CUDA(cudaFuncSetAttribute(k_scatter_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  done = 1;
-  return GPL_OK;
+  static PerContext<char> contexts;
+  char done;
+  return contexts.get(&done, [](char&) -> int {
+    const int side = kTileSides[sizeof(kTileSides) / sizeof(kTileSides[0]) - 1];
+    const int smem = 4 * (side + 2 * kTileMargin) * (side + 2 * kTileMargin) * 4;
+    GPL_CUDA(cudaFuncSetAttribute(k_scatter_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    return GPL_OK;
+  });
 }
 
 int launch_density_batch(int phase, const void* args, const int4* items, const int* count, int grid,

@@ -1,6 +1,7 @@
-"""The standalone Poisson solves in a new context: after cudaDeviceReset the
-kernels' twiddle tables, shared-memory limits and cluster-size attribute are
-those of the new context, and every form gives the bits it gave before.
+"""The standalone Poisson solves and new jobs in a new context: after
+cudaDeviceReset the kernels' twiddle tables, shared-memory limits and
+cluster-size attribute are those of the new context, and everything gives the
+bits it gave before.
 
 Each test runs in a process of its own: a reset ends the context of everything
 else in the process.
@@ -65,6 +66,28 @@ for c, w in zip(cases, want):
 print("same")
 """
 
+# 64 x 64 tiles of bins whose sums need two window words: 83 KB of shared memory
+JOBS = """
+from replace_gb300 import Placer, batch_nesterov_run, netlist as N
+nl = N.generate(9_000, 9_450, n_io=60, seed=5)
+
+def outcome(batched):
+    p = Placer(nl, target_density=0.75, initial_place_max_iter=1, bin_grid_cnt_x=64, bin_grid_cnt_y=64,
+               poisson_path=1, scatter_tile=64)
+    p.initial_place()
+    p.nesterov_init()
+    batch_nesterov_run([p], 5) if batched else p.nesterov_run(5)
+    xy = p.gcell_coords()
+    p.close()
+    return xy
+
+want = [outcome(b) for b in (False, True)]
+ok(rt.cudaDeviceReset())
+for b, w in zip((False, True), want):
+    assert np.array_equal(outcome(b), w), b
+print("same")
+"""
+
 
 def run(body):
     r = subprocess.run([sys.executable, "-c", PRELUDE + body], capture_output=True, text=True, timeout=300)
@@ -73,3 +96,7 @@ def run(body):
 
 def test_poisson_solves_after_a_reset(gpu_lib):
     run(SOLVES)
+
+
+def test_jobs_after_a_reset(gpu_lib):
+    run(JOBS)
