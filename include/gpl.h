@@ -329,6 +329,11 @@ gpl_status gpl_get_gcells(struct gpl_job* job, int32_t* drect, float* scale, uin
  * Scratch memory is allocated on first use per device and grid and cached
  * for the device's current context (after cudaDeviceReset the entries of
  * the old context are dropped, not freed, and new scratch is allocated).
+ * Solves may overlap on any streams and threads: the first stream that
+ * solves a grid has scratch of its own, the others share a second one, where
+ * each solve waits on the GPU for the one before it.  A solve may be captured
+ * once its grid has been solved outside a capture; the order of the graph's
+ * launches with other solves of that grid is the caller's.
  * stream: cudaStream_t (NULL = default stream). */
 gpl_status gpl_poisson_solve(int32_t nx, int32_t ny, int32_t bin_size_x,
                              int32_t bin_size_y, const float* density, float* phi,

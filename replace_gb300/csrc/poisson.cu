@@ -1512,17 +1512,27 @@ void make_w4(int n, std::vector<float2>& w) {
   }
 }
 
-// Scratch and tables of the standalone solve, cached per (device, grid).
+// Scratch and tables of the standalone solve, cached per (device, grid).  The
+// scratch carries a solve's spectrum from pass to pass, so solves that may run
+// at once need their own: the first stream that solves a grid owns an entry,
+// whose solves its own order keeps apart, and all other streams share a second
+// one, where a solve waits on the GPU for the one before it.  (One entry whose
+// solves always wait costs a caller of one stream the event calls, 1.5 us of
+// the 35 of a single solve.)
 namespace {
 struct SolveCache {
   int device = -1, nx = 0, ny = 0, bsx = 0, bsy = 0;
   unsigned long long ctx = 0;   // context the memory belongs to
+  unsigned long long owner = 0; // id of the owning stream (never reused)
+  bool shared = false;          // the other streams' entry
+  std::mutex mu;                // held while a solve is enqueued
+  cudaEvent_t done = nullptr;   // shared: behind the last solve
   char* mem = nullptr;
   float *spec = nullptr, *p1 = nullptr, *p2 = nullptr, *wx = nullptr, *wy = nullptr;
   float2 *w4x = nullptr, *w4y = nullptr, *tw = nullptr;
 };
 std::mutex g_cache_mu;
-std::vector<std::unique_ptr<SolveCache>> g_cache;
+std::vector<std::shared_ptr<SolveCache>> g_cache;
 
 typedef CUresult (*CtxGetCurrentFn)(CUcontext*);
 typedef CUresult (*CtxGetIdFn)(CUcontext, unsigned long long*);
@@ -1567,7 +1577,14 @@ extern "C" gpl_status gpl_poisson_solve(int32_t nx, int32_t ny, int32_t bsx, int
   GPL_CUDA(cudaSetDevice(dev));         // initialises the device's context if needed
   const unsigned long long ctx = current_context_id();
   cudaStream_t s = (cudaStream_t)stream;
-  SolveCache* c = nullptr;
+  // a captured solve takes the entry that is there (no allocation and no wait
+  // for work outside the capture): the header leaves its order to the caller
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  GPL_CUDA(cudaStreamIsCapturing(s, &capture));
+  const bool capturing = capture != cudaStreamCaptureStatusNone;
+  unsigned long long sid = 0;
+  if (!capturing) GPL_CUDA(cudaStreamGetId(s, &sid));
+  std::shared_ptr<SolveCache> c;
   {
     std::lock_guard<std::mutex> lk(g_cache_mu);
     // entries of a context that no longer exists (cudaDeviceReset) hold
@@ -1575,11 +1592,20 @@ extern "C" gpl_status gpl_poisson_solve(int32_t nx, int32_t ny, int32_t bsx, int
     for (auto& e : g_cache)
       if (e && e->device == dev && e->ctx != ctx) e.reset();
     g_cache.erase(std::remove(g_cache.begin(), g_cache.end(), nullptr), g_cache.end());
-    for (auto& e : g_cache)
-      if (e->device == dev && e->nx == nx && e->ny == ny && e->bsx == bsx && e->bsy == bsy) c = e.get();
+    std::shared_ptr<SolveCache> owned, others;         // another stream's, the shared one
+    for (auto& e : g_cache) {
+      if (e->device != dev || e->nx != nx || e->ny != ny || e->bsx != bsx || e->bsy != bsy) continue;
+      if (e->shared) others = e;
+      else if (e->owner == sid) c = e;
+      else owned = e;
+    }
+    if (!c) c = capturing && owned ? owned : others;
     if (!c) {
-      SolveCache e;
+      auto n = std::make_shared<SolveCache>();
+      SolveCache& e = *n;
       e.device = dev; e.ctx = ctx; e.nx = nx; e.ny = ny; e.bsx = bsx; e.bsy = bsy;
+      e.shared = owned != nullptr;
+      e.owner = sid;
       const size_t nb = (size_t)nx * ny;
       size_t bytes = 3 * nb * 4 + (nx + ny) * 4 + (nx + ny) * 8 + (kFftMax / 2) * 8 + 8 * 256;
       GPL_CUDA(cudaMalloc(&e.mem, bytes));
@@ -1597,15 +1623,23 @@ extern "C" gpl_status gpl_poisson_solve(int32_t nx, int32_t ny, int32_t bsx, int
       GPL_CUDA(cudaMemcpy(e.w4x, w4x.data(), nx * 8, cudaMemcpyHostToDevice));
       GPL_CUDA(cudaMemcpy(e.w4y, w4y.data(), ny * 8, cudaMemcpyHostToDevice));
       GPL_CUDA(cudaMemcpy(e.tw, tw.data(), tw.size() * 8, cudaMemcpyHostToDevice));
-      g_cache.emplace_back(new SolveCache(e));
-      c = g_cache.back().get();
+      if (e.shared) GPL_CUDA(cudaEventCreateWithFlags(&e.done, cudaEventDisableTiming));
+      // (a copy from pageable memory may return before it has arrived, and a
+      // caller's non-blocking stream does not wait for it)
+      GPL_CUDA(cudaStreamSynchronize(nullptr));
+      g_cache.push_back(n);
+      c = n;
     }
   }
   PoissonGrid g;
   g.nx = nx; g.ny = ny; g.size_x = bsx; g.size_y = bsy;
   g.core_lx = g.core_ly = 0; g.core_ux = nx * bsx; g.core_uy = ny * bsy;
   g.wx = c->wx; g.wy = c->wy; g.w4x = c->w4x; g.w4y = c->w4y; g.tw = c->tw;
+  std::lock_guard<std::mutex> lk(c->mu);
+  const bool ordered = c->shared && !capturing;
+  if (ordered) GPL_CUDA(cudaStreamWaitEvent(s, c->done));
   int rc = poisson_passes(g, nullptr, nullptr, nullptr, 1.0f, density, nullptr, nullptr, c->spec,
                           c->p1, c->p2, nullptr, fx, fy, phi, s, nullptr);
+  if (ordered) GPL_CUDA(cudaEventRecord(c->done, s));
   return (gpl_status)rc;
 }

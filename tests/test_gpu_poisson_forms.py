@@ -82,3 +82,64 @@ def test_batch_takes_group_form_grids(gpu_lib):
         assert np.array_equal(p.gcell_coords(), q.gcell_coords()), g
         p.close()
         q.close()
+
+
+@pytest.mark.parametrize("threads", [False, True])
+@pytest.mark.parametrize("nx,ny,phi", [(512, 256, False), (1024, 1024, True), (64, 32, True), (128, 128, True)])
+def test_streams_share_no_scratch(gpu_lib, nx, ny, phi, threads):
+    """Solves of one grid on several streams, from one host thread and from
+    several, equal those on one stream bit for bit."""
+    import threading
+    import torch
+    from replace_gb300.placer import poisson_solve
+    g = torch.Generator(device="cuda").manual_seed(nx + ny)
+    n = 4
+    rho = [0.5 + torch.rand((ny, nx), generator=g, device="cuda") for _ in range(n)]
+    want = [torch.zeros((3, ny, nx), device="cuda") for _ in range(n)]
+    got = [torch.zeros((3, ny, nx), device="cuda") for _ in range(n)]
+
+    def solve(k, out, stream):
+        poisson_solve(rho[k].data_ptr(), out[0].data_ptr() if phi else 0, out[1].data_ptr(), out[2].data_ptr(),
+                      nx, ny, 380, 1400, stream=stream.cuda_stream)
+    for k in range(n):
+        solve(k, want[k], torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(n)]
+
+    def repeat(ks):
+        for _ in range(40):
+            for k in ks:
+                solve(k, got[k], streams[k])
+    if threads:
+        ts = [threading.Thread(target=repeat, args=([k],)) for k in range(n)]
+        for t in ts:
+            t.start()
+        for t in ts:
+            t.join()
+    else:
+        repeat(range(n))
+    torch.cuda.synchronize()
+    for k in range(n):
+        assert torch.equal(got[k], want[k]), k
+
+
+def test_capture_on_another_stream(gpu_lib):
+    """A grid solved on one stream can be captured on another."""
+    import torch
+    from replace_gb300.placer import poisson_solve
+    nx, ny = 512, 1024
+    rho = 0.5 + torch.rand((ny, nx), device="cuda")
+    out = torch.zeros((2, ny, nx), device="cuda")
+
+    def solve():
+        poisson_solve(rho.data_ptr(), 0, out[0].data_ptr(), out[1].data_ptr(), nx, ny, 380, 1400,
+                      stream=torch.cuda.current_stream().cuda_stream)
+    solve()
+    want = out.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        solve()
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
