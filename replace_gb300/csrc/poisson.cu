@@ -281,6 +281,9 @@ struct PassBArgs {
   const float2* tw;
   const float2* w4;                  // exp(-i pi k / 2ny), k < ny
   float scale;                       // 4 / (nx ny)
+  // group and cluster form (solve_pair): 4 nx / (ny pi^2) and (wy[1] / wx[1])^2,
+  // each as the float nearest and the float nearest to the rest
+  float num[2], aspect[2];
 };
 
 __device__ __noinline__ void poisson_b_body(const PassBArgs& B, int vb, float2* smem) {
@@ -518,7 +521,9 @@ struct GroupFft {
   static_assert(kBuf >= 2 * N, "the transpose holds the sequence");
 };
 
-// exp(-2 pi i n1 k2 / N) at [k2 * G + n1], k2 < E: one coalesced row per k2.
+// exp(-2 pi i n1 k2 / N) at [k2 * G + n1], k2 < E, where an index in the upper
+// half of its range stands for itself minus the range (group_fft): one
+// coalesced row per k2.
 __device__ __align__(16) float2 g_tw64[64];
 __device__ __align__(16) float2 g_tw128[128];
 __device__ __align__(16) float2 g_tw256[256];
@@ -570,6 +575,18 @@ __host__ __device__ constexpr float sin64(int m) {   // 0 <= m < 32
   return m <= 16 ? cos64_quad(16 - m) : cos64_quad(m - 16);
 }
 
+// The inverse transforms' cos(pi / 16) and cos(pi / 8): the floats above the
+// nearest ones, which lie almost as far on the other side (3.0e-8
+// and 3.1e-8 instead of 3.0e-8 and 2.8e-8).  Nearest in both directions, every
+// rotation by them shortens, and the error of a solve's transforms adds up in
+// its low modes; so one direction shortens and the other lengthens (2048 x 2048:
+// Ex 1.78e-7 -> 1.67e-7, phi 1.69e-7 -> 1.56e-7).
+__host__ __device__ constexpr float up64(float c) {
+  const float a = c < 0.0f ? -c : c;
+  const float u = a == cos64_quad(2) ? 0.98078534f : a == cos64_quad(4) ? 0.92387956f : a;
+  return c < 0.0f ? -u : u;
+}
+
 // (re, im) times exp(kSign 2 pi i m / 64), m < 32 a compile-time constant.
 template <int kSign>
 __device__ __forceinline__ void rot64(float& re, float& im, int m) {
@@ -580,7 +597,7 @@ __device__ __forceinline__ void rot64(float& re, float& im, int m) {
     im = kSign > 0 ? r : -r;
     return;
   }
-  const float c = cos64(m), sn = kSign > 0 ? sin64(m) : -sin64(m);
+  const float c = kSign > 0 ? up64(cos64(m)) : cos64(m), sn = kSign > 0 ? up64(sin64(m)) : -sin64(m);
   re = r * c - i * sn;
   im = r * sn + i * c;
 }
@@ -596,12 +613,8 @@ __device__ __forceinline__ void rot64_full(float& re, float& im, int m) {
 // input order, register r ends with output brev(r).  Two radix-2 stages at a
 // time, so that a value meets one twiddle where two stages would give it two
 // (an odd last stage has none): fewer roundings and fewer instructions than
-// stage by stage.  Field error against a 64-bit solve (relative rms of Ex, three
-// densities, 1e-7) stage by stage and so: 512 x 512 2.07 and 2.00, 1024 x 1024
-// 2.25 and 2.03, 2048 x 2048 2.40 and 2.17, 512 x 2048 3.24 and 2.97; the block
-// form's is 1.86 and 2.61 on the last two, so these grids pay 14 to 17 % of error
-// for a solve of 92 us instead of 315 (decimation in time with the products
-// fused into the additions was worse: 2.56 at 2048 x 2048).  Twiddles
+// stage by stage (field error against 64 bits 2.17e-7 instead of 2.40e-7 at
+// 2048 x 2048, before the steps of group_fft and up64).  Twiddles
 // exp(kSign 2 pi i j / len) = exp(kSign 2 pi i (j 64/len) / 64) are compile-time
 // constants after unrolling.
 template <int M, int kSign>
@@ -667,6 +680,17 @@ __device__ __forceinline__ void group_sync() {
 // N-point FFT of buf (natural order in and out, [GroupFft<N>::kBuf] floats,
 // float2 view) by the calling group; kSign -1 forward, +1 unnormalised
 // inverse.  tws: the tw_table<N>() table in shared memory.
+//
+// The four steps take n = n1 + G n2 and k = k2 + E k1 with n1 and k2 of either
+// sign, -G/2 <= n1 < G/2 and -E/2 <= k2 < E/2: the same sums with the first
+// loads and the last stores shifted.  The field lies in the modes next to 0
+// and N, so its twiddles W^(n1 k2) then turn by little, and floats close to 1
+// and 0 are nearer to them than floats on the rest of the circle; with
+// unsigned indices the modes below N turn through all of it.  Error against 64
+// bits (largest of phi, Ex, Ey, mean of eight densities, 1e-7) of the block
+// form, with unsigned indices, and now (with solve_pair's squares and up64):
+//   512 x 256 2.25 2.25 1.95, 512 x 1024 2.28 2.47 2.09, 1024 x 512 2.16 2.41
+//   1.80, 2048 x 1024 2.29 2.59 1.91, 2048 x 2048 2.04 2.30 1.84.
 template <int N, int kSign>
 __device__ __forceinline__ void group_fft(float2* buf, const float2* tws) {
   using F = GroupFft<N>;
@@ -674,10 +698,12 @@ __device__ __forceinline__ void group_fft(float2* buf, const float2* tws) {
   constexpr int kBits = E == 32 ? 5 : E == 16 ? 4 : 3;
   const int l = threadIdx.x & (G - 1);
   float re[E], im[E];
-  // stage 1: lane n1 = l holds x[n1 + G n2], n2 < E; DFT along n2
+  // stage 1: lane l holds x[n1 + G n2], n2 < E, with n1 = l in the lower half
+  // and l - G in the upper; DFT along n2
+  const int n1 = l < G / 2 ? l : l - G;
 #pragma unroll
   for (int j = 0; j < E; j++) {
-    const float2 v = buf[l + G * j];
+    const float2 v = buf[j ? n1 + G * j : n1 & (N - 1)];
     re[j] = v.x; im[j] = v.y;
   }
   dft_reg<E, kSign>(re, im);
@@ -700,44 +726,48 @@ __device__ __forceinline__ void group_fft(float2* buf, const float2* tws) {
   }
   group_sync<G>();
   if constexpr (G == E) {
-    // stage 2: lane k2 = l takes n1 = 0..G-1, a G-point DFT, X[k2 + E k1]
+    // stage 2: lane l takes the column of k2 = l or l - E, a G-point DFT,
+    // X[k2 + E k1]
 #pragma unroll
-    for (int n1 = 0; n1 < G; n1++) {
-      re[n1] = tr[n1 * S + l];
-      im[n1] = ti[n1 * S + l];
+    for (int i = 0; i < G; i++) {
+      re[i] = tr[i * S + l];
+      im[i] = ti[i * S + l];
     }
     group_sync<G>();
     dft_reg<E, kSign>(re, im);
 #pragma unroll
-    for (int r = 0; r < E; r++) buf[l + E * brev<kBits>(r)] = make_float2(re[r], im[r]);
+    for (int r = 0; r < E; r++) buf[r ? n1 + E * brev<kBits>(r) : n1 & (N - 1)] = make_float2(re[r], im[r]);
   } else if constexpr (E == 2 * G) {
-    // stage 2: lane l takes columns k2 = l and l + G, a G-point DFT each
+    // stage 2: lane l takes the columns of k2 = l and l - G, a G-point DFT each
     constexpr int kBitsG = kBits - 1;
     float r2[2][G], i2[2][G];
 #pragma unroll
     for (int h = 0; h < 2; h++)
 #pragma unroll
-      for (int n1 = 0; n1 < G; n1++) {
-        r2[h][n1] = tr[n1 * S + l + G * h];
-        i2[h][n1] = ti[n1 * S + l + G * h];
+      for (int i = 0; i < G; i++) {
+        r2[h][i] = tr[i * S + l + G * h];
+        i2[h][i] = ti[i * S + l + G * h];
       }
     group_sync<G>();
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       dft_reg<G, kSign>(r2[h], i2[h]);
 #pragma unroll
-      for (int r = 0; r < G; r++) buf[l + G * h + E * brev<kBitsG>(r)] = make_float2(r2[h][r], i2[h][r]);
+      for (int r = 0; r < G; r++) {
+        const int k = l - G * h;
+        buf[r ? k + E * brev<kBitsG>(r) : k & (N - 1)] = make_float2(r2[h][r], i2[h][r]);
+      }
     }
   } else {
-    // stage 2 for G = 2 E: lane pair (2 k2, 2 k2 + 1) takes the even and odd
-    // n1 of column k2, one E-point DFT each, then X[k] = E[k] + W^k O[k]
+    // stage 2 for G = 2 E: lane pair (2 c, 2 c + 1) takes the even and odd
+    // lanes' elements of column c (k2 = c or c - E), one E-point DFT each, then X[k] = E[k] + W^k O[k]
     // (even lane) and X[k + E] = E[k] - W^k O[k] (odd lane), W = W_G
     static_assert(G == 2 * E, "one or two lanes or columns");
-    const int k2 = l >> 1, odd = l & 1;
+    const int c = l >> 1, odd = l & 1, k2 = c < E / 2 ? c : c - E;
 #pragma unroll
     for (int i = 0; i < E; i++) {
-      re[i] = tr[(2 * i + odd) * S + k2];
-      im[i] = ti[(2 * i + odd) * S + k2];
+      re[i] = tr[(2 * i + odd) * S + c];
+      im[i] = ti[(2 * i + odd) * S + c];
     }
     group_sync<G>();
     dft_reg<E, kSign>(re, im);
@@ -751,7 +781,8 @@ __device__ __forceinline__ void group_fft(float2* buf, const float2* tws) {
       rot64<kSign>(orr, oi, k * (64 / G));
       const float er = odd ? pr : re[r], ei = odd ? pi : im[r];
       const float xr = odd ? er - orr : er + orr, xi = odd ? ei - oi : ei + oi;
-      buf[k2 + E * (k + E * odd)] = make_float2(xr, xi);
+      const int at = k2 + E * (k + E * odd);
+      buf[k ? at : at & (N - 1)] = make_float2(xr, xi);
     }
   }
   group_sync<G>();
@@ -854,19 +885,21 @@ template <int N, int kP>
 constexpr size_t cols_bytes() { return (size_t)2 * kP * GroupFft<N>::kBuf * 4 + N * 8; }
 
 // phi^ of a packed column pair (u, u + 1) at row v from Z at v and n - v
-// (src/fft.cpp:117-166)
-__device__ __forceinline__ float2 solve_pair(const PassBArgs& B, float2 z, float2 zn, float2 w4, float2 wx, float wyv,
-                                             int u, int v) {
+// (src/fft.cpp:117-166): 4 / (nx ny) rho^ / (wx^2 + wy^2) with pi / nx taken
+// out of the frequencies, so that the low modes, which carry the field, divide
+// by u^2 + (wy[1] / wx[1])^2 v^2 of exact squares instead of squares of rounded
+// multiples of pi.
+__device__ __forceinline__ float2 solve_pair(const PassBArgs& B, float2 z, float2 zn, float2 w4, int u, int v) {
   const float2 a = dct2_post(z, zn, w4);
+  const float vv = (float)(v * v);
   float out[2];
 #pragma unroll
   for (int h = 0; h < 2; h++) {
     float d = h ? a.y : a.x;
     if (u + h == 0) d *= 0.5f;
     if (v == 0) d *= 0.5f;
-    d *= B.scale;
-    const float wxu = h ? wx.y : wx.x;
-    const float den = __fadd_rn(__fmul_rn(wxu, wxu), __fmul_rn(wyv, wyv));
+    d = __fmaf_rn(d, B.num[0], __fmul_rn(d, B.num[1]));
+    const float den = __fmaf_rn(vv, B.aspect[0], __fmaf_rn(vv, B.aspect[1], (float)((u + h) * (u + h))));
     out[h] = (u + h != 0 || v != 0) ? __fdiv_rn(d, den) : 0.0f;
   }
   return make_float2(out[0], out[1]);
@@ -893,7 +926,6 @@ __global__ void __launch_bounds__(2 * kP * GroupFft<N>::kG) k_poisson_cols_g(Pas
     cp_async8(smem + (size_t)c * kBufF2 + makhoul_pos(v, N), B.spec + (size_t)v * nx + u_base + 2 * c);
   }
   block_copy_async(reinterpret_cast<float*>(tws), reinterpret_cast<const float*>(tw_table<N>()), 2 * N);
-  const float2 wx = make_float2(__ldg(&B.wx[u]), __ldg(&B.wx[u + 1]));
   cp_async_wait_all();
   __syncthreads();
   if (role == 0) group_fft<N, -1>(buf0, tws);
@@ -906,8 +938,8 @@ __global__ void __launch_bounds__(2 * kP * GroupFft<N>::kG) k_poisson_cols_g(Pas
     const float2 zk = buf0[k], zm = buf0[m];
     const float2 w4k = __ldg(&B.w4[k]), w4m = __ldg(&B.w4[m]);
     const float wk = __ldg(&B.wy[k]), wm = __ldg(&B.wy[m]);
-    const float2 pk = solve_pair(B, zk, k ? zm : zk, w4k, wx, wk, u, k);
-    const float2 pm = solve_pair(B, zm, k ? zk : zm, w4m, wx, wm, u, m);
+    const float2 pk = solve_pair(B, zk, k ? zm : zk, w4k, u, k);
+    const float2 pm = solve_pair(B, zm, k ? zk : zm, w4m, u, m);
     const float2 sk = make_float2(__fmul_rn(pk.x, wk), __fmul_rn(pk.y, wk));
     const float2 sm = make_float2(__fmul_rn(pm.x, wm), __fmul_rn(pm.y, wm));
     buf0[k] = pre_pair(pk, pm, w4k, k);
@@ -1096,11 +1128,10 @@ __global__ void __cluster_dims__(kClCtas, 1, 1) __launch_bounds__(ClusterShape<N
     float2* buf0 = col0 + q * kBufF2;
     float2* buf1 = col1 + q * kBufF2;
     const float2 zk = buf0[k], zm = buf0[m];
-    const float2 wx = make_float2(__ldg(&B.wx[u]), __ldg(&B.wx[u + 1]));
     const float2 w4k = __ldg(&B.w4[k]), w4m = __ldg(&B.w4[m]);
     const float wk = __ldg(&B.wy[k]), wm = __ldg(&B.wy[m]);
-    const float2 pk = solve_pair(B, zk, k ? zm : zk, w4k, wx, wk, u, k);
-    const float2 pm = solve_pair(B, zm, k ? zk : zm, w4m, wx, wm, u, m);
+    const float2 pk = solve_pair(B, zk, k ? zm : zk, w4k, u, k);
+    const float2 pm = solve_pair(B, zm, k ? zk : zm, w4m, u, m);
     const float2 sk = make_float2(__fmul_rn(pk.x, wk), __fmul_rn(pk.y, wk));
     const float2 sm = make_float2(__fmul_rn(pm.x, wm), __fmul_rn(pm.y, wm));
     buf0[k] = pre_pair(pk, pm, w4k, k);
@@ -1270,13 +1301,15 @@ int poisson_context(PoissonContext* out) {
     GPL_CUDA(group_prepare<2048>());
     pc.cluster = cluster_prepare<64>() && cluster_prepare<128>() && cluster_prepare<256>();
     for (int n : {64, 128, 256, 512, 1024, 2048}) {
-      // the group form's twiddles, [k2 * G + n1] = exp(-2 pi i n1 k2 / n)
+      // the group form's twiddles (indices of either sign, see group_fft)
       const int g = n <= 128 ? GroupFft<64>::kG : n == 256 ? GroupFft<256>::kG : n == 2048 ? GroupFft<2048>::kG : GroupFft<512>::kG;
       static_assert(GroupFft<512>::kG == GroupFft<1024>::kG && GroupFft<64>::kG == GroupFft<128>::kG, "one width");
       std::vector<float2> t(n);
-      for (int k2 = 0; k2 < n / g; k2++)
+      const int e = n / g;
+      for (int k2 = 0; k2 < e; k2++)
         for (int n1 = 0; n1 < g; n1++) {
-          const double a = -2.0 * M_PI * (double)(n1 * k2) / (double)n;
+          const int m = (n1 < g / 2 ? n1 : n1 - g) * (k2 < e / 2 ? k2 : k2 - e);
+          const double a = -2.0 * M_PI * (double)m / (double)n;
           t[k2 * g + n1] = make_float2((float)cos(a), (float)sin(a));
         }
       const size_t bytes = n * sizeof(float2);
@@ -1318,6 +1351,17 @@ void block_form_bc(const PoissonGrid& g, float* spec, float* p1, float* p2, floa
   smem[0] = smem_a(nx, ny);
   smem[1] = smem_b(nx, ny);
   smem[2] = smem_c(nx, ny);
+}
+
+// solve_pair's constants.
+void solve_constants(const PoissonGrid& g, PassBArgs& B) {
+  const double r = (double)g.nx / g.ny * ((double)g.size_y / g.size_x);
+  const double num = 4.0 * g.nx / (g.ny * M_PI * M_PI), aspect = r * r;
+  B.scale = 0.0f;
+  B.num[0] = (float)num;
+  B.num[1] = (float)(num - B.num[0]);
+  B.aspect[0] = (float)aspect;
+  B.aspect[1] = (float)(aspect - B.aspect[0]);
 }
 
 PassAArgs pass_a_args(const PoissonGrid& g, unsigned long long* const* area_pair, const EvalCtl* ctl,
@@ -1434,7 +1478,7 @@ int poisson_passes(const PoissonGrid& g, unsigned long long* const* area_pair,
     PassBArgs B;
     B.nx = nx; B.ny = ny; B.logn = ilog2(ny); B.col_pairs = 0;
     B.spec = spec; B.p1 = p1; B.p2 = p2; B.wx = g.wx; B.wy = g.wy; B.tw = g.tw; B.w4 = g.w4y;
-    B.scale = 4.0f / (float)nx / (float)ny;
+    solve_constants(g, B);
     PassCArgs C;
     C.nx = nx; C.ny = ny; C.logn = ilog2(nx); C.pairs_per_block = 0;
     C.p1 = p1; C.p2 = p2; C.field = field; C.fx = fx; C.fy = fy; C.phi = phi;
@@ -1468,6 +1512,7 @@ int poisson_passes(const PoissonGrid& g, unsigned long long* const* area_pair,
     int grid[3];
     size_t smem[3];
     block_form_bc(g, spec, p1, p2, field, fx, fy, phi, B, C, grid, smem);
+    solve_constants(g, B);
     if (t) t->begin(kKPoissonB);
     if (nx == 64) k_poisson_cluster<64><<<kClCtas, ClusterShape<64>::kT, ClusterShape<64>::kBytes, s>>>(A, B, C);
     else if (nx == 128) k_poisson_cluster<128><<<kClCtas, ClusterShape<128>::kT, ClusterShape<128>::kBytes, s>>>(A, B, C);
