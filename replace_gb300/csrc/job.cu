@@ -1098,9 +1098,15 @@ namespace gpl {
 
 enum BatchTable { kTScatter = 0, kTWa, kTPa, kTPb, kTPc, kTCell, kTables };
 
+// Streams for the Poisson passes of members on grids that the batched passes
+// do not cover.
+constexpr int kBatchSides = 8;
+
 struct BatchRun {
   int cap = 0, device = 0, sms = 1;
   cudaStream_t s = nullptr;
+  cudaStream_t side[kBatchSides] = {nullptr};   // (made when a member needs them)
+  cudaEvent_t fork = nullptr, join[kBatchSides] = {nullptr};
   char* dev = nullptr;                 // argument tables, control and result records, counts
   char* host = nullptr;                // pinned: control and result records, counts
   char* args[kTables] = {nullptr};
@@ -1125,6 +1131,12 @@ struct BatchRun {
   ~BatchRun() {
     if (exec) cudaGraphExecDestroy(exec);
     if (s) cudaStreamSynchronize(s);
+    for (int k = 0; k < kBatchSides; k++) {
+      if (side[k]) cudaStreamSynchronize(side[k]);
+      if (join[k]) cudaEventDestroy(join[k]);
+      if (side[k]) cudaStreamDestroy(side[k]);
+    }
+    if (fork) cudaEventDestroy(fork);
     if (dev) cudaFree(dev);
     if (items_d) cudaFree(items_d);
     if (host) cudaFreeHost(host);
@@ -1233,6 +1245,13 @@ int batch_join(BatchRun* B, int slot, gpl_job* j, int max_iters, gpl_iter_log* l
   if (!ok) {                       // the job's own Poisson launches (group form)
     g3[0] = g3[1] = g3[2] = 0;
     sm3[0] = sm3[1] = sm3[2] = 0;
+    if (!B->fork) {
+      for (int k = 0; k < kBatchSides; k++) {
+        if (!B->side[k]) GPL_CUDA(cudaStreamCreateWithFlags(&B->side[k], cudaStreamNonBlocking));
+        if (!B->join[k]) GPL_CUDA(cudaEventCreateWithFlags(&B->join[k], cudaEventDisableTiming));
+      }
+      GPL_CUDA(cudaEventCreateWithFlags(&B->fork, cudaEventDisableTiming));
+    }
   }
   // the job's own stream may still hold work (initialisation)
   GPL_CUDA(cudaStreamSynchronize(j->stream));
@@ -1338,6 +1357,29 @@ int batch_launch_round(BatchRun& B) {
                               grid(kBScatterBig), 0, B.s);
     nl++;
   }
+  // Members on grids the batched passes do not cover: the launches of the job
+  // alone, on the batch's control record, spread over side streams beside the
+  // WA and Poisson phases of the rest.  One after another on the round's stream
+  // they were most of it: 16 jobs of 10k cells on 512 x 256 bins 528 us a round,
+  // 256 so (384 with the batched block passes, which these grids took before the
+  // register FFTs).
+  int sides = 0;
+  for (int k = 0; k < B.cap && !rc; k++) {
+    BatchMember& m = B.members[k];
+    if (!m.job || !m.running || !m.own_poisson) continue;
+    const int q = sides % kBatchSides;
+    if (sides == 0) GPL_CUDA(cudaEventRecord(B.fork, B.s));
+    if (sides < kBatchSides) GPL_CUDA(cudaStreamWaitEvent(B.side[q], B.fork));
+    sides++;
+    DeviceModel& d = m.job->d;
+    EvalCtl* own = d.ctl;
+    Timer quiet;
+    d.ctl = B.ctl_d + k;
+    rc = launch_poisson_job(d, false, B.side[q], quiet);
+    d.ctl = own;
+    nl += quiet.kernels;
+  }
+  for (int q = 0; q < std::min(sides, kBatchSides); q++) GPL_CUDA(cudaEventRecord(B.join[q], B.side[q]));
   const int wa_phase[4] = {kBWaSmall, kBWaLarge, kBWaSmallW, kBWaLargeW};
   for (int q = 0; q < 4 && !rc; q++) {
     const int p = wa_phase[q];
@@ -1351,19 +1393,7 @@ int batch_launch_round(BatchRun& B) {
     rc = launch_poisson_batch(q, B.args[kTPa + q], items(p), count(p), grid(p), B.smem_p[q], B.s);
     nl++;
   }
-  // members on grids the batched passes do not cover: the launches of the
-  // job alone, on the batch's control record
-  for (int k = 0; k < B.cap && !rc; k++) {
-    BatchMember& m = B.members[k];
-    if (!m.job || !m.running || !m.own_poisson) continue;
-    DeviceModel& d = m.job->d;
-    EvalCtl* own = d.ctl;
-    Timer quiet;
-    d.ctl = B.ctl_d + k;
-    rc = launch_poisson_job(d, false, B.s, quiet);
-    d.ctl = own;
-    nl += quiet.kernels;
-  }
+  for (int q = 0; q < std::min(sides, kBatchSides); q++) GPL_CUDA(cudaStreamWaitEvent(B.s, B.join[q]));
   if (!rc && B.phase_used[kBDgradBig]) {
     rc = launch_density_batch(kBDgradBig, B.args[kTCell], items(kBDgradBig), count(kBDgradBig), grid(kBDgradBig),
                               0, B.s);

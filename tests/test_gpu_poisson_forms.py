@@ -197,3 +197,30 @@ def test_register_ffts_as_exact_as_shared_memory_ones(gpu_lib, nx, ny):
     got = 1e7 * solve_errors(nx, ny)
     # (a rounding here or there shifts a mean over eight densities by 2 %)
     assert (got <= 1.02 * np.array(BLOCK_FORM[nx, ny])).all(), got
+
+
+def test_batch_members_on_group_form_grids_leave_one_by_one(gpu_lib):
+    """More such members than side streams, which end at different iterations:
+    each one's whole loop equals the job alone."""
+    from replace_gb300 import Placer, batch_nesterov_run
+    grids = [(512, 256), (256, 512), (64, 64), (256, 512), (512, 256), (512, 256), (256, 512), (512, 256),
+             (256, 512), (512, 256), (64, 128)]
+
+    def job(k):
+        n = 6_000 + 500 * k
+        p = Placer(N.generate(n, n + n // 20, n_io=60, seed=k), target_density=0.70 + 0.01 * k, poisson_path=1,
+                   bin_grid_cnt_x=grids[k][0], bin_grid_cnt_y=grids[k][1], initial_place_max_iter=2,
+                   nesterov_place_max_iter=20 + 6 * (k * 7 % 11))
+        p.initial_place()
+        p.nesterov_init()
+        return p
+    ps = [job(k) for k in range(len(grids))]
+    stats, status, _ = batch_nesterov_run(ps)
+    assert len({st.iterations for st in stats}) == len(ps)
+    for k, p in enumerate(ps):
+        q = job(k)
+        rc, st, _ = q.nesterov_run(0, allow_divergence=True)
+        assert status[k] == rc and stats[k].iterations == st.iterations and stats[k].hpwl == st.hpwl
+        assert np.array_equal(p.gcell_coords(), q.gcell_coords()), grids[k]
+        p.close()
+        q.close()
