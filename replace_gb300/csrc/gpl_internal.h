@@ -393,8 +393,11 @@ int wa_nets_per_block(int bucket);
 // `pinned` is the job's ip_state block; `pool` as for dev_alloc.
 int run_initial_place(HostModel& m, cudaStream_t s, int sm_count, gpl_ip_stats* stats, Timer& t,
                       void* pinned, cudaMemPool_t pool, cudaEvent_t sync_ev);
-// device bytes run_initial_place allocates for this model
+// device bytes run_initial_place allocates for this model on the current
+// device: those at the block cap it takes there
 size_t initial_place_bytes(const HostModel& m, int sm_count);
+int initial_place_grid_cap(int sm_count);
+size_t initial_place_bytes_at(const HostModel& m, int grid_cap);
 // One job of the batched initial place: its host model, and the stream,
 // pinned block, pool and event its setup and read-back use (as
 // run_initial_place's); stats may be null; status is the job's result.

@@ -1988,23 +1988,30 @@ struct IpSizes {
   int rows_blk = 32;
 };
 
-// Scratch layout of run_initial_place (the sizes its carving below takes).
-IpSizes ip_sizes(const HostModel& m, int grid_cap) {
-  IpSizes z;
-  const size_t nP = m.place_insts.size();
-  size_t n_mp = 0;
-  for (int i : m.place_insts) n_mp += m.inst_pin_start[i + 1] - m.inst_pin_start[i];
+// The movable instances' pins and a bound of the matrix entries per axis.
+struct IpCounts {
+  size_t n_mp = 0, nnz = 0;
+};
+IpCounts ip_counts(const HostModel& m) {
+  IpCounts c;
+  for (int i : m.place_insts) c.n_mp += m.inst_pin_start[i + 1] - m.inst_pin_start[i];
   // An upper bound of the off-diagonal entries per axis (see for_partners):
   // a net of degree d has at most two bound pins, each partnering at most
   // d - 1 pins, and every other pin partners at most the two bound pins, so
   // the net contributes at most 2 (d - 1) + 2 (d - 2) = 4 d - 6 entries (one
   // bound pin for both ends: (d - 1) + (d - 1) <= 4 d - 6 for d >= 2).
-  size_t nnz = 0;
   for (int n = 0; n < m.n_nets; n++) {
     const size_t deg = m.net_start[n + 1] - m.net_start[n];
-    if (deg > 1 && (int)deg < m.p.initial_place_max_fanout) nnz += 4 * deg - 6;
+    if (deg > 1 && (int)deg < m.p.initial_place_max_fanout) c.nnz += 4 * deg - 6;
   }
-  z.nnz_cap = std::max<size_t>(nnz, 1);
+  return c;
+}
+
+// Scratch layout of run_initial_place (the sizes its carving below takes).
+IpSizes ip_sizes(const HostModel& m, const IpCounts& c, int grid_cap) {
+  IpSizes z;
+  const size_t nP = m.place_insts.size(), n_mp = c.n_mp;
+  z.nnz_cap = std::max<size_t>(c.nnz, 1);
   // solve_rows rows per thread, at most grid_cap blocks per axis
   const size_t rows_per_block = (size_t)kB * solve_rows(nP);
   const int g0 = std::max(1, std::min((int)((nP + rows_per_block - 1) / rows_per_block), grid_cap));
@@ -2040,8 +2047,30 @@ IpSizes ip_sizes(const HostModel& m, int grid_cap) {
   return z;
 }
 
-// (a cooperative grid has at most 8 blocks of kB threads per SM, 2 axes)
-size_t initial_place_bytes(const HostModel& m, int sm_count) { return ip_sizes(m, sm_count * 8).bytes; }
+// Resident blocks per SM of the cooperative solve on the current device; 0
+// where it cannot run.
+int coop_blocks_per_sm() {
+  int dev = 0, coop = 0, per_sm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bi_coop, kB, stage_bytes(kB));
+  cudaGetLastError();
+  return coop ? per_sm : 0;
+}
+
+// SpMV blocks per axis at most: every form takes the grid of the cooperative
+// one (both axes resident), so that all give the same iterates.  The scratch
+// is not monotone in it (slices come eight to a block), so a bound has to be
+// asked at this cap: the cap of eight blocks an SM needs 1.8 MB less at 1.17M
+// instances.
+int initial_place_grid_cap(int sm_count) {
+  const int per_sm = coop_blocks_per_sm();
+  return per_sm > 0 ? std::max(1, per_sm * sm_count / 2) : sm_count * 8;
+}
+size_t initial_place_bytes(const HostModel& m, int sm_count) {
+  return initial_place_bytes_at(m, initial_place_grid_cap(sm_count));
+}
+size_t initial_place_bytes_at(const HostModel& m, int grid_cap) { return ip_sizes(m, ip_counts(m), grid_cap).bytes; }
 
 // One job's initial place on the device: its scratch, tables and solver
 // state (ip_setup), the rounds (run_initial_place's loop, or the batched
@@ -2058,7 +2087,7 @@ struct IpRun {
   IpParams P;
   int nP = 0, nb_mov = 0, grid = 1, xr_grid = 1, scan_blocks = 1;
   bool cluster = false, coop = false;
-  int coop_attr = 0, per_sm = 0;
+  int per_sm = 0;
   std::vector<int2> ctr;         // host centres (read back at the end)
   BiState* st_h = nullptr;       // pinned solver states [2] (+ GridBar)
   int rounds = 0, iters[2] = {0, 0}, coop_rounds = 0;
@@ -2125,10 +2154,7 @@ int ip_setup(HostModel& m, cudaStream_t s, int sm_count, void* pinned, cudaMemPo
     }
   });
   // The cooperative solve needs its whole grid (both axes) resident at once.
-  int dev = 0, coop_attr = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&coop_attr, cudaDevAttrCooperativeLaunch, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bi_coop, kB, stage_bytes(kB));
+  const int per_sm = coop_blocks_per_sm();
   // the cluster solve's stages exceed the default dynamic shared-memory cap
   cudaFuncSetAttribute(k_bi_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_bytes(kClThreads));
   // the SpMV phases' product stages and x window exceed the default cap too
@@ -2145,10 +2171,9 @@ int ip_setup(HostModel& m, cudaStream_t s, int sm_count, void* pinned, cudaMemPo
   // instances up and, because its short kernels interleave with other jobs'
   // kernels, the best one under the placement server at every size.
   bool cluster = mode == 3 && nP <= kClMaxRows;
-  bool coop = !cluster && coop_attr != 0 && per_sm > 0 && mode == 2;
-  // the same grid either way, so both solvers give the same iterates
-  const int grid_cap = (coop_attr != 0 && per_sm > 0) ? std::max(1, per_sm * sm_count / 2) : sm_count * 8;
-  const IpSizes z = ip_sizes(m, grid_cap);
+  bool coop = !cluster && per_sm > 0 && mode == 2;
+  const int grid_cap = initial_place_grid_cap(sm_count);
+  const IpSizes z = ip_sizes(m, ip_counts(m), grid_cap);
   D.nnz_cap = z.nnz_cap;
   D.sell_cap = z.sell_cap;
   D.slot_cap = z.slot_cap;
@@ -2249,7 +2274,6 @@ int ip_setup(HostModel& m, cudaStream_t s, int sm_count, void* pinned, cudaMemPo
   R.scan_blocks = scan_blocks;
   R.cluster = cluster;
   R.coop = coop;
-  R.coop_attr = coop_attr;
   R.per_sm = per_sm;
   R.ctr.assign(ctr.data(), ctr.data() + nP);
   if (prm.verbose_level >= 2)
@@ -2323,7 +2347,7 @@ int run_initial_place(HostModel& m, cudaStream_t s, int sm_count, gpl_ip_stats* 
   const IpParams& P = R.P;
   const int nP = R.nP, nb_mov = R.nb_mov, grid = R.grid, scan_blocks = R.scan_blocks;
   bool cluster = R.cluster, coop = R.coop;
-  const int coop_attr = R.coop_attr, per_sm = R.per_sm, mode = prm.ip_solver;
+  const int per_sm = R.per_sm, mode = prm.ip_solver;
   BiState* st_h = R.st_h;
   const dim3 g2(nb_mov, 2), gs(grid, 2), gx(R.xr_grid, 2);
   const auto wall = wall_now;
@@ -2488,7 +2512,7 @@ int run_initial_place(HostModel& m, cudaStream_t s, int sm_count, gpl_ip_stats* 
         if (prm.verbose_level > 0)
           printf("[InitialPlace] cluster solve not launched (%s)\n", cudaGetErrorString(ce));
         cluster = false;
-        coop = coop_attr != 0 && per_sm > 0 && mode != 1;
+        coop = per_sm > 0 && mode != 1;
       }
     }
     if (!solved && coop) {
