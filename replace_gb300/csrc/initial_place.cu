@@ -52,9 +52,10 @@ struct BiState {
 
 // An SpMV block's x window (first index and length, 0: none) and sliced form
 // (ip_sell_body): its sliced, staged and special rows, the staged entries'
-// first place in sval / scol and their number, and each warp's first entry.
+// first place in sval / scol and their number, how many of the special rows no
+// stage takes, and each warp's first entry.
 struct __align__(64) SellBlock {
-  int lo, span, sliced, staged, special, stage_at, stage_n, pad;
+  int lo, span, sliced, staged, special, stage_at, stage_n, tall;
   int warp_at[8];
 };
 
@@ -488,7 +489,7 @@ __device__ __forceinline__ void ip_sell_body(const IpDev& D, int vb, int axis) {
   __shared__ uint32_t slot_s[kXWinMax];
   __shared__ int hist[160];
   __shared__ int scan[kB];
-  __shared__ int s_lo, s_span, s_base, s_T, s_over, s_cursor, s_staged, s_special, s_stage_at;
+  __shared__ int s_lo, s_span, s_base, s_T, s_over, s_cursor, s_staged, s_special, s_tall, s_stage_at;
   const int n = D.n_mov;
   const int r0 = vb * D.rows_blk, r1 = min(r0 + D.rows_blk, n), R = r1 - r0;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -545,6 +546,7 @@ __device__ __forceinline__ void ip_sell_body(const IpDev& D, int vb, int axis) {
     const int cap = stage_cap(D.rows_blk), t_min = sell_min(D.rows_blk);
     int T = kSellMax, sum = s_over, rows = hist[kSellMax + 1];
     const bool tall = sum > cap;                   // not even the longest rows fit: a warp each
+    s_tall = tall ? rows : 0;
     if (tall) {
       hist[kSellMax + 2] += rows;
       hist[kSellMax + 1] = rows = 0;
@@ -626,6 +628,7 @@ __device__ __forceinline__ void ip_sell_body(const IpDev& D, int vb, int axis) {
       q.sliced = n_sell;
       q.staged = s_staged;
       q.special = s_special;
+      q.tall = s_tall;
       q.stage_at = (int)at + scan[kB - 1];
       q.stage_n = s_cursor;
       for (int w = 0; w < 8; w++) q.warp_at[w] = (int)at + (w && np ? scan[w * np - 1] : 0);
@@ -2312,6 +2315,29 @@ int ip_finish(IpRun& R, gpl_ip_stats* stats, int rc) {
   return GPL_OK;
 }
 
+// How the last round's matrix rows were summed (block_product's forms).
+void print_sell_rows(const IpRun& R, cudaStream_t s) {
+  const IpDev& D = R.D;
+  std::vector<SellBlock> q(2 * (size_t)D.parts);
+  if (cudaMemcpyAsync(q.data(), D.sblk, q.size() * sizeof(SellBlock), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+      cudaStreamSynchronize(s) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  for (int axis = 0; axis < 2; axis++) {
+    int sliced = 0, staged = 0, special = 0, tall = 0, csr = 0;
+    for (int b = 0; b < R.grid; b++) {
+      const SellBlock& k = q[(size_t)axis * D.parts + b];
+      if (k.span) { sliced += k.sliced; staged += k.staged; special += k.special; tall += k.tall; }
+      else csr++;
+    }
+    printf("[InitialPlace] rows of %c: %d sliced, %d staged, %d long ones among many, %d longer than the stage, "
+           "%d in CSR form (%d of %d blocks)\n", axis ? 'y' : 'x', sliced, staged, special - tall, tall,
+           R.nP - sliced - staged - special, csr, R.grid);
+  }
+  fflush(stdout);
+}
+
 // The round's end for one job: its solver states give the error
 // (solver.error() = sqrt(|r|^2 / |b|^2)) and the stop test
 // (src/initialPlace.cpp:93-99).
@@ -2331,7 +2357,10 @@ void ip_round_done(IpRun& R, int round, const BiState* st) {
 // a chunk after the solve is done cost their empty launches.  Against chunks of
 // 8 (13 looks for 100 iterations): 300 cells 8.8 -> 8.6 ms, 3k 14.1 -> 13.5,
 // 10k 58.3 -> 54.1, 150k 80.7 -> 78.0, 400k 145.9 -> 140.5.
-// Solves that end early (the two smallest) gain as well.
+// Solves that end early (the two smallest) gain as well.  A solve that restarts
+// waits for the next chunk, up to 24 iterations of empty launches (0.15 ms);
+// one of 4800 solves of generated designs of 1 to 30k cells restarts, so
+// testing for it in every iteration, a launch each, costs more.
 int chunk_iterations(int max_iter) {
   const int chunks = std::max(1, (max_iter + 24) / 25);
   return std::max(1, (max_iter + chunks - 1) / chunks);
@@ -2580,6 +2609,7 @@ int run_initial_place(HostModel& m, cudaStream_t s, int sm_count, gpl_ip_stats* 
   if (assembly_exec) cudaGraphExecDestroy(assembly_exec);
   if (chunk_exec) cudaGraphExecDestroy(chunk_exec);
   (void)nP;
+  if (prm.verbose_level >= 2 && !rc && !cluster && !coop) print_sell_rows(R, s);
   return ip_finish(R, stats, rc);
 }
 
