@@ -224,3 +224,19 @@ def test_batch_members_on_group_form_grids_leave_one_by_one(gpu_lib):
         assert np.array_equal(p.gcell_coords(), q.gcell_coords()), grids[k]
         p.close()
         q.close()
+
+
+@pytest.mark.parametrize("phi", [True, False])
+@pytest.mark.parametrize("n", [64, 128, 256])
+def test_cluster_solve_matches_fp64(gpu_lib, n, phi):
+    import torch
+    from replace_gb300.placer import poisson_solve
+    d = placed_density(n, n, n)
+    dd = torch.from_numpy(d).cuda()
+    out = [torch.full_like(dd, 7.0) for _ in range(3)]
+    poisson_solve(dd.data_ptr(), out[0].data_ptr() if phi else 0, out[1].data_ptr(), out[2].data_ptr(), n, n, 380, 1400)
+    torch.cuda.synchronize()
+    for got, want in list(zip(out, fp64_solve(d, 380, 1400)))[0 if phi else 1:]:
+        assert rel_l2(got.cpu().numpy(), want) < 2e-6
+    if not phi:
+        assert (out[0] == 7.0).all()
