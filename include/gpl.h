@@ -138,8 +138,9 @@ typedef struct gpl_params {
                                               grids with both counts multiples of 128) */
   int32_t scatter_tile;                    /* scatter tile side in bins (16, 32 or 64); 0 = chosen
                                               by timing at gpl_nesterov_init */
-  int32_t scatter_chunk;                   /* gcells per scatter block (1024 or 2048); 0 = chosen
-                                              by timing (with the tile) */
+  int32_t scatter_chunk;                   /* gcells per scatter block at most (1024 or 2048; small
+                                              designs take smaller blocks); 0 = chosen by timing
+                                              (with the tile) */
   int32_t device_loop;                     /* 0 = the host drives the Nesterov loop, one
                                               evaluation graph at a time, and the initial
                                               place's rounds, one chunk of solver iterations
@@ -164,7 +165,7 @@ typedef struct gpl_job_info {
   float poisson_fft_us;      /* the timings auto mode compared (0 if not timed) */
   float poisson_gemm_us;
   int32_t scatter_tile;      /* the scatter's tile side in bins, chosen by timing (16, 32 or 64) */
-  int32_t scatter_chunk;     /* gcells per scatter block, chosen with the tile */
+  int32_t scatter_chunk;     /* gcells per scatter block at most, chosen with the tile */
   float scatter_us;          /* the chosen shape's scatter time */
 } gpl_job_info;
 

@@ -179,14 +179,14 @@ struct TileArgs {
 // The body of one block (chunk vb); `win` is the block's dynamic shared
 // window.  Shared by the per-job launch and the batched one.
 //
-// What bounds it is instruction issue (60 % of the slots at a million cells),
+// What bounds it is instruction issue and the barriers around the window (600
+// warp instructions for 32 gcells at a million cells, 40 % of the issue slots),
 // so: bin ranges by multiplication (FastDiv), a gcell's overlap widths once
 // per column and row, its up to 3 x 3 bins without loops or range tests when
 // they lie inside the window, and one 32-bit window word per bin where the
 // chunk's sums cannot pass 2^32 (two 16-bit halves in two words otherwise).
 // 12.5k gcells 17.5 -> 9.8 us, 250k with 40 macros 28.9 -> 24, 1.25M 64.0 ->
-// 42.8 (in the loop, events around the launch); a 1024-gcell block used to
-// run 1800 instructions a warp of gcells.
+// 42.8 (in the loop, events around the launch).
 template <bool kOneWord>
 __device__ __forceinline__ void scatter_body(const ScatterArgs& A, const TileArgs& T, int vb, unsigned* win) {
   if (vb >= *T.n_chunks) return;                   // block-uniform
@@ -279,8 +279,8 @@ __device__ __forceinline__ void scatter_big_body(const ScatterArgs& A, const int
   const int nb = G.cnt_x * G.cnt_y;
   const GCellGeo geo = gcell_geo(A.geo_g[g]);
   const int2 h = geo.half;
-  // k_scatter has already written this cell's predicted coordinates; the
-  // block recomputes them with the same arithmetic instead of reading them
+  // the chunk that holds this cell writes its predicted coordinates, maybe
+  // later than this block runs; recomputed here with the same arithmetic
   float2 c;
   if (C.predict) {
     __shared__ float2 cs;
@@ -554,9 +554,10 @@ __device__ __forceinline__ void cell_body(const CellArgs& A, int vb, int vgrid) 
     }
     if (!isfinite(aw) || !isfinite(ad)) bad = 1;
   }
-  // The FP64 pipe takes 15 cycles a warp instruction here, so the sums across
-  // warps and blocks are laid out to need few: each instruction serves all
-  // slots at once (block), or one slot a warp (final).
+  // The FP64 pipe takes 64 cycles a warp instruction on each of an SM's four
+  // schedulers, so the sums across warps and blocks are laid out to need few:
+  // each instruction serves all slots at once (block), or one slot a warp
+  // (final).
   const int wid = threadIdx.x >> 5;
   static_assert(kBlock == 256, "eight warps");
   {

@@ -3,8 +3,6 @@
 
 #include <cuda_runtime.h>
 
-#include <type_traits>
-
 #include "gpl_internal.h"
 
 namespace gpl {
@@ -108,9 +106,6 @@ __device__ __forceinline__ float inside(float c, int h, int lo, int hi) {
   return adj;
 }
 
-// fastExp (src/nesterovBase.cpp:1568-1582): (1 + a/1024)^1024 by ten
-// squarings.  The reference's first step is evaluated in double; for a float
-// argument 1 + a/1024 rounded once to float is the same value.
 // Element i of a small pointer array held in kernel parameters, by selects:
 // indexing a parameter array with a run-time index makes the compiler copy
 // the whole parameter block to local memory.
@@ -156,8 +151,10 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
 }
 
 // fastExp (src/nesterovBase.cpp:1568-1582) of two values: (1 + a / 1024)^1024
-// by ten squarings.  The first step fused rounds as a product and a sum would:
-// the product with 2^-10 is exact, or too small to change 1.
+// by ten squarings.  The reference evaluates the first step in double; rounded
+// once to float, 1 + a / 1024 of a float argument is the same value.  Fused it
+// rounds as a product and a sum would: the product with 2^-10 is exact, or too
+// small to change 1.
 __device__ __forceinline__ F2 fast_exp2(F2 a) {
   a = fma2(a, pack2(0.0009765625f, 0.0009765625f), pack2(1.0f, 1.0f));
 #pragma unroll
@@ -189,106 +186,6 @@ __device__ __forceinline__ void block_reduce_n(double (&v)[N], double* out_base,
     }
   }
   __syncthreads();
-}
-
-// The exact double of a float by integer operations: conversions run on the
-// FP64 pipe, which takes 15 cycles per warp instruction on this part.
-__device__ __forceinline__ double widen(float f) {
-  const unsigned u = __float_as_uint(f), e = u & 0x7f800000u;
-  if (e == 0u || e == 0x7f800000u)                  // zero, denormal, infinity, NaN
-    return (u << 1) == 0u ? __hiloint2double((int)u, 0) : (double)f;
-  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
-}
-__device__ __forceinline__ double widen(double d) { return d; }
-
-// The sums block_reduce_n forms of N values a thread over a block of 256
-// threads -- each warp's 32 lanes in a halving tree, then the eight warps'
-// sums in one -- computed by one warp: lane l holds the values of threads
-// 32 g + l, g < 8, in x[k * 8 + g].  The additions are the same ones (a sum's
-// two operands may swap), but 12 (N = 1) or 19 (N = 2) warp instructions
-// replace 45 or 90 on the narrow FP64 pipe: at each step of the tree a lane
-// keeps the half of its sums that its lane bit selects and sends the other
-// half.  tot[k] is returned to every lane.
-template <int N, class T>
-__device__ __forceinline__ void warp_block_sum(const T (&x)[8 * N], double (&tot)[N]) {
-  static_assert(N == 1 || N == 2, "one or two values");
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  double v[4 * N];
-  {
-    const bool hi = lane & 16;
-#pragma unroll
-    for (int j = 0; j < 4 * N; j++) {
-      const T keep = hi ? x[4 * N + j] : x[j], send = hi ? x[j] : x[4 * N + j];
-      v[j] = widen(keep) + widen(__shfl_xor_sync(full, send, 16));
-    }
-  }
-  auto halve = [&](auto n_c, int o) {               // n sums a lane -> n / 2
-    constexpr int h = decltype(n_c)::value / 2;
-    const bool hi = lane & o;
-#pragma unroll
-    for (int j = 0; j < h; j++) {
-      const double keep = hi ? v[h + j] : v[j], send = hi ? v[j] : v[h + j];
-      v[j] = keep + __shfl_xor_sync(full, send, o);
-    }
-  };
-  halve(std::integral_constant<int, 4 * N>{}, 8);
-  halve(std::integral_constant<int, 2 * N>{}, 4);
-  if constexpr (N == 2) halve(std::integral_constant<int, 2>{}, 2);
-  else v[0] += __shfl_xor_sync(full, v[0], 2);
-  v[0] += __shfl_xor_sync(full, v[0], 1);
-  // a lane's warp g: lane bits 16, 8, 4 (N = 1) or 8, 4, 2 (N = 2; bit 16: k)
-#pragma unroll
-  for (int o = N == 1 ? 16 : 8; o >= (N == 1 ? 4 : 2); o >>= 1) v[0] += __shfl_xor_sync(full, v[0], o);
-  if constexpr (N == 1) {
-    tot[0] = v[0];
-  } else {
-    tot[0] = __shfl_sync(full, v[0], 0);
-    tot[1] = __shfl_sync(full, v[0], 16);
-  }
-}
-
-// Sum of p[0..n) by one block in a fixed order (thread-strided, then fixed
-// trees); reads bypass L1 because other blocks wrote the values.  The result
-// is returned to every thread.
-__device__ __forceinline__ double block_sum_ordered(const double* p, int n, double* sh) {
-  double v = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) v += __ldcg(p + i);
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) sh[wid] = v;
-  __syncthreads();
-  if (wid == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-    v = lane < nw ? sh[lane] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) sh[0] = v;
-  }
-  __syncthreads();
-  const double r = sh[0];
-  __syncthreads();
-  return r;
-}
-
-__device__ __forceinline__ long long block_sum_ordered_ll(const long long* p, int n, long long* sh) {
-  long long v = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) v += __ldcg(p + i);
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) sh[wid] = v;
-  __syncthreads();
-  if (wid == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-    v = lane < nw ? sh[lane] : 0ll;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) sh[0] = v;
-  }
-  __syncthreads();
-  const long long r = sh[0];
-  __syncthreads();
-  return r;
 }
 
 }  // namespace gpl

@@ -1005,17 +1005,16 @@ struct BlockRows {
 // the operands of x_j as loaded; cb(raw): x_j from them; scalars(): run by
 // one thread before any cb), then sums the rows into vs; ends with a block
 // barrier (false: stopped, nothing done).  What bounds it is latency: a load
-// from L2 takes about 850 cycles, and a block's chain of them sets the
-// kernel's time.  So the first groups of the warp's stream, its first rows
+// from L2 takes 300 cycles on an idle chip and more here, and a block's chain
+// of them sets the kernel's time.  So the first groups of the warp's stream, its first rows
 // and the first staged entries, which depend on nothing the solve changes,
 // load before the solver's state is read (head(): the state's scalars and
-// buffers; true: stop) and before the window (400k cells 145.9 -> 140.3 ms
-// against the state first; with the state read first but tested here it
-// costs registers: 143.5), the window's operands four at a time, and then a ring of two groups a warp (48 bytes a lane) runs
-// ahead of the sums over all its slices; four groups cost spills and measured
-// 1 % slower.  The ring's loads are unconditional and of one size: behind
-// conditions the compiler waits for each (5.4 thousand cycles for the slices
-// of a 256-row block instead of 2.7).  Against the form that staged every
+// buffers; true: stop) and before the window (initial place of 400k cells
+// 148.8 -> 145.9 ms against the state first), the window's operands four at a
+// time, and then a ring of two groups a warp (48 bytes a lane) runs ahead of
+// the sums over all its slices; four groups cost spills and measured 1 %
+// slower.  The ring's loads are unconditional and of one size: behind
+// conditions the compiler waits for each.  Against the form that staged every
 // product and summed 32 neighbouring rows a warp, the initial place of 400k
 // cells went 183 -> 148 ms, of 1M cells 369 -> 320, of 30k 65.6 -> 62.3.
 template <class Head, class Ld, class Cb, class Sc>
@@ -1107,7 +1106,7 @@ __device__ __forceinline__ bool block_product(const IpDev& D, int axis, int vb, 
     int p = 0, k = 0;
     uint32_t wl = tab[np * wid];
     int len = (row.x >> 16) < kTall ? (int)(row.x >> 16) : 0;
-    float acc = len >= 0 ? __fmul_rn(__uint_as_float(row.y), xs[own + (row.x & 0xffffu)]) : 0.0f;
+    float acc = __fmul_rn(__uint_as_float(row.y), xs[own + (row.x & 0xffffu)]);
     uint2 row2 = __ldg(slots + (1 < mine ? 32 : 0));
     bool go = true;
     while (go) {
@@ -1218,6 +1217,63 @@ __device__ __forceinline__ void for_block_rows(const BlockRows& b, const float* 
 // buffer `par` of p or v (axis `axis`)
 __device__ __forceinline__ float* pv_buf(float* base, const IpDev& D, int par, int axis) {
   return base + ((size_t)par * 2 + axis) * D.n_mov;
+}
+
+// The exact double of a float by integer operations: conversions run on the
+// FP64 pipe, which is narrow on this part.
+__device__ __forceinline__ double widen(float f) {
+  const unsigned u = __float_as_uint(f), e = u & 0x7f800000u;
+  if (e == 0u || e == 0x7f800000u)                  // zero, denormal, infinity, NaN
+    return (u << 1) == 0u ? __hiloint2double((int)u, 0) : (double)f;
+  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
+}
+__device__ __forceinline__ double widen(double d) { return d; }
+
+// The sums block_reduce_n forms of N values a thread over a block of 256
+// threads -- each warp's 32 lanes in a halving tree, then the eight warps'
+// sums in one -- computed by one warp: lane l holds the values of threads
+// 32 g + l, g < 8, in x[k * 8 + g].  The additions are the same ones (a sum's
+// two operands may swap), but 12 (N = 1) or 19 (N = 2) warp instructions
+// replace 45 or 90 on the narrow FP64 pipe: at each step of the tree a lane
+// keeps the half of its sums that its lane bit selects and sends the other
+// half.  tot[k] is returned to every lane.
+template <int N, class T>
+__device__ __forceinline__ void warp_block_sum(const T (&x)[8 * N], double (&tot)[N]) {
+  static_assert(N == 1 || N == 2, "one or two values");
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  double v[4 * N];
+  {
+    const bool hi = lane & 16;
+#pragma unroll
+    for (int j = 0; j < 4 * N; j++) {
+      const T keep = hi ? x[4 * N + j] : x[j], send = hi ? x[j] : x[4 * N + j];
+      v[j] = widen(keep) + widen(__shfl_xor_sync(full, send, 16));
+    }
+  }
+  auto halve = [&](auto n_c, int o) {               // n sums a lane -> n / 2
+    constexpr int h = decltype(n_c)::value / 2;
+    const bool hi = lane & o;
+#pragma unroll
+    for (int j = 0; j < h; j++) {
+      const double keep = hi ? v[h + j] : v[j], send = hi ? v[j] : v[h + j];
+      v[j] = keep + __shfl_xor_sync(full, send, o);
+    }
+  };
+  halve(std::integral_constant<int, 4 * N>{}, 8);
+  halve(std::integral_constant<int, 2 * N>{}, 4);
+  if constexpr (N == 2) halve(std::integral_constant<int, 2>{}, 2);
+  else v[0] += __shfl_xor_sync(full, v[0], 2);
+  v[0] += __shfl_xor_sync(full, v[0], 1);
+  // a lane's warp g: lane bits 16, 8, 4 (N = 1) or 8, 4, 2 (N = 2; bit 16: k)
+#pragma unroll
+  for (int o = N == 1 ? 16 : 8; o >= (N == 1 ? 4 : 2); o >>= 1) v[0] += __shfl_xor_sync(full, v[0], o);
+  if constexpr (N == 1) {
+    tot[0] = v[0];
+  } else {
+    tot[0] = __shfl_sync(full, v[0], 0);
+    tot[1] = __shfl_sync(full, v[0], 16);
+  }
 }
 
 // Block partial sums of up to 2 products, then the last block of this axis
@@ -1869,8 +1925,8 @@ enum IpPhase {
   kIpResidualInit, kIpResidual, kIpPV, kIpST, kIpXr, kIpMove, kIpSell
 };
 
-// (three blocks per SM: at four the product phases spill, 341 against 307 ms
-// for the initial places of 16 jobs of 2k to 50k cells)
+// (three blocks per SM: at four the product phases spill, 184.1 against 182.2
+// ms for the initial places of 16 jobs of 2k to 50k cells)
 template <int Ph>
 __global__ void __launch_bounds__(kB, 3) k_ipb(const IpDev* __restrict__ Ds, const IpParams* __restrict__ Ps,
                                             const int4* __restrict__ items) {
@@ -1920,7 +1976,7 @@ __global__ void k_ipb_states(const IpDev* __restrict__ Ds, const int* __restrict
 
 // ------------------------------------------------------------ device loop
 // The rounds of the kernel-per-phase form as one CUDA graph: WHILE (rounds
-// go on) { assembly; WHILE (a solve goes on) { 8 iterations; chunk tail };
+// go on) { assembly; WHILE (a solve goes on) { chunk; chunk tail };
 // move; round tail }.  The one-thread tails take the decisions the host loop
 // takes between its chunks and rounds (same tests, same values), so the host
 // waits once per initial place instead of once per chunk.
@@ -2028,7 +2084,8 @@ IpSizes ip_sizes(const HostModel& m, const IpCounts& c, int grid_cap) {
   const size_t scan_blocks = blocks_for((int)n_mp);
   // the sliced entries with their padding (widths in fours, each slice as wide
   // as its longest row) and the staged rows: 1.1 to 1.3 of the entries on
-  // generated netlists (and room for the last warp's reads ahead); a block that finds no room keeps the CSR form
+  // generated netlists, more on chains of two-pin nets (and room for the last
+  // warp's reads ahead); a block that finds no room keeps the CSR form
   z.sell_cap = (z.nnz_cap + 2 * z.nnz_cap / 5) / 128 * 128 + 128 * ((size_t)z.grid + 8);
   z.slot_cap = (size_t)z.grid * sell_slots(z.rows_blk);
   auto rnd = [](size_t b) { return (b + 255) / 256 * 256 + 256; };
@@ -2616,7 +2673,7 @@ int run_initial_place(HostModel& m, cudaStream_t s, int sm_count, gpl_ip_stats* 
 // ------------------------------------------------------------ batched form
 // The rounds of many jobs in lockstep: every round, each member's assembly
 // phases run as one launch per phase over the work table, then chunks of
-// eight solver iterations (four launches each) until every member's two
+// solver iterations (chunk_iterations) until every member's two
 // solves are done (a member that finished early skips the later chunks'
 // blocks: every phase body returns at once on a finished solve, as it does
 // in the job's own chunks), then the move; then each member's error and stop

@@ -525,8 +525,8 @@ int launch_phase2(gpl_job* j, bool want_phi, int area_set) {
 // the predicted coordinates, Poisson only the areas), joined before the gcell
 // kernel, whose last block writes the result record, on the host too.  The
 // Poisson passes are the longer chain and go first: launched after WA, their
-// first blocks wait for its (loop of 10k cells 42.1 -> 40.6 us an iteration,
-// 1M 204 -> 199).  With kernel timing on, everything stays on the job's stream
+// first blocks wait for its (loop of 10k cells 42.1 -> 40.5 us an iteration,
+// 1M 245 -> 240).  With kernel timing on, everything stays on the job's stream
 // so that each class is timed alone.
 int launch_eval(gpl_job* j, bool want_phi, int area_set, bool to_host = true, bool ctl_from_host = false) {
   DeviceModel& d = j->d;
@@ -1205,8 +1205,9 @@ BatchRun* batch_create(int device, int capacity, int* rc_out) {
 
 void batch_destroy(BatchRun* B) { delete B; }
 
-// Whether the job can run in a batch: the FFT Poisson form with its
-// shared-memory passes (the batched kernels' form).
+// Whether the job can run in a batch: the FFT Poisson form, on any grid but
+// 512 x 512 and 1024 x 1024, which the interface refuses (jobs of that size
+// keep the GPU busy alone).
 bool batch_eligible(const gpl_job* j) {
   return j->np_ready && j->d.poisson_path == 1 &&
          !(j->d.cnt_x == j->d.cnt_y && (j->d.cnt_x == 512 || j->d.cnt_x == 1024));
@@ -1217,8 +1218,8 @@ bool batch_eligible(const gpl_job* j) {
 int batch_join(BatchRun* B, int slot, gpl_job* j, int max_iters, gpl_iter_log* log) {
   if (slot < 0 || slot >= B->cap || B->members[slot].job) { set_error("batch: slot in use"); return GPL_ERR_BAD_STATE; }
   if (!batch_eligible(j)) {
-    set_error("batched Nesterov loop: the job does not run the block-form FFT Poisson passes (its grid is "
-              "512 x 512 or 1024 x 1024, or it runs the tensor-core form); run it alone");
+    set_error("batched Nesterov loop: the job is not initialised, runs the tensor-core Poisson form, or has a "
+              "512 x 512 or 1024 x 1024 grid; run it alone");
     return GPL_ERR_INVALID_ARG;
   }
   if (j->device != B->device) { set_error("batch: the job is on another device"); return GPL_ERR_INVALID_ARG; }

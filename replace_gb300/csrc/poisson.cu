@@ -1058,9 +1058,12 @@ __global__ void __launch_bounds__(FieldShape<N>::threads(3)) k_poisson_field_g(P
 // back to the rows' owners.  Group FFTs as above (8 or 16 lanes a pair);
 // elements k and n - k by one thread, in place.
 // Solve with the potential: 64 x 64 19.5 -> 6.2 us, 128 x 128 20.5 -> 10.3,
-// 256 x 256 22.6 -> 18.4.  Jobs keep the block form on these grids: the other
-// rounding, amplified over a loop's iterations, moved single cells of 10k-cell
-// designs by up to 1e-3 of the core in 64 iterations.
+// 256 x 256 22.6 -> 18.4.  Jobs keep the block form on these grids.  Another
+// rounding of the field changes a job's placement (a loop amplifies it: single
+// cells of 10k-cell designs move by up to 1e-3 of the core in 64 iterations),
+// so a job's form changes only where its loop gains much: the group form is
+// taken on 512 x 256 (89 -> 46 us an iteration at 10k cells) and up, this one,
+// for 6 % of a 10k-cell loop, is not.
 constexpr int kClCtas = 16;
 
 template <int N>

@@ -80,7 +80,7 @@ __device__ __forceinline__ int2 pin_pos(const WaEval<kW>& V, const int4& r) {
 
 // The four WA exponentials of one pin (src/nesterovBase.cpp:1320-1355);
 // a direction whose exponent is not above minWireLengthForceBar contributes 0.
-// The kernel is bound by the instructions it issues (57 million a million
+// The kernel is bound by the instructions it issues (49 million at a million
 // cells): two exponentials go through each packed multiply, computed for both
 // sides of the bar and selected (12.5k gcells 8.1 -> 7.4 us, 1.25M 66.5 ->
 // 63.7).  The sums are not packed: a packed multiply and add is fused by the
