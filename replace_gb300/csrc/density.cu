@@ -561,17 +561,21 @@ __device__ __forceinline__ void cell_body(const CellArgs& A, int vb, int vgrid) 
   const int wid = threadIdx.x >> 5;
   static_assert(kBlock == 256, "eight warps");
   {
-    // the sums of a warp's even and of its odd lanes (float, fixed xor tree),
-    // then the block's sixteen in FP64.  The tree's last addition rounds the
-    // largest sum: in float it was half the variance of the block's sum, and
-    // the threads' own sums are a thirtieth.  Rms relative error of the totals
-    // over 40 placements, in float to the end and so: 0.58M gcells 5.1e-10 ->
-    // 3.6e-10, 1.17M 5.8e-10 -> 4.1e-10 (six blocks a SM, in float: 4.5e-10 and
-    // 4.2e-10; five make 17 % fewer, larger warp sums)
+    // warp sums (float, fixed xor tree), then the block's eight warps in FP64.
+    // Where a thread has several gcells the tree's last addition is left to
+    // FP64 too (even and odd lanes' sums apart): it rounds the largest sum, half
+    // the variance of the block's, and five blocks an SM instead of six make 17 %
+    // fewer, larger warp sums there (with one gcell a thread the warps are the
+    // same ones).  Rms relative error of the totals over 40 placements, in float
+    // to the end and so: 0.58M gcells 5.1e-10 -> 3.6e-10, 1.17M 5.8e-10 ->
+    // 4.1e-10 (six blocks, in float: 4.5e-10 and 4.2e-10).
+    const bool apart = vgrid * kBlock < A.n_g;
 #pragma unroll
-    for (int k = 0; k < 4; k++)
+    for (int k = 0; k < 4; k++) {
 #pragma unroll
       for (int o = 16; o > 1; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+      if (!apart) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 1);
+    }
     const int any_bad = __any_sync(0xffffffffu, bad);
     if (lane < 2) {
 #pragma unroll
@@ -582,7 +586,8 @@ __device__ __forceinline__ void cell_body(const CellArgs& A, int vb, int vgrid) 
     if (threadIdx.x < 32) {
       // lane 8 k + w: slot k of warp w
       const float2 two = reinterpret_cast<const float2*>(sh)[lane];
-      double t = (double)two.x + (double)two.y;
+      double t = (double)two.x;
+      if (apart) t += (double)two.y;
 #pragma unroll
       for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
       const int bads = __popc(__ballot_sync(0xffffffffu, lane < 8 && sh_bad[lane & 7]));
