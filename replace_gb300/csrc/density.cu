@@ -571,23 +571,28 @@ __device__ __forceinline__ void cell_body(const CellArgs& A, int vb, int vgrid) 
     // 4.1e-10 (six blocks, in float: 4.5e-10 and 4.2e-10).
     const bool apart = vgrid * kBlock < A.n_g;
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
+    for (int k = 0; k < 4; k++)
 #pragma unroll
       for (int o = 16; o > 1; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-      if (!apart) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 1);
-    }
     const int any_bad = __any_sync(0xffffffffu, bad);
-    if (lane < 2) {
+    if (!apart) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 1);
+      if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) sh[k * 8 + wid] = acc[k];
+      }
+    } else if (lane < 2) {
 #pragma unroll
       for (int k = 0; k < 4; k++) sh[k * 16 + wid * 2 + lane] = acc[k];
-      sh_bad[wid] = any_bad;
     }
+    if (lane == 0) sh_bad[wid] = any_bad;
     __syncthreads();
     if (threadIdx.x < 32) {
-      // lane 8 k + w: slot k of warp w
-      const float2 two = reinterpret_cast<const float2*>(sh)[lane];
-      double t = (double)two.x;
-      if (apart) t += (double)two.y;
+      // lane 8 k + w: slot k of warp w (apart: of its two halves)
+      double t;
+      if (!apart) t = (double)sh[lane];
+      else t = (double)sh[2 * lane] + (double)sh[2 * lane + 1];
 #pragma unroll
       for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
       const int bads = __popc(__ballot_sync(0xffffffffu, lane < 8 && sh_bad[lane & 7]));

@@ -576,11 +576,11 @@ __host__ __device__ constexpr float sin64(int m) {   // 0 <= m < 32
 }
 
 // The inverse transforms' cos(pi / 16) and cos(pi / 8): the floats above the
-// nearest ones, which lie almost as far on the other side (3.0e-8
-// and 3.1e-8 instead of 3.0e-8 and 2.8e-8).  Nearest in both directions, every
-// rotation by them shortens, and the error of a solve's transforms adds up in
-// its low modes; so one direction shortens and the other lengthens (2048 x 2048:
-// Ex 1.78e-7 -> 1.67e-7, phi 1.69e-7 -> 1.56e-7).
+// nearest ones, which lie almost as far on the other side (3.0e-8 and 3.1e-8
+// instead of 3.0e-8 and 2.8e-8).  Nearest in both directions, every rotation by
+// them shortens, and the error of a solve's transforms adds up in its low modes;
+// so one direction shortens and the other lengthens (2048 x 2048: Ex 1.78e-7 ->
+// 1.67e-7, phi 1.69e-7 -> 1.56e-7).
 __host__ __device__ constexpr float up64(float c) {
   const float a = c < 0.0f ? -c : c;
   const float u = a == cos64_quad(2) ? 0.98078534f : a == cos64_quad(4) ? 0.92387956f : a;
@@ -760,8 +760,9 @@ __device__ __forceinline__ void group_fft(float2* buf, const float2* tws) {
     }
   } else {
     // stage 2 for G = 2 E: lane pair (2 c, 2 c + 1) takes the even and odd
-    // lanes' elements of column c (k2 = c or c - E), one E-point DFT each, then X[k] = E[k] + W^k O[k]
-    // (even lane) and X[k + E] = E[k] - W^k O[k] (odd lane), W = W_G
+    // lanes' elements of column c (k2 = c or c - E), one E-point DFT each, then
+    // X[k] = E[k] + W^k O[k] (even lane) and X[k + E] = E[k] - W^k O[k] (odd
+    // lane), W = W_G
     static_assert(G == 2 * E, "one or two lanes or columns");
     const int c = l >> 1, odd = l & 1, k2 = c < E / 2 ? c : c - E;
 #pragma unroll
